@@ -349,9 +349,9 @@ int rbx_last_launch_count(const rbx_integrator* h);
  * (synchronous); U comes from the last force evaluation of the preceding rbx_batch_step when no
  * other call has changed the state since. rbx_batch_get_num_dof gives each system's degrees of
  * freedom.
- * Forces come from neighbour lists of atom groups (each rigid body is one group, each free atom a
- * group of its own): two groups are listed together when their centroids lie within cutoff + a
- * skin of 0.06 nm + both groups' radii. Each system rebuilds its lists when one of its centroids has
+ * Forces come from neighbour lists of units of at most four atoms (a rigid body is cut into units;
+ * a free atom is one): two units of different bodies are listed together when their centroids lie
+ * within cutoff + a skin of 0.12 nm + both units' radii. Each system rebuilds its lists when one of its centroids has
  * moved half the skin, and every list is rebuilt for the state a step call ends in (and for the
  * first evaluation after rbx_batch_set_state or rbx_batch_restore), so the forces and energy at a
  * call's start and end depend on the positions alone: a system's results are a function of its own
@@ -411,13 +411,13 @@ int rbx_batch_set_graph_steps(rbx_batch* b, int k);
  *   1. the step kernel's tile shape (rbx_set_tile_threads: 256 or 128 threads, single/mixed
  *      precision with bodies of at most 32 atoms), by the integrator launches' own event times
  *      over 2 x trial_steps steps after an untimed run of trial_steps;
- *   2. the block size of the cell list-build kernel (64, 128 or 256 threads per cell);
+ *   2. the block size of the list-build kernel (64, 128 or 256 threads);
  *   3. where a step takes under 1 ms, so that launch overhead matters, the steps per captured graph
  *      (0, 10 or 50).
  * Trials 2 and 3 run trial_steps steps (2k+1 for a graph of k) twice and time the second run with
  * CUDA events. It keeps the fastest of each, and then restores the batch's exact state
  * (rbx_batch_restore): no choice changes any result, since each body is integrated alike in any
- * tile, each group's list (and so each atom's force sum) keeps its order, and graphs replay the
+ * tile, each unit's list (and so each atom's force sum) keeps its order, and graphs replay the
  * same launches.
  * chosen[2] (optional) receives the block size and the graph run length; rbx_batch_get_tile_threads
  * the tile shape. rbx_batch_set_tuning and rbx_batch_set_tile_threads set them by hand. */

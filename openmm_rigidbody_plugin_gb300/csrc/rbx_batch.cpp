@@ -26,8 +26,11 @@ using namespace rbx;
 namespace {
 
 constexpr double kOne4PiEps0 = 138.935456;  // kJ nm / (mol e^2)
-constexpr double kSkin = 0.06;              // nm: neighbour-list skin (of group centroids)
-constexpr int kMaxTypes = 32;               // atom types of the type-pair table (FFDev::types)
+// Neighbour-list skin (nm, of unit centroids). A longer list costs the force pass one distance test
+// per entry, a shorter one more builds: 256 boxes of the mix at 750 K take 19.7, 18.8, 18.3 and 17.9 ms
+// per 20 steps at 0.06, 0.09, 0.12 and 0.15 nm, 66,666 waters at 1100 K 7.5, 7.1, 7.2 and 7.0; at 300 K,
+// where lists last longer, the shorter ones gain, and their memory grows with the cube.
+constexpr double kSkin = 0.12;
 
 #define BATCH_TRY(call)                                                                             \
     do {                                                                                            \
@@ -35,24 +38,18 @@ constexpr int kMaxTypes = 32;               // atom types of the type-pair table
         if (e_ != cudaSuccess) return set_error(RBX_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-float int_bits(int v) {
-    float f;
-    std::memcpy(&f, &v, sizeof f);
-    return f;
-}
-
-// body(s) for every system s, the systems split into contiguous ranges of about equal group counts
+// body(s) for every system s, the systems split into contiguous ranges of about equal unit counts
 // over the host's cores. Each call writes only its own system's outputs, so the results do not
 // depend on the split; a thread that cannot be started leaves its range to the calling thread.
 template <class F> void for_each_system(const std::vector<FFSys>& sys, F&& body) {
     const int S = (int)sys.size();
-    const long long groups = S ? (long long)sys[S - 1].g1 - sys[0].g0 : 0;
+    const long long units = S ? (long long)sys[S - 1].u1 - sys[0].u0 : 0;
     const int nt = (int)std::min<long long>({(long long)std::max(1u, std::thread::hardware_concurrency()), 32LL,
-                                             std::max(1LL, groups / 20000)});
+                                             std::max(1LL, units / 20000)});
     std::vector<int> lo(nt + 1, S);
     lo[0] = 0;
     for (int t = 1, s = 0; t < nt; t++) {
-        while (s < S && (long long)(sys[s].g0 - sys[0].g0) * nt < groups * t) s++;
+        while (s < S && (long long)(sys[s].u0 - sys[0].u0) * nt < units * t) s++;
         lo[t] = s;
     }
     auto run = [&](int t) {
@@ -86,21 +83,19 @@ struct rbx_batch {
     std::vector<int> offsets;
     // force field
     DevArray<FFSys> d_sys;
-    DevArray<int> d_iatom, d_isys, d_cell_of, d_cell_count, d_cell_start, d_cell_cursor, d_cell_list;
-    DevArray<int> d_grp_k0, d_grp_n, d_gsys, d_kgrp;
-    DevArray<int2> d_grp_kn;
-    DevArray<int> d_mc_cell, d_mc_sys, d_sc_sys, d_sc_g0;
-    DevArray<int> d_pass_groups[kForcePasses];  // FFDev::pass_groups
-    DevArray<float4> d_param, d_cpos, d_gcen, d_gref, d_gq, d_types;
+    DevArray<int> d_iatom, d_ugrp, d_usys, d_place, d_unit_at, d_cell_of, d_cell_count, d_cell_start, d_cell_cursor;
+    DevArray<int> d_sgrp, d_mc_cell, d_mc_sys, d_ncnt, d_atype;
+    DevArray<int2> d_unit;
+    DevArray<float4> d_param, d_ucen, d_uref, d_scen, d_spos, d_spar, d_types;
     DevArray<unsigned char> d_rebuild;  // FFDev::rebuild
-    DevArray<unsigned int> d_nbr;       // neighbour lists of groups (FFDev::nbr)
-    DevArray<int> d_ncnt, d_atype;
+    DevArray<unsigned int> d_nbr;       // neighbour lists of units (FFDev::nbr)
     DevArray<unsigned int> d_rebuilds;  // list builds per system (FFDev::rebuilds)
-    // host copies for the set-up with a state: systems, cells allocated per system, group layout
+    // host copies for the set-up with a state: systems, cells allocated per system, unit layout
     std::vector<FFSys> sys_h;
-    std::vector<int> cells_alloc, iatom_h, grp_k0_h, grp_n_h;
+    std::vector<int> cells_alloc, iatom_h;
+    std::vector<int2> unit_h;
     std::vector<double> box_h;
-    DevArray<double> d_e_group, d_energy;
+    DevArray<double> d_e_unit, d_energy;
     FFDev ff{};
     // per-system reductions
     DevArray<int> d_body0, d_free0;
@@ -152,47 +147,36 @@ namespace {
 
 int check(const rbx_batch* b) { return b ? RBX_OK : set_error(RBX_ERR_INVALID_ARGUMENT, "null batch handle"); }
 
-// Neighbour-list geometry for a state (host positions, user order): each group's radius about its
+// Neighbour-list geometry for a state (host positions, user order): each unit's radius about its
 // centroid (constant for a rigid body), and from the largest radius of each system its list cells
-// (at least cutoff + skin + two radii per edge), the build work lists and the list capacity.
+// (at least cutoff + skin + two radii per edge), the cell work list and the list capacity.
 int setup_lists(rbx_batch* b, const double* x) {
     const int S = b->S;
     std::vector<FFSys> sys = b->sys_h;
-    std::vector<int> mc_cell, mc_sys, sc_sys, sc_g0;
-    std::vector<uint32_t> zkey(b->grp_n_h.size());  // spatial order of each system's groups (see below)
-    std::vector<double> rho(S, 0.0);                // largest atom distance from a group centroid
-    // per system (in parallel): centroids, their Z-order codes and the largest radius
+    std::vector<int> mc_cell, mc_sys;
+    std::vector<double> rho(S, 0.0);  // largest atom distance from a unit centroid
     for_each_system(sys, [&](int s) {
         const FFSys& f = sys[s];
         const double L = b->box_h[s];
         auto img = [L](double d) { return d - L * std::nearbyint(d / L); };
         double rho_max = 0.0;
-        for (int g = f.g0; g < f.g1; g++) {
-            const int k0 = b->grp_k0_h[g], n = b->grp_n_h[g];
+        for (int u = f.u0; u < f.u1; u++) {
+            const int k0 = b->unit_h[u].x, n = b->unit_h[u].y & 0xff;
             const double* x0 = x + 3 * (size_t)b->iatom_h[k0];
             double c[3] = {0.0, 0.0, 0.0};
             for (int a = 1; a < n; a++)
                 for (int d = 0; d < 3; d++) c[d] += img(x[3 * (size_t)b->iatom_h[k0 + a] + d] - x0[d]);
             for (int d = 0; d < 3; d++) c[d] = x0[d] + c[d] / n;
-            // Z-order (Morton) code of the centroid on a 1024^3 grid of the box
-            uint32_t z = 0;
-            for (int d = 0; d < 3; d++) {
-                double u = c[d] / L;
-                u -= std::floor(u);
-                const uint32_t q = std::min<uint32_t>(1023, (uint32_t)(u * 1024.0));
-                for (int bit = 0; bit < 10; bit++) z |= ((q >> bit) & 1u) << (3 * bit + d);
-            }
-            zkey[g] = z;
             for (int a = 0; a < n; a++) {
                 double r2 = 0.0;
                 for (int d = 0; d < 3; d++) {
                     const double v = img(x[3 * (size_t)b->iatom_h[k0 + a] + d] - c[d]);
                     r2 += v * v;
                 }
-                rho_max = std::max(rho_max, std::sqrt(r2));
+                rho_max = std::max(rho_max, r2);
             }
         }
-        rho[s] = rho_max;
+        rho[s] = std::sqrt(rho_max);
     });
     double cap_need = 1.0;
     for (int s = 0; s < S; s++) {
@@ -205,73 +189,53 @@ int setup_lists(rbx_batch* b, const double* x) {
         if (nc > b->cells_alloc[s]) nc = b->cells_alloc[s];
         if (nc < 3) nc = 1;
         f.nc = nc;
-        if (nc > 1) {
+        if (nc > 1)
             for (int c = 0; c < nc * nc * nc; c++) {
                 mc_cell.push_back(f.c0 + c);
                 mc_sys.push_back(s);
             }
-        } else {
-            for (int g = f.g0; g < f.g1; g += 64) {
-                sc_sys.push_back(s);
-                sc_g0.push_back(g);
-            }
-        }
-        const int G = f.g1 - f.g0;
+        const int U = f.u1 - f.u0;
         const double reach = (double)f.rl + 2.0 * rho_max;
-        const double expect = 4.18879 * reach * reach * reach * (double)G / (L * L * L);
-        cap_need = std::max(cap_need, std::min((double)std::max(G - 1, 1), 1.35 * expect + 32.0));
+        const double expect = 4.18879 * reach * reach * reach * (double)U / (L * L * L);
+        cap_need = std::max(cap_need, std::min((double)std::max(U - 1, 1), 1.35 * expect + 32.0));
     }
     const int cap = std::max(32, ((int)std::ceil(cap_need) + 31) / 32 * 32);
-    const size_t entries = (size_t)std::max(b->ff.n_groups, 1) * (size_t)cap;
+    const size_t entries = (size_t)std::max(b->ff.n_units, 1) * (size_t)cap;
     if (b->d_nbr.n < entries && b->d_nbr.alloc(entries) != cudaSuccess)
-        return set_error(RBX_ERR_CUDA, "cudaMalloc of the neighbour lists failed (%d entries per group)", cap);
-    // The force pass takes its groups in this order: system by system, each system's groups in
-    // Z-order of their centroids (ties by index), so that the warps resident on an SM at once work
-    // on neighbouring groups and find much of each other's neighbours in L1. The order schedules
-    // work only: every group's forces are formed alike whichever warp forms them. Each system's
-    // share of a pass is filled and sorted in place, the systems in parallel.
-    {
-        std::vector<int> pass[kForcePasses];
-        std::vector<size_t> at((size_t)kForcePasses * (S + 1), 0);  // at[k * (S + 1) + s]: system s's start in pass k
-        for (int s = 0; s < S; s++)
-            for (int g = sys[s].g0; g < sys[s].g1; g++) at[(size_t)force_pass_of(b->grp_n_h[g]) * (S + 1) + s + 1]++;
-        for (int k = 0; k < kForcePasses; k++) {
-            size_t* a = &at[(size_t)k * (S + 1)];
-            for (int s = 0; s < S; s++) a[s + 1] += a[s];
-            pass[k].resize(a[S]);
-        }
-        for_each_system(sys, [&](int s) {
-            size_t fill[kForcePasses];
-            for (int k = 0; k < kForcePasses; k++) fill[k] = at[(size_t)k * (S + 1) + s];
-            for (int g = sys[s].g0; g < sys[s].g1; g++) {
-                const int k = force_pass_of(b->grp_n_h[g]);
-                pass[k][fill[k]++] = g;
-            }
-            auto by_key = [&](int u, int v) { return zkey[u] < zkey[v] || (zkey[u] == zkey[v] && u < v); };
-            for (int k = 0; k < kForcePasses; k++)
-                std::sort(pass[k].begin() + at[(size_t)k * (S + 1) + s], pass[k].begin() + fill[k], by_key);
-        });
-        for (int k = 0; k < kForcePasses; k++)
-            if (!pass[k].empty())
-                BATCH_TRY(cudaMemcpy(b->d_pass_groups[k].p, pass[k].data(), sizeof(int) * pass[k].size(),
-                                     cudaMemcpyHostToDevice));
-    }
+        return set_error(RBX_ERR_CUDA, "cudaMalloc of the neighbour lists failed (%d entries per unit)", cap);
     BATCH_TRY(cudaMemcpy(b->d_sys.p, sys.data(), sizeof(FFSys) * (size_t)S, cudaMemcpyHostToDevice));
     if (!mc_cell.empty()) {
         BATCH_TRY(cudaMemcpy(b->d_mc_cell.p, mc_cell.data(), sizeof(int) * mc_cell.size(), cudaMemcpyHostToDevice));
         BATCH_TRY(cudaMemcpy(b->d_mc_sys.p, mc_sys.data(), sizeof(int) * mc_sys.size(), cudaMemcpyHostToDevice));
     }
-    if (!sc_sys.empty()) {
-        BATCH_TRY(cudaMemcpy(b->d_sc_sys.p, sc_sys.data(), sizeof(int) * sc_sys.size(), cudaMemcpyHostToDevice));
-        BATCH_TRY(cudaMemcpy(b->d_sc_g0.p, sc_g0.data(), sizeof(int) * sc_g0.size(), cudaMemcpyHostToDevice));
-    }
     BATCH_TRY(cudaMemset(b->d_rebuild.p, 1, (size_t)S));
     FFDev& D = b->ff;
     D.n_mc = (int)mc_cell.size();
-    D.n_sc = (int)sc_sys.size();
     D.cap = cap;
     D.nbr = b->d_nbr.p;
     return RBX_OK;
+}
+
+// Most atoms per unit of a system, from its group sizes: the size with the least pair work, as the
+// force pass costs it (per unit pair 28 instructions to find and fetch the listed unit, per atom of
+// it 11, per atom pair 17; an atom record is paid for whether it holds an atom or not). Each group is
+// cut evenly.
+int unit_atoms(const std::vector<int>& group_sizes) {
+    double best_cost = 0.0;
+    int best = 1;
+    for (int m = 1; m <= kMaxUnit; m++) {
+        double units = 0.0, atoms = 0.0;
+        for (int n : group_sizes) {
+            units += (n + m - 1) / m;
+            atoms += n;
+        }
+        const double cost = units * (units * (28.0 + 11.0 * m) + 17.0 * m * atoms);
+        if (m == 1 || cost < best_cost) {
+            best_cost = cost;
+            best = m;
+        }
+    }
+    return best;
 }
 
 DevBuf buffers(rbx_batch* b) {
@@ -419,17 +383,19 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     if (rc) { delete b; return rc; }
 
     // force field tables: interacting atoms (charge or LJ) system by system and, within a system,
-    // body by body (ascending id; each free atom a group of its own)
+    // body by body (ascending id; each free atom a group of its own), each group cut into units with
+    // their Lennard-Jones atoms first
     std::vector<FFSys> sys(num_systems);
-    std::vector<int> iatom, isys, grp_k0, grp_n, gsys, kgrp;
+    std::vector<int> iatom, usys, ugrp;
+    std::vector<int2> unit;
     std::vector<float4> param;
-    int cells = 0;
+    int cells = 0, groups = 0, slots = 1;
     for (int s = 0; s < num_systems; s++) {
         FFSys& f = sys[s];
         f.a0 = atom_offsets[s];
         f.a1 = atom_offsets[s + 1];
         f.i0 = (int)iatom.size();
-        f.g0 = (int)grp_k0.size();
+        f.u0 = (int)unit.size();
         std::map<int, std::vector<int>> bodies;
         std::vector<int> free_atoms;
         for (int i = f.a0; i < f.a1; i++) {
@@ -437,23 +403,36 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
             if (body_indices[i] > 0) bodies[body_indices[i]].push_back(i);
             else free_atoms.push_back(i);
         }
-        auto add_group = [&](const std::vector<int>& atoms) {
-            grp_k0.push_back((int)iatom.size());
-            grp_n.push_back((int)atoms.size());
-            gsys.push_back(s);
-            for (int i : atoms) {
-                kgrp.push_back((int)grp_k0.size() - 1);
-                iatom.push_back(i);
-                isys.push_back(s);
-                const float qs = (float)(std::sqrt(kOne4PiEps0) * charges[i]);
-                param.push_back(make_float4(qs, (float)(0.5 * sigmas[i]), (float)std::sqrt(std::max(epsilons[i], 0.0)),
-                                            int_bits(ids[i])));
+        std::vector<int> sizes(free_atoms.size(), 1);
+        for (auto& kv : bodies) sizes.push_back((int)kv.second.size());
+        const int most = unit_atoms(sizes);
+        auto add_group = [&](const int* atoms, int n) {
+            const int m = (n + most - 1) / most;
+            for (int k = 0; k < m; k++) {
+                const int lo = (int)((long long)n * k / m), hi = (int)((long long)n * (k + 1) / m);
+                int lj = 0;
+                const int k0 = (int)iatom.size();
+                for (int pass = 0; pass < 2; pass++)
+                    for (int a = lo; a < hi; a++) {
+                        const int i = atoms[a];
+                        const float root = (float)std::sqrt(std::max(epsilons[i], 0.0));
+                        if ((root != 0.0f) != (pass == 0)) continue;
+                        lj += pass == 0;
+                        iatom.push_back(i);
+                        param.push_back(make_float4((float)(std::sqrt(kOne4PiEps0) * charges[i]), (float)(0.5 * sigmas[i]),
+                                                    root, 0.0f));
+                    }
+                unit.push_back(make_int2(k0, (hi - lo) | lj << 8));
+                usys.push_back(s);
+                ugrp.push_back(groups);
+                slots = std::max(slots, hi - lo);
             }
+            groups++;
         };
-        for (auto& kv : bodies) add_group(kv.second);
-        for (int i : free_atoms) add_group(std::vector<int>{i});
+        for (auto& kv : bodies) add_group(kv.second.data(), (int)kv.second.size());
+        for (int i : free_atoms) add_group(&i, 1);
         f.i1 = (int)iatom.size();
-        f.g1 = (int)grp_k0.size();
+        f.u1 = (int)unit.size();
         if (f.i1 - f.i0 >= kMaxSystemAtoms) {
             delete b;
             return set_error(RBX_ERR_UNSUPPORTED, "system %d: %d interacting atoms (at most %d)", s, f.i1 - f.i0,
@@ -463,7 +442,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         // Pairs are tested by minimum image when the lists are built (and, where cutoff + two radii
         // may reach half the box, when forces are formed), so cutoff + skin + radii may exceed half
         // the box: an image within the cutoff (below half the box) is always the minimum image, and
-        // its group pair is always listed.
+        // its unit pair is always listed.
         f.rl = (float)(rc_s + kSkin);
         f.half_skin2 = (float)(0.25 * kSkin * kSkin);
         f.pair_image = 1;  // until the radii are known (rbx_batch_set_state)
@@ -486,28 +465,17 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     b->cells_alloc.resize(num_systems);
     for (int s = 0; s < num_systems; s++) b->cells_alloc[s] = sys[s].nc;
     b->iatom_h = iatom;
-    b->grp_k0_h = grp_k0;
-    b->grp_n_h = grp_n;
+    b->unit_h = unit;
     b->box_h.assign(box_edges, box_edges + num_systems);
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) { delete b; return set_error(RBX_ERR_CUDA, "cudaSetDevice(%d): %s", device, cudaGetErrorString(e)); }
-    const int nint = (int)iatom.size(), ngrp = (int)grp_k0.size();
+    const int nint = (int)iatom.size(), nunit = (int)unit.size();
     rc = upload_vec(b->d_sys, sys);
     if (!rc) rc = upload_vec(b->d_iatom, iatom);
-    if (!rc) rc = upload_vec(b->d_isys, isys);
     if (!rc) rc = upload_vec(b->d_param, param);
-    if (!rc) rc = upload_vec(b->d_grp_k0, grp_k0);
-    if (!rc) rc = upload_vec(b->d_grp_n, grp_n);
-    {
-        std::vector<int2> kn(grp_k0.size());
-        for (size_t g = 0; g < kn.size(); g++) kn[g] = make_int2(grp_k0[g], grp_n[g]);
-        if (!rc) rc = upload_vec(b->d_grp_kn, kn);
-    }
-    if (!rc) rc = upload_vec(b->d_gsys, gsys);
-    if (!rc) rc = upload_vec(b->d_kgrp, kgrp);
-    std::vector<int> pass_groups[kForcePasses];  // the force passes' groups, by size
-    for (int g = 0; g < (int)grp_n.size(); g++) pass_groups[force_pass_of(grp_n[g])].push_back(g);
-    for (int k = 0; k < kForcePasses && !rc; k++) rc = upload_vec(b->d_pass_groups[k], pass_groups[k]);
+    if (!rc) rc = upload_vec(b->d_unit, unit);
+    if (!rc) rc = upload_vec(b->d_usys, usys);
+    if (!rc) rc = upload_vec(b->d_ugrp, ugrp);
     // atom types: the distinct (scaled charge, sigma/2, sqrt(epsilon)) triples; with at most
     // kMaxTypes of them the force pass reads one 16-byte record per neighbour (position and type)
     // and takes each pair's coefficients from a table of type pairs
@@ -527,7 +495,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         if ((int)types.size() > kMaxTypes) types.clear();
     }
     if (types.empty()) type_of.clear();
-    // the type-pair table: (K q_i q_j, 12 C12, 6 C6) with C12 = 4 eps sig^12, C6 = 4 eps sig^6 and
+    // the type-pair table: (K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j) with C12 = 4 eps sig^12, C6 = 4 eps sig^6 and
     // Lorentz-Berthelot sig = (sig_i + sig_j)/2, eps = sqrt(eps_i eps_j), formed in FP64 from the
     // FP32 type values (the force is (12 C12 r^-6 - 6 C6) r^-8 r)
     const int nt = (int)types.size();
@@ -537,23 +505,20 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
             const double sig = (double)types[i].y + (double)types[j].y, eps = (double)types[i].z * (double)types[j].z;
             const double s6 = sig * sig * sig * sig * sig * sig;
             pair_table[(size_t)i * nt + j] = make_float4((float)((double)types[i].x * (double)types[j].x),
-                                                         (float)(48.0 * eps * s6 * s6), (float)(24.0 * eps * s6), 0.0f);
+                                                         (float)(48.0 * eps * s6 * s6), (float)(24.0 * eps * s6), types[j].x);
         }
     if (!rc) rc = upload_vec(b->d_types, pair_table);
     if (!rc) rc = upload_vec(b->d_atype, type_of);
-    // work lists (filled with the state): at most every cell, and every 64-group chunk
-    size_t sc_max = 0;
-    for (int s = 0; s < num_systems; s++) sc_max += (size_t)(sys[s].g1 - sys[s].g0 + 63) / 64;
-    const int g1 = std::max(ngrp, 1), n1 = std::max(nint, 1);
-    if (!rc && (b->d_cell_of.alloc(g1) != cudaSuccess || b->d_cell_list.alloc(g1) != cudaSuccess ||
-                b->d_gcen.alloc(g1) != cudaSuccess || b->d_gref.alloc(g1) != cudaSuccess ||
-                b->d_gq.alloc(g1) != cudaSuccess || b->d_ncnt.alloc(g1) != cudaSuccess ||
+    const size_t u1 = std::max(nunit, 1), records = u1 * slots;
+    if (!rc && (b->d_place.alloc(u1) != cudaSuccess || b->d_unit_at.alloc(u1) != cudaSuccess ||
+                b->d_cell_of.alloc(u1) != cudaSuccess || b->d_ucen.alloc(u1) != cudaSuccess ||
+                b->d_uref.alloc(u1) != cudaSuccess || b->d_scen.alloc(u1) != cudaSuccess ||
+                b->d_sgrp.alloc(u1) != cudaSuccess || b->d_ncnt.alloc(u1) != cudaSuccess ||
+                b->d_spos.alloc(records) != cudaSuccess || b->d_spar.alloc(types.empty() ? records : 0) != cudaSuccess ||
                 b->d_cell_count.alloc(cells) != cudaSuccess || b->d_cell_start.alloc(cells + 1) != cudaSuccess ||
-                b->d_cell_cursor.alloc(cells) != cudaSuccess || b->d_cpos.alloc(n1) != cudaSuccess ||
-                b->d_e_group.alloc(g1) != cudaSuccess || b->d_mc_cell.alloc(std::max(cells, 1)) != cudaSuccess ||
+                b->d_cell_cursor.alloc(cells) != cudaSuccess || b->d_e_unit.alloc(u1) != cudaSuccess ||
+                b->d_mc_cell.alloc(std::max(cells, 1)) != cudaSuccess ||
                 b->d_mc_sys.alloc(std::max(cells, 1)) != cudaSuccess ||
-                b->d_sc_sys.alloc(std::max<size_t>(sc_max, 1)) != cudaSuccess ||
-                b->d_sc_g0.alloc(std::max<size_t>(sc_max, 1)) != cudaSuccess ||
                 b->d_energy.alloc(num_systems) != cudaSuccess || b->d_ke.alloc(2 * (size_t)num_systems) != cudaSuccess ||
                 b->d_user.alloc(3 * (size_t)N) != cudaSuccess || b->d_sys_status.alloc(num_systems) != cudaSuccess ||
                 b->d_rebuild.alloc(num_systems) != cudaSuccess || b->d_rebuilds.alloc(num_systems) != cudaSuccess))
@@ -562,8 +527,9 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
                 cudaMemset(b->d_cell_count.p, 0, sizeof(int) * (size_t)cells) != cudaSuccess ||
                 cudaMemset(b->d_rebuild.p, 1, (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_rebuilds.p, 0, sizeof(unsigned int) * (size_t)num_systems) != cudaSuccess ||
-                cudaMemset(b->d_ncnt.p, 0, sizeof(int) * (size_t)g1) != cudaSuccess ||
-                cudaMemset(b->d_cell_list.p, 0, sizeof(int) * (size_t)g1) != cudaSuccess))
+                cudaMemset(b->d_ncnt.p, 0, sizeof(int) * u1) != cudaSuccess ||
+                cudaMemset(b->d_place.p, 0, sizeof(int) * u1) != cudaSuccess ||
+                cudaMemset(b->d_unit_at.p, 0, sizeof(int) * u1) != cudaSuccess))
         rc = set_error(RBX_ERR_CUDA, "initialisation of the force-field arrays failed");
     if (!rc && cudaMallocHost((void**)&b->h_out, sizeof(double) * 3 * (size_t)num_systems) != cudaSuccess)
         rc = set_error(RBX_ERR_CUDA, "pinned allocation failed");
@@ -571,49 +537,45 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     FFDev& D = b->ff;
     D.S = num_systems;
     D.n_int = nint;
-    D.n_groups = ngrp;
+    D.n_units = nunit;
     D.n_cells = cells;
     D.sys = b->d_sys.p;
     D.iatom = b->d_iatom.p;
-    D.isys = b->d_isys.p;
     D.param = b->d_param.p;
-    D.grp_k0 = b->d_grp_k0.p;
-    D.grp_n = b->d_grp_n.p;
-    D.grp_kn = b->d_grp_kn.p;
-    D.gsys = b->d_gsys.p;
-    D.kgrp = b->d_kgrp.p;
-    D.gcen = b->d_gcen.p;
-    D.gref = b->d_gref.p;
-    D.gq = b->d_gq.p;
+    D.unit = b->d_unit.p;
+    D.ugrp = b->d_ugrp.p;
+    D.usys = b->d_usys.p;
+    D.ucen = b->d_ucen.p;
+    D.uref = b->d_uref.p;
+    D.place = b->d_place.p;
+    D.unit_at = b->d_unit_at.p;
     D.cell_of = b->d_cell_of.p;
     D.cell_count = b->d_cell_count.p;
     D.cell_start = b->d_cell_start.p;
     D.cell_cursor = b->d_cell_cursor.p;
-    D.cell_list = b->d_cell_list.p;
-    D.cpos = b->d_cpos.p;
-    D.e_group = b->d_e_group.p;
+    D.scen = b->d_scen.p;
+    D.sgrp = b->d_sgrp.p;
+    for (int a = 0; a < kMaxUnit; a++) {
+        D.spos[a] = a < slots ? b->d_spos.p + a * u1 : nullptr;
+        D.spar[a] = a < slots && types.empty() ? b->d_spar.p + a * u1 : nullptr;
+    }
+    D.slots = slots;
+    D.e_unit = b->d_e_unit.p;
     D.energy = b->d_energy.p;
     D.fcap = 0.0f;
     D.sys_status = b->d_sys_status.p;
     D.rebuild = b->d_rebuild.p;
     D.rebuilds = b->d_rebuilds.p;
-    D.nbr = nullptr;  // allocated with the state (its capacity follows the groups' radii)
+    D.nbr = nullptr;  // allocated with the state (its capacity follows the units' radii)
     D.ncnt = b->d_ncnt.p;
     D.cap = 0;
     D.types = b->d_types.p;
     D.atype = b->d_atype.p;
     D.ntypes = (int)types.size();
-    for (int k = 0; k < kForcePasses; k++) {
-        D.n_pass[k] = (int)pass_groups[k].size();
-        D.pass_groups[k] = b->d_pass_groups[k].p;
-    }
-    D.cell_threads = 128;
+    D.build_threads = 128;
     D.n_mc = 0;
-    D.n_sc = 0;
     D.mc_cell = b->d_mc_cell.p;
     D.mc_sys = b->d_mc_sys.p;
-    D.sc_sys = b->d_sc_sys.p;
-    D.sc_g0 = b->d_sc_g0.p;
     // the owned OpenMM-layout buffers (forces of non-interacting atoms stay zero)
     rbx_buffers rb;
     if ((rc = rbx_context_buffers(b->integ, &rb))) { delete b; return rc; }
@@ -826,15 +788,13 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
     int rc = check(b);
     if (rc) return rc;
     if (!bytes) return set_error(RBX_ERR_INVALID_ARGUMENT, "null output");
-    size_t n = b->d_sys.bytes() + b->d_iatom.bytes() + b->d_isys.bytes() + b->d_cell_of.bytes() +
-               b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() + b->d_cell_list.bytes() +
-               b->d_grp_k0.bytes() + b->d_grp_n.bytes() + b->d_grp_kn.bytes() + b->d_gsys.bytes() + b->d_kgrp.bytes() +
-               b->d_mc_cell.bytes() + b->d_mc_sys.bytes() + b->d_sc_sys.bytes() + b->d_sc_g0.bytes() +
-               b->d_pass_groups[0].bytes() + b->d_pass_groups[1].bytes() + b->d_pass_groups[2].bytes() +
-               b->d_param.bytes() + b->d_cpos.bytes() + b->d_gcen.bytes() + b->d_gref.bytes() + b->d_gq.bytes() +
-               b->d_types.bytes() + b->d_rebuild.bytes() + b->d_nbr.bytes() + b->d_ncnt.bytes() + b->d_atype.bytes() +
-               b->d_rebuilds.bytes() + b->d_e_group.bytes() + b->d_energy.bytes() + b->d_body0.bytes() +
-               b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes();
+    size_t n = b->d_sys.bytes() + b->d_iatom.bytes() + b->d_param.bytes() + b->d_unit.bytes() + b->d_ugrp.bytes() +
+               b->d_usys.bytes() + b->d_ucen.bytes() + b->d_uref.bytes() + b->d_place.bytes() + b->d_unit_at.bytes() +
+               b->d_cell_of.bytes() + b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
+               b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_spos.bytes() + b->d_spar.bytes() + b->d_mc_cell.bytes() +
+               b->d_mc_sys.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_rebuild.bytes() + b->d_nbr.bytes() +
+               b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_e_unit.bytes() + b->d_energy.bytes() +
+               b->d_body0.bytes() + b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes();
     *bytes = n + (b->integ ? device_bytes(b->integ) : 0);
     return RBX_OK;
 }
@@ -906,7 +866,7 @@ int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, i
         return r;
     };
     const int k0 = b->graph_k;
-    int best_ct = b->ff.cell_threads, best_k = k0;
+    int best_ct = b->ff.build_threads, best_k = k0;
     float best = 0.0f, ms = 0.0f;
     b->graph_k = 0;
     b->drop_graph();
@@ -936,18 +896,17 @@ int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, i
         const int rc1 = rbx_set_tile_threads(b->integ, best_nt);
         if (!rc) rc = rc1;
     }
-    // 2. block size of the cell list-build kernel, direct launches
+    // 2. block size of the list-build kernel, direct launches
     const int cts[3] = {64, 128, 256};
     for (int i = 0; i < 3 && !rc; i++) {
-        if (!b->ff.n_mc && cts[i] != best_ct) continue;
-        b->ff.cell_threads = cts[i];
+        b->ff.build_threads = cts[i];
         if ((rc = per_step(trial_steps, ms))) break;
-        if (i == 0 || ms < best || !b->ff.n_mc) {
+        if (i == 0 || ms < best) {
             best = ms;
             best_ct = cts[i];
         }
     }
-    b->ff.cell_threads = best_ct;
+    b->ff.build_threads = best_ct;
     // 3. steps per captured graph, where launch overhead matters (steps under 1 ms)
     if (!rc && best < 1.0f) {
         const int ks[3] = {0, 10, 50};
@@ -1004,8 +963,8 @@ int rbx_batch_set_tuning(rbx_batch* b, int cell_threads, int graph_steps) {
     if (cell_threads != 64 && cell_threads != 128 && cell_threads != 256)
         return set_error(RBX_ERR_INVALID_ARGUMENT, "cell kernel block size must be 64, 128 or 256");
     if ((rc = rbx_batch_set_graph_steps(b, graph_steps))) return rc;
-    if (cell_threads != b->ff.cell_threads) b->drop_graph();
-    b->ff.cell_threads = cell_threads;
+    if (cell_threads != b->ff.build_threads) b->drop_graph();
+    b->ff.build_threads = cell_threads;
     return RBX_OK;
 }
 

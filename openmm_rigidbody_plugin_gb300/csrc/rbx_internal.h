@@ -95,54 +95,59 @@ struct DevBuf {
 // Cutoff LJ + reaction-field force field over many independent cubic boxes (rbx_forces.cu).
 // Interacting atoms (non-zero charge or LJ epsilon) are listed system by system and, within a
 // system, body by body: the interacting atoms of one rigid body (or one free atom) form a group,
-// a contiguous range of the list. Neighbour lists pair groups, not atoms: a rigid group's atoms stay
-// within its radius of its centroid whatever it rotates, so only centroid motion ages a list.
-// Cells (of groups, by centroid) of all systems are numbered consecutively.
+// a contiguous range of the list, and each group is cut into units of at most kMaxUnit atoms (a
+// water is one unit of 3). Neighbour lists pair units, not atoms: a rigid unit's atoms stay within
+// its radius of its centroid whatever the body rotates, so only centroid motion ages a list.
+// Cells (of units, by centroid) of all systems are numbered consecutively. Units are numbered as
+// listed (index u) and, from every list build on, by place in cell order (p), system by system.
+constexpr int kMaxUnit = 4;
 struct FFSys {
     int a0, a1;   // device slots of the system's atoms
     int i0, i1;   // its interacting atoms, as a range of the interacting-atom list
-    int g0, g1;   // its groups
+    int u0, u1;   // its units (as indices u, and as places p)
     int c0, nc;   // first cell and cells per box edge of the list build (1: one cell, all pairs)
     float L, invL, rc2, krf, crf;
-    float rl;          // cutoff + skin: groups are listed when their centroids lie within rl + both radii
+    float rl;          // cutoff + skin: units are listed when their centroids lie within rl + both radii
     float half_skin2;  // (skin/2)^2: a centroid moved this far since the build invalidates the lists
     int pair_image;    // 1: cutoff + two radii may reach half the box; the force pass takes the
-                       // minimum image per pair (else one shift per listed group)
+                       // minimum image per pair (else one shift per listed unit)
 };
 struct FFDev {
-    int S, n_int, n_groups, n_cells;
+    int S, n_int, n_units, n_cells;
     const FFSys* sys;     // [S]
     const int* iatom;     // [n_int] device slot of each interacting atom
-    const int* isys;      // [n_int] its system
-    const float4* param;  // [n_int] sqrt(K) q, sigma/2, sqrt(epsilon), body id (int bits; 0 = free)
-    const int* grp_k0;    // [n_groups] first interacting atom of each group
-    const int* grp_n;     // [n_groups] its atoms
-    const int2* grp_kn;   // [n_groups] (grp_k0, grp_n) together: one load per listed group
-    const int* gsys;      // [n_groups] its system
-    const int* kgrp;      // [n_int] group of each interacting atom
-    float4* gcen;         // [n_groups] centroid (wrapped into the box) and radius, every evaluation
-    float4* gref;         // [n_groups] centroid at the last build
-    float4* gq;           // [n_groups] cell order: centroid and radius (list builds)
-    int* cell_of;         // [n_groups]
+    const float4* param;  // [n_int] sqrt(K) q, sigma/2, sqrt(epsilon), 0
+    const int2* unit;     // [n_units] u: first interacting atom; atoms | (atoms with LJ) << 8 (they come first)
+    const int* ugrp;      // [n_units] u: group (units of one group are never paired)
+    const int* usys;      // [n_units] system of u, and of place p
+    float4* ucen;         // [n_units] u: centroid (wrapped into the box) and radius, every evaluation
+    float4* uref;         // [n_units] u: centroid at the last build
+    int* place;           // [n_units] u -> p of the last build
+    int* unit_at;         // [n_units] p -> u
+    int* cell_of;         // [n_units] u
     int* cell_count;      // [n_cells], zero between evaluations
     int* cell_start;      // [n_cells + 1] (entry c0 + nc^3 of each system ends it)
     int* cell_cursor;     // [n_cells]
-    int* cell_list;       // [n_groups] group indices in cell order (of the last list build)
-    float4* cpos;         // [n_int] x, y, z (wrapped into the box), sqrt(K) q (or the atom's type)
-    double* e_group;      // [n_groups] half pair-energy sums of each group (energy evaluations)
-    // Neighbour lists of groups, rebuilt per system when one of its centroids has moved more than
+    float4* scen;         // [n_units] p: centroid and radius
+    int* sgrp;            // [n_units] p: group
+    // p: atom records x, y, z (at the image nearest the unit's centroid), type: record a of place p at
+    // spos[a][p] (a < slots; those past the unit's atoms lie far outside every cutoff)
+    float4* spos[kMaxUnit];
+    float4* spar[kMaxUnit];  // p: the atoms' parameters, likewise (more than kMaxTypes types only)
+    int slots;
+    double* e_unit;       // [n_units] u: half pair-energy sums (energy evaluations)
+    // Neighbour lists of units, rebuilt per system when one of its centroids has moved more than
     // half the skin since the last build, and for every system at the last evaluation of every
     // step call and at the first evaluation after a state is set
-    unsigned char* rebuild;  // [S] 1: rebuild this system's lists before the next force pass
+    unsigned char* rebuild;  // [S] rebuild this system's lists before the next force pass: 1 set by the
+                             // host, 2 by the displacement test
     unsigned int* rebuilds;  // [S] list builds of each system so far (a statistic)
-    unsigned int* nbr;       // entries: listed group - g0 of the system; entry e of group g at
-                             // g*cap + e
-    int* ncnt;               // [n_groups] entries per group
-    int cap;                 // entries per group allocated
+    unsigned int* nbr;       // entry e of place p at p * cap + e: the listed unit's place - u0
+    int* ncnt;               // [n_units] p: entries
+    int cap;                 // entries per unit allocated
     // Atom types (ntypes > 0): the distinct (sqrt(K) q, sigma/2, sqrt(epsilon)) of the interacting
-    // atoms; cpos .w then holds the atom's type (int bits) instead of its charge, so that the force
-    // pass reads one 16-byte record per neighbour, and takes each pair's (K q_i q_j, C12, C6) from
-    // a table of type pairs
+    // atoms; spos .w then holds the atom's type (int bits), and the force pass takes each pair's
+    // coefficients from a table of type pairs: entry (i, j) is K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j
     const float4* types;     // [ntypes * ntypes] the type-pair table
     const int* atype;        // [n_int] type of each interacting atom
     int ntypes;
@@ -151,24 +156,14 @@ struct FFDev {
     unsigned int* sys_status;  // [S] bit 0: a force of the system is non-finite or beyond the
                                // fixed-point range (never during a capped relaxation); bit 1: a list
                                // outgrew its capacity
-    int cell_threads;     // block size of the cell list-build kernel: 64, 128 (default) or 256
-    // work lists of the list builds (set with the state): every cell of the multi-cell boxes with
-    // its system, and every 64-group chunk (first group) of the single-cell boxes
-    int n_mc, n_sc;
+    int build_threads;    // block size of the list-build kernel: 64, 128 (default) or 256
+    // work list of the cell sort (set with the state): every cell of the multi-cell boxes with its system
+    int n_mc;
     const int* mc_cell;
     const int* mc_sys;
-    const int* sc_sys;
-    const int* sc_g0;
-    // groups of the force passes (set at creation, put in spatial order with the state), by size:
-    // at most 4, at most 8 and more than 8 interacting atoms (force_pass_of)
-    int n_pass[3];
-    const int* pass_groups[3];
 };
-// The force pass runs in three launches by group size: at most 4 interacting atoms (waters, free
-// atoms), at most 8 (tetrahedral bodies) and more (rings, larger bodies, in chunks of 12).
-constexpr int kForcePasses = 3;
-inline int force_pass_of(int atoms) { return atoms <= 4 ? 0 : atoms <= 8 ? 1 : 2; }
-// Interacting atoms of one system: the force pass streams (atom << 5 | lane) words.
+constexpr int kMaxTypes = 32;  // atom types of the type-pair table (FFDev::types)
+// Interacting atoms of one system (a limit of this interface: list entries are 32-bit words).
 constexpr int kMaxSystemAtoms = 1 << 26;
 int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* stream);
 // Fixed-point forces of slots [0, natoms) -> user-order doubles out[3*natoms] (kJ/mol/nm).
