@@ -75,6 +75,29 @@ template <class T> int upload_vec(DevArray<T>& a, const std::vector<T>& h) {
     return RBX_OK;
 }
 
+// Device storage of SystemChunks: systems of the given item counts in chunks of `size` (at least one
+// chunk each), `width` partial sums per chunk.
+struct ChunkStore {
+    DevArray<int2> chunk;
+    DevArray<int> chunk0;
+    DevArray<double> part;
+    int set(const std::vector<int>& items, int size, int width) {
+        std::vector<int2> c;
+        std::vector<int> c0;
+        for (int s = 0; s < (int)items.size(); s++) {
+            c0.push_back((int)c.size());
+            for (int i = 0; i == 0 || i < items[s]; i += size) c.push_back(make_int2(s, i));
+        }
+        c0.push_back((int)c.size());
+        int rc = upload_vec(chunk, c);
+        if (!rc) rc = upload_vec(chunk0, c0);
+        if (!rc && part.alloc(c.size() * width) != cudaSuccess) rc = set_error(RBX_ERR_CUDA, "cudaMalloc of partial sums failed");
+        return rc;
+    }
+    SystemChunks view() const { return SystemChunks{(int)chunk.n, chunk.p, chunk0.p, part.p}; }
+    size_t bytes() const { return chunk.bytes() + chunk0.bytes() + part.bytes(); }
+};
+
 }  // namespace
 
 struct rbx_batch {
@@ -99,6 +122,7 @@ struct rbx_batch {
     FFDev ff{};
     // per-system reductions
     DevArray<int> d_body0, d_free0;
+    ChunkStore ke_chunks, e_chunks;  // of bodies and free atoms, of units
     std::vector<int> body0_h, free0_h;  // host copies: library-order body / free-atom ranges per system
     DevArray<unsigned int> d_sys_status;  // [S] force-kernel failures (FFDev::sys_status)
     DevArray<double> d_ke, d_user;
@@ -476,6 +500,9 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     if (!rc) rc = upload_vec(b->d_unit, unit);
     if (!rc) rc = upload_vec(b->d_usys, usys);
     if (!rc) rc = upload_vec(b->d_ugrp, ugrp);
+    std::vector<int> units_of(num_systems);
+    for (int s = 0; s < num_systems; s++) units_of[s] = sys[s].u1 - sys[s].u0;
+    if (!rc) rc = b->e_chunks.set(units_of, kEnergyChunk, 1);
     // atom types: the distinct (scaled charge, sigma/2, sqrt(epsilon)) triples; with at most
     // kMaxTypes of them the force pass reads one 16-byte record per neighbour (position and type)
     // and takes each pair's coefficients from a table of type pairs
@@ -561,6 +588,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     }
     D.slots = slots;
     D.e_unit = b->d_e_unit.p;
+    D.e_chunks = b->e_chunks.view();
     D.energy = b->d_energy.p;
     D.fcap = 0.0f;
     D.sys_status = b->d_sys_status.p;
@@ -609,6 +637,11 @@ int rbx_batch_set_state(rbx_batch* b, void* stream, const double* positions, con
     std::vector<int> body0, free0;
     if ((rc = system_ranges(b->integ, b->offsets, body0, free0, b->dof))) return rc;
     if ((rc = upload_vec(b->d_body0, body0)) || (rc = upload_vec(b->d_free0, free0))) return rc;
+    if (!b->ke_chunks.chunk.n) {  // the counts are fixed at creation
+        std::vector<int> items(b->S);
+        for (int s = 0; s < b->S; s++) items[s] = body0[s + 1] - body0[s] + free0[s + 1] - free0[s];
+        if ((rc = b->ke_chunks.set(items, kKEChunk, 2))) return rc;
+    }
     b->body0_h = body0;
     b->free0_h = free0;
     BATCH_TRY(cudaMemsetAsync(b->d_sys_status.p, 0, sizeof(unsigned int) * (size_t)b->S, (cudaStream_t)stream));
@@ -728,10 +761,11 @@ int rbx_batch_energies(rbx_batch* b, void* stream, double* out) {
     if (!b->u_valid && ((rc = force_rebuild(b, stream)) || (rc = forces(b, stream, true)))) return rc;
     b->u_valid = true;
     b->f_valid = true;
-    if (launch_kinetic_systems(b->prec, device_system(b->integ), buffers(b), b->d_body0.p, b->d_free0.p, b->S,
-                               b->d_ke.p, stream) < 0)
+    const int launched = launch_kinetic_systems(b->prec, device_system(b->integ), buffers(b), b->d_body0.p, b->d_free0.p,
+                                                b->ke_chunks.view(), b->S, b->d_ke.p, stream);
+    if (launched < 0)
         return set_error(RBX_ERR_CUDA, "kinetic-energy kernel failed: %s", cudaGetErrorString(cudaGetLastError()));
-    b->last_launches += 1;
+    b->last_launches += launched;
     cudaStream_t st = (cudaStream_t)stream;
     BATCH_TRY(cudaMemcpyAsync(b->h_out, b->d_energy.p, sizeof(double) * b->S, cudaMemcpyDeviceToHost, st));
     BATCH_TRY(cudaMemcpyAsync(b->h_out + b->S, b->d_ke.p, sizeof(double) * 2 * b->S, cudaMemcpyDeviceToHost, st));
@@ -794,7 +828,8 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
                b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_spos.bytes() + b->d_spar.bytes() + b->d_mc_cell.bytes() +
                b->d_mc_sys.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_rebuild.bytes() + b->d_nbr.bytes() +
                b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_e_unit.bytes() + b->d_energy.bytes() +
-               b->d_body0.bytes() + b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes();
+               b->d_body0.bytes() + b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() +
+               b->ke_chunks.bytes() + b->e_chunks.bytes();
     *bytes = n + (b->integ ? device_bytes(b->integ) : 0);
     return RBX_OK;
 }

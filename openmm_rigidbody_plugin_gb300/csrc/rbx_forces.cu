@@ -29,8 +29,8 @@
 //   8. ff_force    one warp per unit (all systems): the unit's atoms in registers, each lane taking
 //                  one listed unit at a time; per-lane partial sums joined by a fixed butterfly, no
 //                  atomics; forces written as OpenMM fixed point (2^32) to the slots
-//   9. ff_energy   (energy evaluations only) one block per system: fixed-order FP64 sum of its
-//                  units' pair energies.
+//   9. ff_energy   (energy evaluations only) one block per 2048 units of a system, joined per
+//                  system: fixed-order FP64 sum of its units' pair energies.
 // The atoms of one group never meet in a list: pairs of one rigid body are excluded, as the
 // plugin's ForceField helper removes them (python/forcefield.py:131-138).
 #include <cuda_runtime.h>
@@ -617,18 +617,20 @@ template <int JS> void launch_force_pass(const FFDev& D, bool energy, long long*
     else launch_force_kernel<JS, false, false>(D, f, stride, st);
 }
 
-__global__ void ff_energy(FFDev D) {
+// One block per chunk of a system's units.
+__global__ void ff_energy(FFDev D, double* part) {
     __shared__ double s[256];
-    const FFSys S = D.sys[blockIdx.x];
+    const int2 c = D.e_chunks.chunk[blockIdx.x];
+    const int u0 = D.sys[c.x].u0 + c.y, u1 = min(u0 + kEnergyChunk, D.sys[c.x].u1);
     double e = 0.0;
-    for (int u = S.u0 + threadIdx.x; u < S.u1; u += blockDim.x) e += D.e_unit[u];
+    for (int u = u0 + (int)threadIdx.x; u < u1; u += blockDim.x) e += D.e_unit[u];
     s[threadIdx.x] = e;
     __syncthreads();
     for (int w = blockDim.x / 2; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) D.energy[blockIdx.x] = s[0];
+    if (threadIdx.x == 0) part[blockIdx.x] = s[0];
 }
 
 __global__ void forces_to_user(const long long* __restrict__ f, int stride, int n, double* __restrict__ out) {
@@ -674,8 +676,14 @@ int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* 
     }
     n++;
     if (energy) {
-        ff_energy<<<D.S, 256, 0, st>>>(D);
+        const SystemChunks& c = D.e_chunks;
+        double* part = c.n == D.S ? D.energy : c.part;  // every system one chunk: its sum is the result
+        ff_energy<<<c.n, 256, 0, st>>>(D, part);
         n++;
+        if (part != D.energy) {
+            if (launch_join_chunks(part, c.chunk0, D.S, 1, D.energy, stream) < 0) return -1;
+            n++;
+        }
     }
     return cudaPeekAtLastError() == cudaSuccess ? n : -1;
 }

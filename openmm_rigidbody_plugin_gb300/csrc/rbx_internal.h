@@ -92,6 +92,17 @@ struct DevBuf {
     int stride;
 };
 
+// Systems cut into chunks for per-system reductions: chunk c covers items from chunk[c].y of system
+// chunk[c].x, chunks [chunk0[s], chunk0[s + 1]) belong to system s; part holds each chunk's sums.
+struct SystemChunks {
+    int n;
+    const int2* chunk;
+    const int* chunk0;
+    double* part;
+};
+constexpr int kKEChunk = 512;       // bodies and free atoms per chunk of the kinetic energies
+constexpr int kEnergyChunk = 2048;  // units per chunk of the potential energies
+
 // Cutoff LJ + reaction-field force field over many independent cubic boxes (rbx_forces.cu).
 // Interacting atoms (non-zero charge or LJ epsilon) are listed system by system and, within a
 // system, body by body: the interacting atoms of one rigid body (or one free atom) form a group,
@@ -136,6 +147,7 @@ struct FFDev {
     float4* spar[kMaxUnit];  // p: the atoms' parameters, likewise (more than kMaxTypes types only)
     int slots;
     double* e_unit;       // [n_units] u: half pair-energy sums (energy evaluations)
+    SystemChunks e_chunks;  // of the units of each system
     // Neighbour lists of units, rebuilt per system when one of its centroids has moved more than
     // half the skin since the last build, and for every system at the last evaluation of every
     // step call and at the first evaluation after a state is set
@@ -283,8 +295,10 @@ int system_ranges(rbx_integrator* h, const std::vector<int>& slot_offsets, std::
 int launch_sync_positions(int prec, const DevSys& s, const DevBuf& b, void* stream);
 // Scale the body COM velocities and quaternion momenta and the free atoms' velocities.
 int launch_scale_momenta(int prec, const DevSys& s, const DevBuf& b, double factor, void* stream);
-// [KE_t, KE_r] of each system (out[2*S]), FP64, fixed order, one block per system.
+// [KE_t, KE_r] of each system (out[2*S]), FP64, fixed order.
 int launch_kinetic_systems(int prec, const DevSys& s, const DevBuf& b, const int* body0, const int* free0,
-                           int num_systems, double* out, void* stream);
+                           const SystemChunks& c, int num_systems, double* out, void* stream);
+// out[width * s + k] = sum over system s's chunks of part[width * c + k], fixed order.
+int launch_join_chunks(const double* part, const int* chunk0, int num_systems, int width, double* out, void* stream);
 
 }  // namespace rbx

@@ -102,29 +102,36 @@ __global__ void __launch_bounds__(kKEThreads) kinetic_kernel(DevSys S, DevBuf B,
     }
 }
 
-// [KE_t, KE_r] per system: one block per system over its library-order ranges of bodies and free
-// atoms, FP64, fixed-order tree.
+// [KE_t, KE_r] per system, FP64 in a fixed order: one block per chunk of kKEChunk items of a system
+// (its library-order range of bodies, then its free atoms), then a warp per system over its chunks.
+// Bound: the FP64 pipe (about 70 operations per body, two divisions' worth among them) and the latency
+// of a block's chain, so a large system is spread over the GPU: rbx_batch_energies of 66,666 bodies takes
+// 0.054 ms instead of 1.50 with one block per system, of 256 systems of 64 to 4096 bodies 0.106 instead
+// of 0.148. The chunks of a system do
+// not depend on the other systems.
 template <int P>
-__global__ void __launch_bounds__(kKEThreads) kinetic_systems_kernel(DevSys S, DevBuf B, const int* body0,
-                                                                     const int* free0, double* out) {
+__global__ void __launch_bounds__(kKEThreads) kinetic_chunks_kernel(DevSys S, DevBuf B, const int* body0, const int* free0,
+                                                                    const int2* chunk, double* part) {
     using V4 = typename Tr<P>::V4;
     __shared__ double s_t[kKEThreads], s_r[kKEThreads];
-    const int sys = blockIdx.x;
+    const int sys = chunk[blockIdx.x].x, first = chunk[blockIdx.x].y;
+    const int b0 = body0[sys], nb = body0[sys + 1] - b0, f0 = free0[sys];
+    const int end = min(first + kKEChunk, nb + free0[sys + 1] - f0);
     double kt = 0.0, kr = 0.0;
-    for (int b = body0[sys] + threadIdx.x; b < body0[sys + 1]; b += blockDim.x) {
-        V3<double> v, invI;
-        Q4<double> q, pi;
-        double invm;
-        BodyRead<P>::get(S, b, v, q, pi, invm, invI);
-        V3<double> L = qBt(q, pi) * 0.5;
-        kt += dot(v, v) / invm;
-        kr += dot(L, mul(invI, L));
-    }
-    const V4* vel = (const V4*)B.velm;
-    for (int j = free0[sys] + threadIdx.x; j < free0[sys + 1]; j += blockDim.x) {
-        V4 vm = vel[S.free_loc[j]];
-        double vx = vm.x, vy = vm.y, vz = vm.z;
-        kt += (vx * vx + vy * vy + vz * vz) / (double)vm.w;
+    for (int i = first + (int)threadIdx.x; i < end; i += blockDim.x) {
+        if (i < nb) {
+            V3<double> v, invI;
+            Q4<double> q, pi;
+            double invm;
+            BodyRead<P>::get(S, b0 + i, v, q, pi, invm, invI);
+            V3<double> L = qBt(q, pi) * 0.5;
+            kt += dot(v, v) / invm;
+            kr += dot(L, mul(invI, L));
+        } else {
+            const V4 vm = ((const V4*)B.velm)[S.free_loc[f0 + i - nb]];
+            const double vx = vm.x, vy = vm.y, vz = vm.z;
+            kt += (vx * vx + vy * vy + vz * vz) / (double)vm.w;
+        }
     }
     s_t[threadIdx.x] = kt;
     s_r[threadIdx.x] = kr;
@@ -137,8 +144,22 @@ __global__ void __launch_bounds__(kKEThreads) kinetic_systems_kernel(DevSys S, D
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        out[2 * sys] = 0.5 * s_t[0];
-        out[2 * sys + 1] = 0.5 * s_r[0];
+        part[2 * blockIdx.x] = 0.5 * s_t[0];
+        part[2 * blockIdx.x + 1] = 0.5 * s_r[0];
+    }
+}
+
+// Sums of `width` values per chunk over each system's chunks [chunk0[s], chunk0[s + 1]), a warp per
+// system, in a fixed order.
+__global__ void __launch_bounds__(256) join_chunks_kernel(const double* part, const int* chunk0, int num_systems, int width,
+                                                          double* out) {
+    const int s = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (s >= num_systems) return;
+    for (int k = 0; k < width; k++) {
+        double v = 0.0;
+        for (int c = chunk0[s] + lane; c < chunk0[s + 1]; c += 32) v += part[(size_t)width * c + k];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) out[(size_t)width * s + k] = v;
     }
 }
 
@@ -335,15 +356,22 @@ int launch_scale_momenta(int prec, const DevSys& s, const DevBuf& b, double fact
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
+int launch_join_chunks(const double* part, const int* chunk0, int num_systems, int width, double* out, void* stream) {
+    join_chunks_kernel<<<(num_systems + 7) / 8, 256, 0, (cudaStream_t)stream>>>(part, chunk0, num_systems, width, out);
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+}
+
 int launch_kinetic_systems(int prec, const DevSys& s, const DevBuf& b, const int* body0, const int* free0,
-                           int num_systems, double* out, void* stream) {
-    if (num_systems <= 0) return 0;
+                           const SystemChunks& c, int num_systems, double* out, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
+    // every system one chunk: its sums are the result
+    double* part = c.n == num_systems ? out : c.part;
     switch (prec) {
-        case PREC_SINGLE: kinetic_systems_kernel<PREC_SINGLE><<<num_systems, kKEThreads, 0, st>>>(s, b, body0, free0, out); break;
-        case PREC_MIXED: kinetic_systems_kernel<PREC_MIXED><<<num_systems, kKEThreads, 0, st>>>(s, b, body0, free0, out); break;
-        default: kinetic_systems_kernel<PREC_DOUBLE><<<num_systems, kKEThreads, 0, st>>>(s, b, body0, free0, out); break;
+        case PREC_SINGLE: kinetic_chunks_kernel<PREC_SINGLE><<<c.n, kKEThreads, 0, st>>>(s, b, body0, free0, c.chunk, part); break;
+        case PREC_MIXED: kinetic_chunks_kernel<PREC_MIXED><<<c.n, kKEThreads, 0, st>>>(s, b, body0, free0, c.chunk, part); break;
+        default: kinetic_chunks_kernel<PREC_DOUBLE><<<c.n, kKEThreads, 0, st>>>(s, b, body0, free0, c.chunk, part); break;
     }
+    if (part != out) return launch_join_chunks(part, c.chunk0, num_systems, 2, out, stream) < 0 ? -1 : 2;
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
