@@ -346,7 +346,17 @@ template <class T> int upload(DevArray<T>& a, const std::vector<T>& h) {
 // larger than one tile).
 // Greedy packing of the library order into tiles of at most TB bodies and TA body atoms.
 void pack_tiles(rbx_integrator* h) {
-    const int TA = tile_atoms(h->prec, h->tile_threads), TB = tile_bodies(h->prec, h->tile_threads), nb = h->nb;
+    // Bodies per tile: the kernel's limit, or fewer (whole warps) where that leaves SMs without a tile. A
+    // system that fits one wave of resident tiles (3 per SM; 6 of the narrow shape) is spread over all
+    // of it: the step is then a chain of latencies, shorter with fewer bodies per tile. Single/mixed,
+    // part1 + fused + part2: 333 bodies 30.4 -> 23.3 us, 21,017 bodies 34.8 -> 32.8; twice as many tiles
+    // than fit cost 45 us there. Double precision is bound by each SM's FP64 pipe, so more and smaller
+    // tiles even the SMs out as long as warps stay full: 50,118 bodies 606 us in tiles of up to 512
+    // atoms, 575 at 3 tiles per SM, 503 at 6, 822 in half-empty warps.
+    const int nb = h->nb, TA = tile_atoms(h->prec, h->tile_threads);
+    const int wave = h->prec == PREC_DOUBLE ? 6 * kSMs : 3 * kSMs * (kThreadsF / h->tile_threads);
+    const int per_tile = std::max(1, (nb + 32 * wave - 1) / (32 * wave)) * 32;
+    const int TB = std::min(tile_bodies(h->prec, h->tile_threads), per_tile);
     h->tile_body0.assign(1, 0);
     for (int L = 0; L < nb;) {
         int atoms = 0, cnt = 0;

@@ -49,6 +49,7 @@ constexpr int kTileAtomsD = 512;
 constexpr int kThreadsF = 256;
 constexpr int kThreadsFNarrow = 128;
 constexpr int kTileAtomsF = 4 * kThreadsF;
+constexpr int kSMs = 152;           // SMs of a GB300
 constexpr int kWarpBody = 32;       // bodies of more atoms are summed by a whole warp
 constexpr int kBconstRows = 11;     // rows of the FP32 body-constant table (single/mixed)
 constexpr int kRefBodyRows = 10;    // rows of ref_start per body
