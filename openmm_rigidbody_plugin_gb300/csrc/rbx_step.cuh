@@ -12,7 +12,8 @@
 //   1. one thread per atom gathers the fixed-point force, rebuilds the COM displacement
 //      delta = At(q) d and its torque delta x F, and parks F and tau in shared memory;
 //      (single/mixed: phase 1's loads are issued before phase 0, so that the slot -> force
-//      dependency overlaps it: 4 % faster)
+//      dependency overlaps it: 4 % faster; slots and body-frame coordinates, which no kernel
+//      writes between steps, even before the wait for the kernel before, rbx_launch.cuh)
 //   2. one thread per body sums its atoms' F and tau in a fixed order (deterministic, no
 //      atomics; a whole warp per body for bodies of more than 32 atoms), applies the half
 //      kick(s), drift and free rotation, and writes its state;
@@ -31,6 +32,7 @@
 
 #include "rbx_fast.cuh"
 #include "rbx_internal.h"
+#include "rbx_launch.cuh"
 #include "rbx_math.cuh"
 #include "rbx_tiles.h"
 
@@ -82,8 +84,9 @@ template <> __device__ __forceinline__ float fixed_to<float>(long long v) {
 }
 template <> __device__ __forceinline__ double fixed_to<double>(long long v) { return __ll2double_rn(v) * 0x1p-32; }
 
-template <class T> __device__ __forceinline__ V3<T> load_force(const long long* __restrict__ f, int loc, int stride) {
-    return v3<T>(fixed_to<T>(__ldg(f + loc)), fixed_to<T>(__ldg(f + loc + stride)), fixed_to<T>(__ldg(f + loc + 2 * stride)));
+// (through L2: the kernel before wrote it, so not by the read-only path, and each is read once)
+template <class T> __device__ __forceinline__ V3<T> load_force(const long long* f, int loc, int stride) {
+    return v3<T>(fixed_to<T>(__ldcg(f + loc)), fixed_to<T>(__ldcg(f + loc + stride)), fixed_to<T>(__ldcg(f + loc + 2 * stride)));
 }
 
 template <class To, class From> __device__ __forceinline__ V3<To> cvt(V3<From> a) {
@@ -228,7 +231,7 @@ __device__ __forceinline__ bool free_atom_ff(const DevBuf& B, double dt_d, int l
         !ff_from_double(vm.w, w) || !ff_from_double(dt_d, dt))
         return false;
     const ff wh = ff_mul(w, ff{0.5f * dt.hi, 0.5f * dt.lo});  // (1/m) dt/2; halving is exact
-    const long long f[3] = {__ldg(B.force + loc), __ldg(B.force + loc + B.stride), __ldg(B.force + loc + 2 * B.stride)};
+    const long long f[3] = {__ldcg(B.force + loc), __ldcg(B.force + loc + B.stride), __ldcg(B.force + loc + 2 * B.stride)};
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         const ff dv = ff_mul(fixed_to_ff(f[c]), wh);
@@ -266,8 +269,9 @@ __device__ __forceinline__ void free_atom_tile(const DevSys& S, const DevBuf& B,
     using V4 = typename Tr<P>::V4;
     using RS = typename Tr<P>::RS;
     const int j = ft * (int)blockDim.x + (int)threadIdx.x;
+    const int loc = j < S.nf ? __ldg(S.free_loc + j) : 0;
+    chain_wait();
     if (j >= S.nf) return;
-    const int loc = __ldg(S.free_loc + j);
     if constexpr (P == PREC_MIXED && !REF) {
         double vsum = 0.0;
         if (free_atom_ff<KIND>(B, dt, loc, vsum)) {
@@ -474,6 +478,7 @@ template <int KIND, bool EXACT, bool REF, bool LARGE>
 __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel_d(DevSys S, DevBuf B, double dt) {
     constexpr int P = PREC_DOUBLE;
     constexpr int TA = kTileAtomsD, TB = kTileBodies;
+    chain_release();
     const int tile = block_tile(S);
     if (tile < 0) {
         free_atom_tile<P, KIND, REF>(S, B, dt, -1 - tile);
@@ -487,7 +492,8 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
     const int nbt = b1 - b0;
     const int a0 = __ldg(S.atom0 + b0), nat = __ldg(S.atom0 + b1) - a0;
     const int nbp = S.nb_pad;
-    double* __restrict__ st = (double*)S.state;
+    double* st = (double*)S.state;
+    chain_wait();
 
     bool big = false;
     if (tid < nbt) {
@@ -642,6 +648,7 @@ template <int P, int KIND, bool EXACT, bool REF, int NT, bool LARGE>
 __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B, double dt_d) {
     using FSmem = rbx::FSmem<NT>;
     constexpr int APT = 4;  // body atoms per thread in phase 1
+    chain_release();
     const int tile = block_tile(S);
     if (tile < 0) {
         free_atom_tile<P, KIND, REF>(S, B, dt_d, -1 - tile);
@@ -660,8 +667,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
     const int nbt = b1 - b0;
     const int a0 = __ldg(S.atom0 + b0), nat = __ldg(S.atom0 + b1) - a0;
     const int nbp = S.nb_pad;
-    float* __restrict__ ghi = (float*)S.state;  // state rows 0..13 (hi)
-    float* __restrict__ glo = ghi + 14 * nbp;   // rows 14..27 (lo)
+    float* ghi = (float*)S.state;  // state rows 0..13 (hi)
+    float* glo = ghi + 14 * nbp;   // rows 14..27 (lo)
     const float dt = (float)dt_d;
 
     // Phase 1 loads first (slots, body-frame coordinates; the orientation; then the forces at the
@@ -687,9 +694,13 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
         int s0 = 0, e0 = 0;
         if (tid < nbt) {
             const int b = b0 + tid;
-            q0 = q4<float>(ghi[b + 6 * nbp], ghi[b + 7 * nbp], ghi[b + 8 * nbp], ghi[b + 9 * nbp]);
             s0 = __ldg(S.atom0 + b) - a0;
             e0 = __ldg(S.atom0 + b + 1) - a0;
+        }
+        chain_wait();  // state, forces and positions from here on
+        if (tid < nbt) {
+            const int b = b0 + tid;
+            q0 = q4<float>(ghi[b + 6 * nbp], ghi[b + 7 * nbp], ghi[b + 8 * nbp], ghi[b + 9 * nbp]);
         }
 #pragma unroll
         for (int i = 0; i < APT; i++) {
@@ -943,8 +954,7 @@ int launch_step_nt(const DevSys& s, const DevBuf& b, double dt, cudaStream_t str
     }
     const int tiles = s.n_body_tiles + s.n_free_tiles;
     if (tiles == 0) return 0;
-    kernel<<<tiles, threads, smem, stream>>>(s, b, dt);
-    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+    return launch_chained(kernel, tiles, threads, smem, stream, s, b, dt) == cudaSuccess ? 1 : -1;
 }
 
 // The kernel for the integrator's bodies (any of more than kWarpBody atoms: the LARGE form) and,
