@@ -411,15 +411,14 @@ int rbx_batch_set_graph_steps(rbx_batch* b, int k);
  *   1. the step kernel's tile shape (rbx_set_tile_threads: 256 or 128 threads, single/mixed
  *      precision with bodies of at most 32 atoms), by the integrator launches' own event times
  *      over 2 x trial_steps steps after an untimed run of trial_steps;
- *   2. the block size of the list-build kernel (64, 128 or 256 threads);
- *   3. where a step takes under 1 ms, so that launch overhead matters, the steps per captured graph
- *      (0, 10 or 50).
- * Trials 2 and 3 run trial_steps steps (2k+1 for a graph of k) twice and time the second run with
- * CUDA events. It keeps the fastest of each, and then restores the batch's exact state
- * (rbx_batch_restore): no choice changes any result, since each body is integrated alike in any
- * tile, each unit's list (and so each atom's force sum) keeps its order, and graphs replay the
+ *   2. where a step takes under 1 ms, so that launch overhead matters, the steps per captured graph
+ *      (0, 10 or 50): trial_steps steps (2k+1 for a graph of k) run twice, the second run timed with
+ *      CUDA events.
+ * It keeps the fastest of each, and then restores the batch's exact state (rbx_batch_restore): no
+ * choice changes any result, since each body is integrated alike in any tile, and graphs replay the
  * same launches.
- * chosen[2] (optional) receives the block size and the graph run length; rbx_batch_get_tile_threads
+ * chosen[2] (optional) receives the list-build block size (64, 128 or 256; lists are built by the force
+ * pass, so it no longer changes the schedule) and the graph run length; rbx_batch_get_tile_threads
  * the tile shape. rbx_batch_set_tuning and rbx_batch_set_tile_threads set them by hand. */
 int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, int* chosen);
 int rbx_batch_set_tuning(rbx_batch* b, int cell_threads, int graph_steps);

@@ -106,11 +106,11 @@ struct rbx_batch {
     std::vector<int> offsets;
     // force field
     DevArray<FFSys> d_sys;
-    DevArray<int> d_iatom, d_ugrp, d_usys, d_place, d_unit_at, d_cell_of, d_cell_count, d_cell_start, d_cell_cursor;
+    DevArray<int> d_iatom, d_ugrp, d_usys, d_place, d_unit_at, d_cell_count, d_cell_start, d_cell_cursor;
     DevArray<int> d_sgrp, d_mc_cell, d_mc_sys, d_ncnt, d_atype;
     DevArray<int2> d_unit;
     DevArray<float4> d_param, d_ucen, d_uref, d_scen, d_spos, d_spar, d_types;
-    DevArray<unsigned char> d_rebuild;  // FFDev::rebuild
+    DevArray<unsigned char> d_moved, d_build;
     DevArray<unsigned int> d_nbr;       // neighbour lists of units (FFDev::nbr)
     DevArray<unsigned int> d_rebuilds;  // list builds per system (FFDev::rebuilds)
     // host copies for the set-up with a state: systems, cells allocated per system, unit layout
@@ -140,6 +140,7 @@ struct rbx_batch {
     std::vector<std::pair<int, int>> ev_marks;  // (start event, end event) per group
     std::vector<int> ev_kind;                   // 0 = forces, 1 = integrator
     int ev_used = 0;
+    int list_threads = 128;  // rbx_batch_set_tuning's block size: lists are built by the force pass now
     int graph_k = 0;
     int graph_launches = 0;  // kernels in one replay of the graph
     double graph_dt = 0.0;
@@ -203,6 +204,7 @@ int setup_lists(rbx_batch* b, const double* x) {
         rho[s] = std::sqrt(rho_max);
     });
     double cap_need = 1.0;
+    long long most_units = 0, most_cells = 0;
     for (int s = 0; s < S; s++) {
         FFSys& f = sys[s];
         const double L = b->box_h[s], rho_max = rho[s];
@@ -219,6 +221,8 @@ int setup_lists(rbx_batch* b, const double* x) {
                 mc_sys.push_back(s);
             }
         const int U = f.u1 - f.u0;
+        most_units = std::max<long long>(most_units, U);
+        most_cells = std::max<long long>(most_cells, (long long)nc * nc * nc);
         const double reach = (double)f.rl + 2.0 * rho_max;
         const double expect = 4.18879 * reach * reach * reach * (double)U / (L * L * L);
         cap_need = std::max(cap_need, std::min((double)std::max(U - 1, 1), 1.35 * expect + 32.0));
@@ -232,8 +236,10 @@ int setup_lists(rbx_batch* b, const double* x) {
         BATCH_TRY(cudaMemcpy(b->d_mc_cell.p, mc_cell.data(), sizeof(int) * mc_cell.size(), cudaMemcpyHostToDevice));
         BATCH_TRY(cudaMemcpy(b->d_mc_sys.p, mc_sys.data(), sizeof(int) * mc_sys.size(), cudaMemcpyHostToDevice));
     }
-    BATCH_TRY(cudaMemset(b->d_rebuild.p, 1, (size_t)S));
     FFDev& D = b->ff;
+    const bool small = prep_limit(most_units, most_cells);
+    D.prep_units = small ? (int)most_units : 0;
+    D.prep_cells = small ? (int)most_cells : 0;
     D.n_mc = (int)mc_cell.size();
     D.cap = cap;
     D.nbr = b->d_nbr.p;
@@ -297,18 +303,15 @@ struct Timed {
     }
 };
 
-// Marks every system's lists for a rebuild at the next evaluation. Forces and energies at the state a
-// call starts or ends in are formed from lists built at that state, so they are a function of the
-// positions alone (not of when earlier calls last rebuilt); the evaluations in between rebuild a
-// system's lists when its atoms have moved half the skin.
-int force_rebuild(rbx_batch* b, void* stream) {
-    BATCH_TRY(cudaMemsetAsync(b->d_rebuild.p, 1, (size_t)b->S, (cudaStream_t)stream));
-    return RBX_OK;
-}
-
-int forces(rbx_batch* b, void* stream, bool energy) {
+// One force evaluation. `rebuild` rebuilds every system's lists at the current positions: forces and
+// energies at the state a call starts or ends in are formed so, as a function of the positions alone
+// (not of when earlier calls last rebuilt); the evaluations in between rebuild a system's lists when
+// one of its units has moved half the skin.
+int forces(rbx_batch* b, void* stream, bool energy, bool rebuild) {
     Timed t(b, stream, 0);
-    const int n = launch_forces(b->ff, b->prec, buffers(b), energy, stream);
+    FFDev D = b->ff;
+    D.force_all = rebuild;
+    const int n = launch_forces(D, b->prec, buffers(b), energy, stream);
     if (n < 0) return set_error(RBX_ERR_CUDA, "force kernels failed: %s", cudaGetErrorString(cudaGetLastError()));
     b->last_launches += n;
     return RBX_OK;
@@ -336,7 +339,7 @@ int capture(rbx_batch* b, double dt) {
     int rc = RBX_OK;
     const int before = b->last_launches;
     for (int i = 0; i < b->graph_k && !rc; i++) {
-        rc = forces(b, b->cap_stream, false);
+        rc = forces(b, b->cap_stream, false, false);
         if (!rc) rc = fused(b, b->cap_stream, dt);
     }
     b->graph_launches = b->last_launches - before;
@@ -538,7 +541,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     if (!rc) rc = upload_vec(b->d_atype, type_of);
     const size_t u1 = std::max(nunit, 1), records = u1 * slots;
     if (!rc && (b->d_place.alloc(u1) != cudaSuccess || b->d_unit_at.alloc(u1) != cudaSuccess ||
-                b->d_cell_of.alloc(u1) != cudaSuccess || b->d_ucen.alloc(u1) != cudaSuccess ||
+                b->d_ucen.alloc(u1) != cudaSuccess ||
                 b->d_uref.alloc(u1) != cudaSuccess || b->d_scen.alloc(u1) != cudaSuccess ||
                 b->d_sgrp.alloc(u1) != cudaSuccess || b->d_ncnt.alloc(u1) != cudaSuccess ||
                 b->d_spos.alloc(records) != cudaSuccess || b->d_spar.alloc(types.empty() ? records : 0) != cudaSuccess ||
@@ -548,11 +551,13 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
                 b->d_mc_sys.alloc(std::max(cells, 1)) != cudaSuccess ||
                 b->d_energy.alloc(num_systems) != cudaSuccess || b->d_ke.alloc(2 * (size_t)num_systems) != cudaSuccess ||
                 b->d_user.alloc(3 * (size_t)N) != cudaSuccess || b->d_sys_status.alloc(num_systems) != cudaSuccess ||
-                b->d_rebuild.alloc(num_systems) != cudaSuccess || b->d_rebuilds.alloc(num_systems) != cudaSuccess))
+                b->d_moved.alloc(num_systems) != cudaSuccess || b->d_build.alloc(num_systems) != cudaSuccess ||
+                b->d_rebuilds.alloc(num_systems) != cudaSuccess))
         rc = set_error(RBX_ERR_CUDA, "cudaMalloc of force-field arrays failed");
     if (!rc && (cudaMemset(b->d_sys_status.p, 0, sizeof(unsigned int) * (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_cell_count.p, 0, sizeof(int) * (size_t)cells) != cudaSuccess ||
-                cudaMemset(b->d_rebuild.p, 1, (size_t)num_systems) != cudaSuccess ||
+                cudaMemset(b->d_moved.p, 0, (size_t)num_systems) != cudaSuccess ||
+                cudaMemset(b->d_build.p, 0, (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_rebuilds.p, 0, sizeof(unsigned int) * (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_ncnt.p, 0, sizeof(int) * u1) != cudaSuccess ||
                 cudaMemset(b->d_place.p, 0, sizeof(int) * u1) != cudaSuccess ||
@@ -576,7 +581,6 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.uref = b->d_uref.p;
     D.place = b->d_place.p;
     D.unit_at = b->d_unit_at.p;
-    D.cell_of = b->d_cell_of.p;
     D.cell_count = b->d_cell_count.p;
     D.cell_start = b->d_cell_start.p;
     D.cell_cursor = b->d_cell_cursor.p;
@@ -592,7 +596,9 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.energy = b->d_energy.p;
     D.fcap = 0.0f;
     D.sys_status = b->d_sys_status.p;
-    D.rebuild = b->d_rebuild.p;
+    D.force_all = 0;
+    D.moved = b->d_moved.p;
+    D.build = b->d_build.p;
     D.rebuilds = b->d_rebuilds.p;
     D.nbr = nullptr;  // allocated with the state (its capacity follows the units' radii)
     D.ncnt = b->d_ncnt.p;
@@ -600,7 +606,8 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.types = b->d_types.p;
     D.atype = b->d_atype.p;
     D.ntypes = (int)types.size();
-    D.build_threads = 128;
+    D.prep_units = 0;
+    D.prep_cells = 0;
     D.n_mc = 0;
     D.mc_cell = b->d_mc_cell.p;
     D.mc_sys = b->d_mc_sys.p;
@@ -693,7 +700,7 @@ int rbx_batch_step(rbx_batch* b, void* stream, int nsteps, double dt) {
     // changed the state since (formed, as an evaluation here would form them, from lists built at
     // these positions with the energy variant), else one evaluation. The reference likewise keeps
     // the forces of the last step for the next one (CudaRigidBodyKernels.cpp:421-426).
-    if (!b->f_valid && ((rc = force_rebuild(b, stream)) || (rc = forces(b, stream, true)))) return rc;
+    if (!b->f_valid && (rc = forces(b, stream, true, true))) return rc;
     b->f_valid = false;
     b->u_valid = false;
     if ((rc = integrate(b, stream, STEP_PART1, dt))) return rc;
@@ -709,11 +716,11 @@ int rbx_batch_step(rbx_batch* b, void* stream, int nsteps, double dt) {
         }
     }
     for (; remaining > 0; remaining--) {
-        if ((rc = forces(b, stream, false)) || (rc = fused(b, stream, dt))) return rc;
+        if ((rc = forces(b, stream, false, false)) || (rc = fused(b, stream, dt))) return rc;
     }
     // the last evaluation builds every list at the final positions and also forms their potential
     // energy
-    if ((rc = force_rebuild(b, stream)) || (rc = forces(b, stream, true))) return rc;
+    if ((rc = forces(b, stream, true, true))) return rc;
     if ((rc = integrate(b, stream, STEP_PART2, dt))) return rc;
     b->u_valid = true;
     b->f_valid = true;
@@ -735,9 +742,8 @@ int rbx_batch_relax(rbx_batch* b, void* stream, int nsteps, double dt, double ma
     b->ff.fcap = (float)max_force;
     b->u_valid = false;
     b->f_valid = false;
-    if ((rc = force_rebuild(b, stream))) return rc;
     for (int n = 0; n < nsteps && !rc; n++) {
-        rc = forces(b, stream, false);
+        rc = forces(b, stream, false, n == 0);
         if (!rc && launch_scale_momenta(b->prec, sys, buffers(b), damping, stream) < 0)
             rc = set_error(RBX_ERR_CUDA, "momentum damping failed");
         if (!rc) rc = rbx_integrate_part1(b->integ, stream, &rb, dt);
@@ -758,7 +764,7 @@ int rbx_batch_energies(rbx_batch* b, void* stream, double* out) {
     b->last_launches = 0;
     // the potential energy of the last step call's final positions when it is still current (formed
     // in that call's last force evaluation); otherwise a force evaluation that forms it
-    if (!b->u_valid && ((rc = force_rebuild(b, stream)) || (rc = forces(b, stream, true)))) return rc;
+    if (!b->u_valid && (rc = forces(b, stream, true, true))) return rc;
     b->u_valid = true;
     b->f_valid = true;
     const int launched = launch_kinetic_systems(b->prec, device_system(b->integ), buffers(b), b->d_body0.p, b->d_free0.p,
@@ -784,7 +790,7 @@ int rbx_batch_forces(rbx_batch* b, void* stream, double* forces_out, double* ene
     if (!b->d_body0.p) return set_error(RBX_ERR_STATE, "no state: call rbx_batch_set_state first");
     BATCH_TRY(cudaSetDevice(b->device));
     b->last_launches = 0;
-    if ((rc = force_rebuild(b, stream)) || (rc = forces(b, stream, true))) return rc;
+    if ((rc = forces(b, stream, true, true))) return rc;
     b->u_valid = true;
     b->f_valid = true;
     cudaStream_t st = (cudaStream_t)stream;
@@ -824,9 +830,9 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
     if (!bytes) return set_error(RBX_ERR_INVALID_ARGUMENT, "null output");
     size_t n = b->d_sys.bytes() + b->d_iatom.bytes() + b->d_param.bytes() + b->d_unit.bytes() + b->d_ugrp.bytes() +
                b->d_usys.bytes() + b->d_ucen.bytes() + b->d_uref.bytes() + b->d_place.bytes() + b->d_unit_at.bytes() +
-               b->d_cell_of.bytes() + b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
+               b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
                b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_spos.bytes() + b->d_spar.bytes() + b->d_mc_cell.bytes() +
-               b->d_mc_sys.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_rebuild.bytes() + b->d_nbr.bytes() +
+               b->d_mc_sys.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() + b->d_build.bytes() + b->d_nbr.bytes() +
                b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_e_unit.bytes() + b->d_energy.bytes() +
                b->d_body0.bytes() + b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() +
                b->ke_chunks.bytes() + b->e_chunks.bytes();
@@ -901,7 +907,7 @@ int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, i
         return r;
     };
     const int k0 = b->graph_k;
-    int best_ct = b->ff.build_threads, best_k = k0;
+    int best_k = k0;
     float best = 0.0f, ms = 0.0f;
     b->graph_k = 0;
     b->drop_graph();
@@ -931,17 +937,8 @@ int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, i
         const int rc1 = rbx_set_tile_threads(b->integ, best_nt);
         if (!rc) rc = rc1;
     }
-    // 2. block size of the list-build kernel, direct launches
-    const int cts[3] = {64, 128, 256};
-    for (int i = 0; i < 3 && !rc; i++) {
-        b->ff.build_threads = cts[i];
-        if ((rc = per_step(trial_steps, ms))) break;
-        if (i == 0 || ms < best) {
-            best = ms;
-            best_ct = cts[i];
-        }
-    }
-    b->ff.build_threads = best_ct;
+    // 2. one step, direct launches
+    if (!rc) rc = per_step(trial_steps, best);
     // 3. steps per captured graph, where launch overhead matters (steps under 1 ms)
     if (!rc && best < 1.0f) {
         const int ks[3] = {0, 10, 50};
@@ -970,7 +967,7 @@ int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, i
     if (rc) return rc;
     if (rc2) return rc2;
     if (chosen) {
-        chosen[0] = best_ct;
+        chosen[0] = b->list_threads;
         chosen[1] = best_k;
     }
     return RBX_OK;
@@ -998,8 +995,7 @@ int rbx_batch_set_tuning(rbx_batch* b, int cell_threads, int graph_steps) {
     if (cell_threads != 64 && cell_threads != 128 && cell_threads != 256)
         return set_error(RBX_ERR_INVALID_ARGUMENT, "cell kernel block size must be 64, 128 or 256");
     if ((rc = rbx_batch_set_graph_steps(b, graph_steps))) return rc;
-    if (cell_threads != b->ff.build_threads) b->drop_graph();
-    b->ff.build_threads = cell_threads;
+    b->list_threads = cell_threads;
     return RBX_OK;
 }
 

@@ -13,24 +13,22 @@
 // list ages only as the centroids move: each system rebuilds its lists when one of its centroids has
 // moved half the skin since its last build, and every list is rebuilt for the state a call starts or
 // ends in (so the forces there depend only on the positions, never on when earlier calls rebuilt).
-// One evaluation, all systems at once:
-//   1. ff_check    one thread per unit: its centroid and radius, the centroid's displacement since
-//                  the last build (flags the system's rebuild) and, for lists that stay, its atoms'
-//                  records at its place in cell order
-//   then, for the flagged systems only (the kernels return at once for the others):
-//   2. ff_bin      cell of each unit's centroid and cell counts, cells of at least cutoff + skin
-//                  + twice the largest radius per edge
-//   3. ff_scan     one block per system: exclusive scan of its cells' counts (and count reset)
-//   4. ff_scatter  slot in its cell (single-cell systems keep their unit order, no atomics)
-//   5. ff_sort     one warp per cell of a multi-cell box: sorts the cell by unit index
-//   6. ff_place    every unit's place, and its records there
-//   7. ff_build    one warp per unit: the units in range among the 27 cells around it (or, in a
-//                  single-cell box, all units by minimum image), in place order, into its list
-//   8. ff_force    one warp per unit (all systems): the unit's atoms in registers, each lane taking
-//                  one listed unit at a time; per-lane partial sums joined by a fixed butterfly, no
-//                  atomics; forces written as OpenMM fixed point (2^32) to the slots
-//   9. ff_energy   (energy evaluations only) one block per 2048 units of a system, joined per
-//                  system: fixed-order FP64 sum of its units' pair energies.
+// One evaluation, all systems at once. Batches whose systems are all small (prep_limit) take
+//   ff_prep     one block per system: each unit's centroid, radius and displacement since the last
+//               build; lists that stay get their atoms' records at their places in cell order, the
+//               others a new cell order first (cells of at least cutoff + skin + twice the largest
+//               radius per edge, counted, scanned and sorted in shared memory)
+// and the others the same in kernels over all units (ff_check, ff_bin, ff_scan, ff_scatter, ff_sort,
+// ff_place; those after ff_check return at once for systems whose lists stay). Then
+//   ff_force    one warp per unit (all systems). Where the lists are to be rebuilt the warp first
+//               builds its own: the units in range among the 27 cells around it (or, in a
+//               single-cell box, all units by minimum image), in place order. Then the forces: the
+//               unit's atoms in registers, each lane taking one listed unit at a time; per-lane
+//               partial sums joined by a fixed butterfly, no atomics; forces written as OpenMM fixed
+//               point (2^32) to the slots
+//   ff_energy   (energy evaluations only) one block per 2048 units of a system, joined per system:
+//               fixed-order FP64 sum of its units' pair energies.
+// All are launched as a chain (rbx_launch.cuh).
 // The atoms of one group never meet in a list: pairs of one rigid body are excluded, as the
 // plugin's ForceField helper removes them (python/forcefield.py:131-138).
 #include <cuda_runtime.h>
@@ -38,6 +36,7 @@
 #include <cstdint>
 
 #include "rbx_internal.h"
+#include "rbx_launch.cuh"
 
 namespace rbx {
 
@@ -118,10 +117,129 @@ __device__ __forceinline__ void write_place(const FFDev& D, int p, int k0, int n
     }
 }
 
-// 1. Per unit: centroid, radius and the rebuild test. A system that the host has marked gets its
-// records with its new places (ff_place).
+// Cell of a centroid in its system.
+__device__ __forceinline__ int cell_index(const FFSys& S, float4 c) {
+    return (wrap_cell(c.z, S.invL, S.nc) * S.nc + wrap_cell(c.y, S.invL, S.nc)) * S.nc + wrap_cell(c.x, S.invL, S.nc);
+}
+
+// Key of a unit in the order within its cell: its place on a 4 x 4 x 4 grid of the cell in Z-order,
+// then its index, so that the units a list takes of one cell lie in short runs of places and a run of
+// places is compact.
+constexpr unsigned int kKeyUnit = (1u << 26) - 1;
+__device__ __forceinline__ unsigned int cell_key(const FFSys& S, float4 c, int u) {
+    const float x[3] = {c.x, c.y, c.z};
+    unsigned int z = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int g = (int)(x[k] * S.invL * (float)(4 * S.nc)) & 3;
+        z |= (unsigned int)((g & 1) << k | (g >> 1) << (3 + k));
+    }
+    return z << 26 | (unsigned int)(u - S.u0);
+}
+
+__device__ __forceinline__ bool moved_too_far(const FFDev& D, const FFSys& S, int u, float4 c) {
+    const float4 r = D.uref[u];
+    const float3 d = min_image(c.x - r.x, c.y - r.y, c.z - r.z, S);
+    return fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) > S.half_skin2;
+}
+
+// Unit u at its new place p: records, group, build centroid.
+__device__ __forceinline__ void settle(const FFDev& D, const DevBuf& B, int prec, const FFSys& S, int u, int p) {
+    const int2 kn = D.unit[u];
+    const int k0 = kn.x, n = kn.y & 0xff;
+    float3 x[kMaxUnit];
+    const float4 c = unit_centroid(D, B, prec, S, k0, n, x);
+    write_place(D, p, k0, n, c, x);
+    if (!D.ntypes)
+        for (int a = 0; a < D.slots; a++) D.spar[a][p] = a < n ? D.param[k0 + a] : make_float4(0.f, 0.f, 0.f, 0.f);
+    D.place[u] = p;
+    D.unit_at[p] = u;
+    D.sgrp[p] = D.ugrp[u];
+    D.uref[u] = c;
+}
+
+// Everything before the force pass for one system, in one block. The cell counts and the keys of the
+// system's units, in cell order, are in shared memory. Within a cell units are ranked by key (all
+// different), so the order does not depend on the order of the atomics.
+// Bound: latency (a chain of dependent loads, and in rebuilds a dozen barriers), so one launch in place
+// of six. Per 20 steps with energies and a frame: 512 waters 539 against 623 us in separate kernels, 24
+// boxes of 64 to 190 bodies 708 against 832.
+__global__ void __launch_bounds__(1024) ff_prep(FFDev D, DevBuf B, int prec) {
+    extern __shared__ unsigned int keys[];  // prep_units
+    __shared__ int wsum[32];
+    int* cell = (int*)(keys + D.prep_units);  // prep_cells
+    const int s = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
+    chain_release();
+    const FFSys S = D.sys[s];
+    chain_wait();
+    bool build = D.force_all;
+    for (int u = S.u0 + tid; u < S.u1; u += nthr) {
+        const int2 kn = D.unit[u];
+        const int k0 = kn.x, n = kn.y & 0xff;
+        float3 x[kMaxUnit];
+        const float4 c = unit_centroid(D, B, prec, S, k0, n, x);
+        D.ucen[u] = c;
+        if (D.force_all) continue;
+        write_place(D, D.place[u], k0, n, c, x);
+        build |= moved_too_far(D, S, u, c);
+    }
+    build = __syncthreads_or(build);
+    if (tid == 0) {
+        D.build[s] = build;
+        if (build) D.rebuilds[s]++;
+    }
+    if (!build) return;
+    if (S.nc == 1) {  // one cell: unit order
+        for (int u = S.u0 + tid; u < S.u1; u += nthr) settle(D, B, prec, S, u, u);
+        return;
+    }
+    const int ncell = S.nc * S.nc * S.nc, units = S.u1 - S.u0;
+    for (int i = tid; i < ncell; i += nthr) cell[i] = 0;
+    __syncthreads();
+    for (int u = S.u0 + tid; u < S.u1; u += nthr) atomicAdd(cell + cell_index(S, D.ucen[u]), 1);
+    __syncthreads();
+    // exclusive scan of the counts: each thread a run of cells, the runs' sums by warp shuffles
+    const int per = (ncell + nthr - 1) / nthr, i0 = min(tid * per, ncell), i1 = min(i0 + per, ncell);
+    int sum = 0;
+    for (int i = i0; i < i1; i++) sum += cell[i];
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((tid & 31) >= o) incl += v;
+    }
+    if ((tid & 31) == 31) wsum[tid >> 5] = incl;
+    __syncthreads();
+    int at = incl - sum;
+    for (int w = 0; w < (tid >> 5); w++) at += wsum[w];
+    for (int i = i0; i < i1; i++) {
+        const int n = cell[i];
+        cell[i] = at;
+        D.cell_start[S.c0 + i] = S.u0 + at;
+        at += n;
+    }
+    if (tid == 0) D.cell_start[S.c0 + ncell] = S.u1;
+    __syncthreads();
+    for (int u = S.u0 + tid; u < S.u1; u += nthr) {
+        const float4 c = D.ucen[u];
+        keys[atomicAdd(cell + cell_index(S, c), 1)] = cell_key(S, c, u);
+    }
+    __syncthreads();  // cell[i] is now the end of cell i
+    for (int i = tid; i < units; i += nthr) {
+        const unsigned int key = keys[i];
+        const int u = S.u0 + (int)(key & kKeyUnit), c = cell_index(S, D.ucen[u]);
+        const int b = c ? cell[c - 1] : 0, e = cell[c];
+        int rank = 0;
+        for (int j = b; j < e; j++) rank += keys[j] < key;
+        settle(D, B, prec, S, u, S.u0 + b + rank);
+    }
+}
+
+// The same for batches with larger systems, in kernels over all units.
+// Per unit: centroid, radius and the rebuild test.
 __global__ void ff_check(FFDev D, DevBuf B, int prec) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_release();
+    chain_wait();
     if (u >= D.n_units) return;
     const int s = D.usys[u];
     const FFSys S = D.sys[s];
@@ -130,44 +248,39 @@ __global__ void ff_check(FFDev D, DevBuf B, int prec) {
     float3 x[kMaxUnit];
     const float4 c = unit_centroid(D, B, prec, S, k0, n, x);
     D.ucen[u] = c;
-    if (D.rebuild[s] == 1) return;
+    if (D.force_all) return;
     write_place(D, D.place[u], k0, n, c, x);
-    const float4 r = D.uref[u];
-    const float3 d = min_image(c.x - r.x, c.y - r.y, c.z - r.z, S);
-    if (fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) > S.half_skin2) D.rebuild[s] = 2;
+    if (moved_too_far(D, S, u, c)) D.moved[s] = 1;
 }
+
+// Whether a system's lists are rebuilt in this evaluation (after ff_check).
+__device__ __forceinline__ bool rebuilding(const FFDev& D, int s) { return D.force_all || D.moved[s]; }
 
 __global__ void ff_bin(FFDev D) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_release();
+    chain_wait();
     if (u >= D.n_units) return;
     const int s = D.usys[u];
-    if (!D.rebuild[s]) return;
+    if (!rebuilding(D, s)) return;
     const FFSys S = D.sys[s];
-    if (S.nc == 1) {
-        D.cell_of[u] = S.c0;
-        return;
-    }
-    const float4 c = D.ucen[u];
-    const int cx = wrap_cell(c.x, S.invL, S.nc), cy = wrap_cell(c.y, S.invL, S.nc), cz = wrap_cell(c.z, S.invL, S.nc);
-    const int cell = S.c0 + (cz * S.nc + cy) * S.nc + cx;
-    D.cell_of[u] = cell;
-    atomicAdd(D.cell_count + cell, 1);
+    if (S.nc > 1) atomicAdd(D.cell_count + S.c0 + cell_index(S, D.ucen[u]), 1);
 }
 
 // Exclusive scan of one system's cell counts, in chunks of blockDim.x; the counts are reset.
 __global__ void ff_scan(FFDev D) {
     __shared__ int s[256];
-    if (!D.rebuild[blockIdx.x]) return;
-    if (threadIdx.x == 0) D.rebuilds[blockIdx.x]++;
+    chain_release();
+    chain_wait();
+    const bool build = rebuilding(D, blockIdx.x);
+    if (threadIdx.x == 0) {
+        D.build[blockIdx.x] = build;
+        if (build) D.rebuilds[blockIdx.x]++;
+    }
+    if (!build) return;
     const FFSys S = D.sys[blockIdx.x];
     const int ncell = S.nc * S.nc * S.nc;
-    if (S.nc == 1) {
-        if (threadIdx.x == 0) {
-            D.cell_start[S.c0] = S.u0;
-            D.cell_start[S.c0 + 1] = S.u1;
-        }
-        return;
-    }
+    if (S.nc == 1) return;
     int base = S.u0;
     for (int c0 = 0; c0 < ncell; c0 += blockDim.x) {
         const int c = c0 + threadIdx.x;
@@ -192,32 +305,20 @@ __global__ void ff_scan(FFDev D) {
     if (threadIdx.x == 0) D.cell_start[S.c0 + ncell] = base;  // equals S.u1
 }
 
-// Key of a unit in the order within its cell: its place on a 4 x 4 x 4 grid of the cell in Z-order,
-// then its index, so that the units a list takes of one cell lie in short runs of places and a run of
-// places is compact.
-__device__ __forceinline__ unsigned int cell_key(const FFDev& D, const FFSys& S, int u) {
-    const float4 c = D.ucen[u];
-    const float x[3] = {c.x, c.y, c.z};
-    unsigned int z = 0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int g = (int)(x[k] * S.invL * (float)(4 * S.nc)) & 3;
-        z |= (unsigned int)((g & 1) << k | (g >> 1) << (3 + k));
-    }
-    return z << 26 | (unsigned int)(u - S.u0);
-}
-
 __global__ void ff_scatter(FFDev D) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_release();
+    chain_wait();
     if (u >= D.n_units) return;
     const int s = D.usys[u];
-    if (!D.rebuild[s]) return;
-    if (D.sys[s].nc == 1) {
+    if (!rebuilding(D, s)) return;
+    const FFSys S = D.sys[s];
+    if (S.nc == 1) {
         D.unit_at[u] = u;  // one cell: unit order
         return;
     }
-    const int p = atomicAdd(D.cell_cursor + D.cell_of[u], 1);
-    D.unit_at[p] = (int)cell_key(D, D.sys[s], u);
+    const float4 c = D.ucen[u];
+    D.unit_at[atomicAdd(D.cell_cursor + S.c0 + cell_index(S, c), 1)] = (int)cell_key(S, c, u);
 }
 
 // Sort each cell of a multi-cell box by its units' keys, so that every cell, and so every list, is in
@@ -225,14 +326,15 @@ __global__ void ff_scatter(FFDev D) {
 // entries against all of them (the entries are distinct, so the ranks are a permutation); a cell
 // larger than the stage falls back to an insertion sort by one lane.
 constexpr int kSortWarps = 4, kSortStage = 512;
-constexpr unsigned int kKeyUnit = (1u << 26) - 1;
 __global__ void __launch_bounds__(32 * kSortWarps) ff_sort(FFDev D) {
     __shared__ unsigned int stage[kSortWarps][kSortStage];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int w = blockIdx.x * kSortWarps + warp;
+    chain_release();
+    chain_wait();
     if (w >= D.n_mc) return;
     const int sy = D.mc_sys[w];
-    if (!D.rebuild[sy]) return;
+    if (!rebuilding(D, sy)) return;
     const int c = D.mc_cell[w], u0 = D.sys[sy].u0;
     const int b = D.cell_start[c], e = D.cell_start[c + 1], n = e - b;
     unsigned int* key = (unsigned int*)D.unit_at + b;
@@ -260,98 +362,115 @@ __global__ void __launch_bounds__(32 * kSortWarps) ff_sort(FFDev D) {
     }
 }
 
-// 6. The units of the rebuilt systems at their new places: records, group, build centroid.
 __global__ void ff_place(FFDev D, DevBuf B, int prec) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_release();
+    chain_wait();
     if (p >= D.n_units) return;
     const int s = D.usys[p];  // places [u0, u1) belong to the system of unit p
-    if (!D.rebuild[s]) return;
-    const int u = D.unit_at[p];
-    const FFSys S = D.sys[s];
-    const int2 kn = D.unit[u];
-    const int k0 = kn.x, n = kn.y & 0xff;
-    float3 x[kMaxUnit];
-    const float4 c = unit_centroid(D, B, prec, S, k0, n, x);
-    write_place(D, p, k0, n, c, x);
-    if (!D.ntypes)
-        for (int a = 0; a < D.slots; a++)
-            D.spar[a][p] = a < n ? D.param[k0 + a] : make_float4(0.f, 0.f, 0.f, 0.f);
-    D.place[u] = p;
-    D.sgrp[p] = D.ugrp[u];
-    D.uref[u] = c;
+    if (rebuilding(D, s)) settle(D, B, prec, D.sys[s], D.unit_at[p], p);
 }
 
-// 7. Lists, one warp per unit: the lanes test 32 candidates at a time (their centroids and groups lie
-// in place order, so a row of neighbour cells is one contiguous run) and append the ones in range in
-// order, a ballot giving each its slot. Against one thread per unit of a cell walking the 27 cells
-// staged in shared memory, no lane idles (a cell holds about 48 units of 128 threads) and the list is
-// written coalesced. A full list marks the system as failed (the capacity is sized from the densest
-// system with a wide margin, so this does not happen in a liquid).
-template <bool IMAGE>
-__device__ __forceinline__ void scan_run(const FFDev& D, const FFSys& S, unsigned int* __restrict__ list, float4 c, int grp,
-                                         float3 shift, int q0, int q1, int lane, int& n) {
-    for (int qb = q0; qb < q1; qb += 32) {
-        const int q = qb + lane;
-        bool hit = false;
-        if (q < q1) {
-            const float4 cq = D.scen[q];
-            const int gq = D.sgrp[q];
-            float3 d = make_float3(c.x - (cq.x + shift.x), c.y - (cq.y + shift.y), c.z - (cq.z + shift.z));
-            if (IMAGE) d = min_image(d.x, d.y, d.z, S);
-            const float lim = S.rl + c.w + cq.w;
-            hit = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) < lim * lim && gq != grp;
+// Lists, a warp per unit: the lanes test 32 candidates at a time (their centroids and groups lie in place
+// order, so a row of neighbour cells is one contiguous run) and append the ones in range in order, a
+// ballot giving each its slot. Against one thread per unit of a cell walking the 27 cells staged in
+// shared memory, no lane idles (a cell holds about 48 units of 128 threads) and the list is written
+// coalesced. A full list marks the system as failed (the capacity is sized from the densest system with
+// a wide margin, so this does not happen in a liquid).
+// Bound: load latency. The bounds of all runs are fetched at once, a run per lane, and kAhead chunks of
+// candidates are in flight. Measured per 20 steps: 512 waters 548, 528 and 531 us with 1, 2 and 4 chunks,
+// 256 boxes of the mix 18.4, 18.1 and 18.3 ms. Built by the force pass itself: a kernel of its own, which
+// has nothing to do in most steps, cost 588 us and 19.0 ms.
+// Returns the length of the list of the unit at place p with centroid c.
+__device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p, int s, float4 c, int lane) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    constexpr int kAhead = 2;
+    const int grp = D.sgrp[p];
+    unsigned int* list = D.nbr + (size_t)p * D.cap;
+    // lane's run of places [r0, r1) and its periodic shift: the whole box (minimum image per pair) or, of
+    // the cells around the unit's own, a row of up to three inside the box (lanes 0 to 8) or the one
+    // across its edge (9 to 17). The shifts are exact for units in range: a cell edge is at least
+    // cutoff + skin + twice the largest radius, and there are at least three per edge.
+    const bool image = S.nc == 1;
+    int r0 = 0, r1 = 0, runs = 1;
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    if (image) {
+        r0 = S.u0;
+        r1 = S.u1;
+    } else {
+        const int nc = S.nc;
+        const int cx = wrap_cell(c.x, S.invL, nc), cy = wrap_cell(c.y, S.invL, nc), cz = wrap_cell(c.z, S.invL, nc);
+        const bool edge = cx == 0 || cx == nc - 1;
+        runs = edge ? 18 : 9;
+        if (lane < runs) {
+            int z = cz + lane % 9 / 3 - 1, y = cy + lane % 3 - 1;
+            sz = z < 0 ? -S.L : (z >= nc ? S.L : 0.f);
+            z = z < 0 ? z + nc : (z >= nc ? z - nc : z);
+            sy = y < 0 ? -S.L : (y >= nc ? S.L : 0.f);
+            y = y < 0 ? y + nc : (y >= nc ? y - nc : y);
+            const int* row = D.cell_start + S.c0 + (z * nc + y) * nc;
+            const int x0 = lane < 9 ? max(cx - 1, 0) : (cx == 0 ? nc - 1 : 0);
+            const int x1 = lane < 9 ? min(cx + 1, nc - 1) : x0;
+            sx = lane < 9 ? 0.f : (cx == 0 ? -S.L : S.L);
+            r0 = row[x0];
+            r1 = row[x1 + 1];
         }
-        const unsigned int m = __ballot_sync(0xffffffffu, hit);
-        const int at = n + __popc(m & ((1u << lane) - 1u));
-        if (hit && at < D.cap) list[at] = (unsigned int)(q - S.u0);
-        n += __popc(m);
     }
-}
-
-constexpr int kBuildUnits = 8;  // units per warp of the list build
-__global__ void __launch_bounds__(256) ff_build(FFDev D) {
-    const int warps = (int)blockDim.x >> 5, warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-    for (int k = 0; k < kBuildUnits; k++) {
-        const int p = (blockIdx.x * kBuildUnits + k) * warps + warp;
-        if (p >= D.n_units) return;
-        const int s = D.usys[p];
-        if (!D.rebuild[s]) continue;
-        const FFSys S = D.sys[s];
-        const float4 c = D.scen[p];
-        const int grp = D.sgrp[p];
-        unsigned int* list = D.nbr + (size_t)p * D.cap;
-        int n = 0;
-        if (S.nc == 1) {
-            scan_run<true>(D, S, list, c, grp, make_float3(0.f, 0.f, 0.f), S.u0, S.u1, lane, n);
-        } else {
-            // the cells around the unit's own, one contiguous run of places per row (two where the row
-            // wraps), with the row's periodic image shift (exact for units in range: a cell edge is at
-            // least cutoff + skin + twice the largest radius, and there are at least three per edge)
-            const int nc = S.nc, local = D.cell_of[D.unit_at[p]] - S.c0;
-            const int cx = local % nc, cy = (local / nc) % nc, cz = local / (nc * nc);
-            for (int oz = -1; oz <= 1; oz++) {
-                int z = cz + oz;
-                const float shz = z < 0 ? -S.L : (z >= nc ? S.L : 0.f);
-                z = z < 0 ? z + nc : (z >= nc ? z - nc : z);
-                for (int oy = -1; oy <= 1; oy++) {
-                    int y = cy + oy;
-                    const float shy = y < 0 ? -S.L : (y >= nc ? S.L : 0.f);
-                    y = y < 0 ? y + nc : (y >= nc ? y - nc : y);
-                    const int* row = D.cell_start + S.c0 + (z * nc + y) * nc;
-                    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, nc - 1);
-                    if (cx == 0)
-                        scan_run<false>(D, S, list, c, grp, make_float3(-S.L, shy, shz), row[nc - 1], row[nc], lane, n);
-                    scan_run<false>(D, S, list, c, grp, make_float3(0.f, shy, shz), row[x0], row[x1 + 1], lane, n);
-                    if (cx == nc - 1)
-                        scan_run<false>(D, S, list, c, grp, make_float3(S.L, shy, shz), row[0], row[1], lane, n);
-                }
+    int run = 0, n = 0, q0 = __shfl_sync(kAll, r0, 0), q1 = __shfl_sync(kAll, r1, 0);
+    float hx = __shfl_sync(kAll, sx, 0), hy = __shfl_sync(kAll, sy, 0), hz = __shfl_sync(kAll, sz, 0);
+    bool more = true;  // chunks left: the next begins at q0 of the run that ends at q1
+    auto settle_run = [&]() {
+        while (q0 >= q1) {
+            if (++run >= runs) {
+                more = false;
+                return;
+            }
+            q0 = __shfl_sync(kAll, r0, run);
+            q1 = __shfl_sync(kAll, r1, run);
+            hx = __shfl_sync(kAll, sx, run);
+            hy = __shfl_sync(kAll, sy, run);
+            hz = __shfl_sync(kAll, sz, run);
+        }
+    };
+    settle_run();
+    while (more) {
+        int q[kAhead], gq[kAhead];
+        float4 cq[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            q[k] = more && q0 + lane < q1 ? q0 + lane : -1;
+            cq[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            gq[k] = grp;
+            if (q[k] >= 0) {
+                cq[k] = D.scen[q[k]];
+                gq[k] = D.sgrp[q[k]];
+            }
+            cq[k].x += hx;
+            cq[k].y += hy;
+            cq[k].z += hz;
+            if (more) {
+                q0 += 32;
+                settle_run();
             }
         }
-        if (lane == 0) {
-            D.ncnt[p] = min(n, D.cap);
-            if (n > D.cap && D.sys_status) atomicOr(D.sys_status + s, 2u);
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            float3 d = make_float3(c.x - cq[k].x, c.y - cq[k].y, c.z - cq[k].z);
+            if (image) d = min_image(d.x, d.y, d.z, S);
+            const float lim = S.rl + c.w + cq[k].w;
+            const bool hit = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) < lim * lim && gq[k] != grp;
+            const unsigned int m = __ballot_sync(kAll, hit);
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            if (hit && at < D.cap) list[at] = (unsigned int)(q[k] - S.u0);
+            n += __popc(m);
         }
     }
+    if (lane == 0) {
+        D.ncnt[p] = min(n, D.cap);
+        if (n > D.cap && D.sys_status) atomicOr(D.sys_status + s, 2u);
+    }
+    __syncwarp();  // the lanes read each other's entries
+    return min(n, D.cap);
 }
 
 // Compensated FP32 accumulator (Knuth's two-sum): the running sum keeps its rounding error in `lo`.
@@ -380,7 +499,7 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
     *to = __float2ll_rn(fminf(fmaxf(f, -kMaxF), kMaxF) * 0x1p32f);
 }
 
-// 8. Forces from the lists: one warp per unit, the unit's atoms in registers. The lanes take the list
+// Forces from the lists: one warp per unit, the unit's atoms in registers. The lanes take the list
 // entries 32 at a time: each finds its listed unit's periodic shift (the minimum image of the
 // centroids) and drops the entry when the centroids lie farther apart than cutoff + both radii (no
 // pair of the two is then within the cutoff); a ballot packs the others into a per-warp ring. From
@@ -423,7 +542,7 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
     constexpr unsigned int kAll = 0xffffffffu;
     extern __shared__ float4 stab[];  // PT: the type-pair table
     const int lane = T.lane, nt = D.ntypes;
-    const unsigned int* __restrict__ nb = D.nbr + (size_t)T.p * D.cap;
+    const unsigned int* nb = D.nbr + (size_t)T.p * D.cap;
     const int u0 = S.u0;
     const float4 c = T.c;
     const float two_krf = 2.0f * S.krf, rc2 = S.rc2;
@@ -570,15 +689,17 @@ __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, co
     unit_forces<JS, 1, 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
 }
 
-// Blocks per SM: 64 registers for the pass of every step, more where a variant would spill.
+// Blocks per SM: 64 registers for the pass of every step, 80 for the larger variants (with 128, forces
+// of 40 boxes with 64-type solutes took 1.09 ms instead of 0.98).
 template <int JS, bool ENERGY, bool PT> constexpr int force_blocks() {
-    return JS <= 2 || (JS == 3 && PT && !ENERGY) ? 4 : PT || !ENERGY ? 3 : 2;
+    return JS <= 2 || (JS == 3 && PT && !ENERGY) ? 4 : 3;
 }
 
 template <int JS, bool ENERGY, bool PT, bool RELAX>
 __global__ void __launch_bounds__(32 * kFW, (force_blocks<JS, ENERGY, PT>())) ff_force(FFDev D, long long* __restrict__ force, int stride) {
     extern __shared__ float4 stab[];  // PT: the type-pair table
     __shared__ float4 ring[kFW][kRing];
+    chain_release();
     const int nt = D.ntypes;
     if (PT) {
         for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) stab[t] = D.types[t];
@@ -587,13 +708,16 @@ __global__ void __launch_bounds__(32 * kFW, (force_blocks<JS, ENERGY, PT>())) ff
     const int warp = (int)threadIdx.x >> 5;
     UnitTask T;
     T.p = blockIdx.x * kFW + warp;
-    if (T.p >= D.n_units) return;
+    const bool on = T.p < D.n_units;
     T.lane = (int)threadIdx.x & 31;
-    T.s = D.usys[T.p];
-    T.n = D.ncnt[T.p];
+    T.s = on ? D.usys[T.p] : 0;
+    const FFSys S = D.sys[T.s];
+    chain_wait();
+    if (!on) return;
     T.c = D.scen[T.p];
     T.ring = ring[warp];
-    const FFSys S = D.sys[T.s];
+    T.n = D.build[T.s] ? build_list(D, S, T.p, T.s, T.c, T.lane) : D.ncnt[T.p];
+    if (T.p == S.u0 && T.lane == 0) D.moved[T.s] = 0;  // for the next evaluation's ff_check
     const int nn = D.unit[D.unit_at[T.p]].y, ni = nn & 0xff, nl = nn >> 8;
     if (S.pair_image)
         unit_dispatch<JS, ENERGY, PT, RELAX, true>(D, S, T, ni, nl, force, stride);
@@ -602,25 +726,26 @@ __global__ void __launch_bounds__(32 * kFW, (force_blocks<JS, ENERGY, PT>())) ff
 }
 
 template <int JS, bool ENERGY, bool RELAX>
-void launch_force_kernel(const FFDev& D, long long* f, int stride, cudaStream_t st) {
+cudaError_t launch_force_kernel(const FFDev& D, long long* f, int stride, cudaStream_t st) {
     const int grid = (D.n_units + kFW - 1) / kFW;
     if (D.ntypes)
-        ff_force<JS, ENERGY, true, RELAX><<<grid, 32 * kFW, sizeof(float4) * D.ntypes * D.ntypes, st>>>(D, f, stride);
-    else
-        ff_force<JS, ENERGY, false, RELAX><<<grid, 32 * kFW, 0, st>>>(D, f, stride);
+        return launch_chained(ff_force<JS, ENERGY, true, RELAX>, grid, 32 * kFW, sizeof(float4) * D.ntypes * D.ntypes, st,
+                              D, f, stride);
+    return launch_chained(ff_force<JS, ENERGY, false, RELAX>, grid, 32 * kFW, 0, st, D, f, stride);
 }
 
 // A capped relaxation forms no energies.
-template <int JS> void launch_force_pass(const FFDev& D, bool energy, long long* f, int stride, cudaStream_t st) {
-    if (D.fcap > 0.0f) launch_force_kernel<JS, false, true>(D, f, stride, st);
-    else if (energy) launch_force_kernel<JS, true, false>(D, f, stride, st);
-    else launch_force_kernel<JS, false, false>(D, f, stride, st);
+template <int JS> cudaError_t launch_force_pass(const FFDev& D, bool energy, long long* f, int stride, cudaStream_t st) {
+    if (D.fcap > 0.0f) return launch_force_kernel<JS, false, true>(D, f, stride, st);
+    return energy ? launch_force_kernel<JS, true, false>(D, f, stride, st) : launch_force_kernel<JS, false, false>(D, f, stride, st);
 }
 
 // One block per chunk of a system's units.
 __global__ void ff_energy(FFDev D, double* part) {
     __shared__ double s[256];
+    chain_release();
     const int2 c = D.e_chunks.chunk[blockIdx.x];
+    chain_wait();
     const int u0 = D.sys[c.x].u0 + c.y, u1 = min(u0 + kEnergyChunk, D.sys[c.x].u1);
     double e = 0.0;
     for (int u = u0 + (int)threadIdx.x; u < u1; u += blockDim.x) e += D.e_unit[u];
@@ -652,40 +777,39 @@ int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* 
     if (D.n_int == 0) return 0;
     const int t = 256, gg = (D.n_units + t - 1) / t;
     int n = 0;
-    ff_check<<<gg, t, 0, st>>>(D, B, prec);
-    ff_bin<<<gg, t, 0, st>>>(D);
-    ff_scan<<<D.S, 256, 0, st>>>(D);
-    ff_scatter<<<gg, t, 0, st>>>(D);
-    n += 4;
-    if (D.n_mc) {
-        ff_sort<<<(D.n_mc + kSortWarps - 1) / kSortWarps, 32 * kSortWarps, 0, st>>>(D);
+    cudaError_t e = cudaSuccess;
+    auto put = [&](cudaError_t r) {
+        if (e == cudaSuccess) e = r;
         n++;
+    };
+    if (D.prep_units) {
+        const int threads = D.prep_units >= 1024 ? 1024 : (D.prep_units + 31) / 32 * 32;
+        put(launch_chained(ff_prep, D.S, threads, sizeof(int) * (D.prep_units + D.prep_cells), st, D, B, prec));
+    } else {
+        put(launch_chained(ff_check, gg, t, 0, st, D, B, prec));
+        put(launch_chained(ff_bin, gg, t, 0, st, D));
+        put(launch_chained(ff_scan, D.S, 256, 0, st, D));
+        put(launch_chained(ff_scatter, gg, t, 0, st, D));
+        if (D.n_mc) put(launch_chained(ff_sort, (D.n_mc + kSortWarps - 1) / kSortWarps, 32 * kSortWarps, 0, st, D));
+        put(launch_chained(ff_place, gg, t, 0, st, D, B, prec));
     }
-    ff_place<<<gg, t, 0, st>>>(D, B, prec);
-    // block size chosen by the autotuner (results do not depend on it: a warp builds each list)
-    const int per_block = D.build_threads / 32 * kBuildUnits;
-    ff_build<<<(D.n_units + per_block - 1) / per_block, D.build_threads, 0, st>>>(D);
-    n += 2;
-    if (cudaMemsetAsync(D.rebuild, 0, (size_t)D.S, st) != cudaSuccess) return -1;
     long long* f = const_cast<long long*>(B.force);
     switch (D.slots) {
-        case 1: launch_force_pass<1>(D, energy, f, B.stride, st); break;
-        case 2: launch_force_pass<2>(D, energy, f, B.stride, st); break;
-        case 3: launch_force_pass<3>(D, energy, f, B.stride, st); break;
-        default: launch_force_pass<4>(D, energy, f, B.stride, st);
+        case 1: put(launch_force_pass<1>(D, energy, f, B.stride, st)); break;
+        case 2: put(launch_force_pass<2>(D, energy, f, B.stride, st)); break;
+        case 3: put(launch_force_pass<3>(D, energy, f, B.stride, st)); break;
+        default: put(launch_force_pass<4>(D, energy, f, B.stride, st));
     }
-    n++;
     if (energy) {
         const SystemChunks& c = D.e_chunks;
         double* part = c.n == D.S ? D.energy : c.part;  // every system one chunk: its sum is the result
-        ff_energy<<<c.n, 256, 0, st>>>(D, part);
-        n++;
+        put(launch_chained(ff_energy, c.n, 256, 0, st, D, part));
         if (part != D.energy) {
             if (launch_join_chunks(part, c.chunk0, D.S, 1, D.energy, stream) < 0) return -1;
             n++;
         }
     }
-    return cudaPeekAtLastError() == cudaSuccess ? n : -1;
+    return e == cudaSuccess ? n : -1;
 }
 
 }  // namespace rbx

@@ -136,7 +136,6 @@ struct FFDev {
     float4* uref;         // [n_units] u: centroid at the last build
     int* place;           // [n_units] u -> p of the last build
     int* unit_at;         // [n_units] p -> u
-    int* cell_of;         // [n_units] u
     int* cell_count;      // [n_cells], zero between evaluations
     int* cell_start;      // [n_cells + 1] (entry c0 + nc^3 of each system ends it)
     int* cell_cursor;     // [n_cells]
@@ -152,8 +151,10 @@ struct FFDev {
     // Neighbour lists of units, rebuilt per system when one of its centroids has moved more than
     // half the skin since the last build, and for every system at the last evaluation of every
     // step call and at the first evaluation after a state is set
-    unsigned char* rebuild;  // [S] rebuild this system's lists before the next force pass: 1 set by the
-                             // host, 2 by the displacement test
+    int force_all;           // this evaluation rebuilds every system's lists
+    unsigned char* moved;    // [S] set by the displacement test (batches with large systems), zero between
+                             // evaluations
+    unsigned char* build;    // [S] this evaluation's force pass builds the system's lists
     unsigned int* rebuilds;  // [S] list builds of each system so far (a statistic)
     unsigned int* nbr;       // entry e of place p at p * cap + e: the listed unit's place - u0
     int* ncnt;               // [n_units] p: entries
@@ -169,7 +170,9 @@ struct FFDev {
     unsigned int* sys_status;  // [S] bit 0: a force of the system is non-finite or beyond the
                                // fixed-point range (never during a capped relaxation); bit 1: a list
                                // outgrew its capacity
-    int build_threads;    // block size of the list-build kernel: 64, 128 (default) or 256
+    // the largest system's units and list cells, where every system is small enough for one block
+    // (prep_limit); prep_units = 0 otherwise
+    int prep_units, prep_cells;
     // work list of the cell sort (set with the state): every cell of the multi-cell boxes with its system
     int n_mc;
     const int* mc_cell;
@@ -178,6 +181,11 @@ struct FFDev {
 constexpr int kMaxTypes = 32;  // atom types of the type-pair table (FFDev::types)
 // Interacting atoms of one system (a limit of this interface: list entries are 32-bit words).
 constexpr int kMaxSystemAtoms = 1 << 26;
+// Whether the set-up of a system of this many units and list cells is left to one block (ff_prep): a
+// unit per thread, and keys and cell counts in 48 KB of shared memory. Larger systems gain more from
+// every SM than from fewer launches: 60 boxes of 300 to 2500 waters take 4.53 ms per 20 steps in
+// kernels over all units and 4.66 in a block each.
+inline bool prep_limit(long long units, long long cells) { return units <= 1024 && units + cells <= 12000; }
 int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* stream);
 // Fixed-point forces of slots [0, natoms) -> user-order doubles out[3*natoms] (kJ/mol/nm).
 int launch_forces_to_user(const long long* force, int stride, int natoms, double* out, void* stream);
