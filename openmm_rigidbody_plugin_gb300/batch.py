@@ -102,16 +102,16 @@ class BatchedSystems:
         _lib.check(self._lib.rbx_batch_set_state(self._h, _stream(stream), _d(x), _d(v)))
 
     def get_state(self, stream=None):
-        x = np.zeros((self.num_atoms, 3))
-        v = np.zeros((self.num_atoms, 3))
+        x = np.empty((self.num_atoms, 3))
+        v = np.empty((self.num_atoms, 3))
         _lib.check(self._lib.rbx_batch_get_state(self._h, _stream(stream), _d(x), _d(v)))
         return x, v
 
     def get_system_state(self, s, stream=None):
         """Positions and velocities of system s only."""
         n = int(self.offsets[s + 1] - self.offsets[s])
-        x = np.zeros((n, 3))
-        v = np.zeros((n, 3))
+        x = np.empty((n, 3))
+        v = np.empty((n, 3))
         _lib.check(self._lib.rbx_batch_get_system_state(self._h, _stream(stream), int(s), _d(x), _d(v)))
         return x, v
 
@@ -143,14 +143,14 @@ class BatchedSystems:
 
     def energies(self, stream=None):
         """[U, KE_t, KE_r] per system (kJ/mol), shape (num_systems, 3)."""
-        out = np.zeros((self.num_systems, 3))
+        out = np.empty((self.num_systems, 3))
         _lib.check(self._lib.rbx_batch_energies(self._h, _stream(stream), _d(out)))
         return out
 
     def forces(self, stream=None):
         """Forces at the current positions (user order, kJ/mol/nm) and the potential energies."""
-        f = np.zeros((self.num_atoms, 3))
-        e = np.zeros(self.num_systems)
+        f = np.empty((self.num_atoms, 3))
+        e = np.empty(self.num_systems)
         _lib.check(self._lib.rbx_batch_forces(self._h, _stream(stream), _d(f), _d(e)))
         return f, e
 

@@ -323,8 +323,8 @@ class IntegratorKernel:
         return b
 
     def context_get_state(self, stream=None):
-        x = np.zeros((self.num_atoms, 3))
-        v = np.zeros((self.num_atoms, 3))
+        x = np.empty((self.num_atoms, 3))
+        v = np.empty((self.num_atoms, 3))
         _lib.check(self._lib.rbx_context_get_state(self._h, _stream_handle(stream), _dptr(x), _dptr(v)))
         return x, v
 
