@@ -108,7 +108,7 @@ struct rbx_batch {
     DevArray<FFSys> d_sys;
     DevArray<int> d_iatom, d_ugrp, d_usys, d_place, d_unit_at, d_cell_count, d_cell_start, d_cell_cursor;
     DevArray<int> d_sgrp, d_mc_cell, d_mc_sys, d_ncnt, d_atype;
-    DevArray<int2> d_unit;
+    DevArray<int2> d_unit, d_sunit;
     DevArray<float4> d_param, d_ucen, d_uref, d_scen, d_spos, d_spar, d_types;
     DevArray<unsigned char> d_moved, d_build;
     DevArray<unsigned int> d_nbr;       // neighbour lists of units (FFDev::nbr)
@@ -419,13 +419,11 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     int cells = 0, groups = 0, slots = 1;
     for (int s = 0; s < num_systems; s++) {
         FFSys& f = sys[s];
-        f.a0 = atom_offsets[s];
-        f.a1 = atom_offsets[s + 1];
-        f.i0 = (int)iatom.size();
+        const size_t i0 = iatom.size();
         f.u0 = (int)unit.size();
         std::map<int, std::vector<int>> bodies;
         std::vector<int> free_atoms;
-        for (int i = f.a0; i < f.a1; i++) {
+        for (int i = atom_offsets[s]; i < atom_offsets[s + 1]; i++) {
             if (charges[i] == 0.0 && epsilons[i] == 0.0) continue;
             if (body_indices[i] > 0) bodies[body_indices[i]].push_back(i);
             else free_atoms.push_back(i);
@@ -458,11 +456,10 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         };
         for (auto& kv : bodies) add_group(kv.second.data(), (int)kv.second.size());
         for (int i : free_atoms) add_group(&i, 1);
-        f.i1 = (int)iatom.size();
         f.u1 = (int)unit.size();
-        if (f.i1 - f.i0 >= kMaxSystemAtoms) {
+        if (iatom.size() - i0 >= (size_t)kMaxSystemAtoms) {
             delete b;
-            return set_error(RBX_ERR_UNSUPPORTED, "system %d: %d interacting atoms (at most %d)", s, f.i1 - f.i0,
+            return set_error(RBX_ERR_UNSUPPORTED, "system %d: %zu interacting atoms (at most %d)", s, iatom.size() - i0,
                              kMaxSystemAtoms - 1);
         }
         const double L = box_edges[s], rc_s = cutoffs[s];
@@ -483,6 +480,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         cells += nc * nc * nc;
         f.L = (float)L;
         f.invL = (float)(1.0 / L);
+        f.rc = (float)rc_s;
         f.rc2 = (float)(rc_s * rc_s);
         const double krf = (eps_solvent - 1.0) / ((2.0 * eps_solvent + 1.0) * rc_s * rc_s * rc_s);
         f.krf = (float)krf;
@@ -543,7 +541,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     if (!rc && (b->d_place.alloc(u1) != cudaSuccess || b->d_unit_at.alloc(u1) != cudaSuccess ||
                 b->d_ucen.alloc(u1) != cudaSuccess ||
                 b->d_uref.alloc(u1) != cudaSuccess || b->d_scen.alloc(u1) != cudaSuccess ||
-                b->d_sgrp.alloc(u1) != cudaSuccess || b->d_ncnt.alloc(u1) != cudaSuccess ||
+                b->d_sgrp.alloc(u1) != cudaSuccess || b->d_sunit.alloc(u1) != cudaSuccess || b->d_ncnt.alloc(u1) != cudaSuccess ||
                 b->d_spos.alloc(records) != cudaSuccess || b->d_spar.alloc(types.empty() ? records : 0) != cudaSuccess ||
                 b->d_cell_count.alloc(cells) != cudaSuccess || b->d_cell_start.alloc(cells + 1) != cudaSuccess ||
                 b->d_cell_cursor.alloc(cells) != cudaSuccess || b->d_e_unit.alloc(u1) != cudaSuccess ||
@@ -586,6 +584,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.cell_cursor = b->d_cell_cursor.p;
     D.scen = b->d_scen.p;
     D.sgrp = b->d_sgrp.p;
+    D.sunit = b->d_sunit.p;
     for (int a = 0; a < kMaxUnit; a++) {
         D.spos[a] = a < slots ? b->d_spos.p + a * u1 : nullptr;
         D.spar[a] = a < slots && types.empty() ? b->d_spar.p + a * u1 : nullptr;
@@ -831,7 +830,7 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
     size_t n = b->d_sys.bytes() + b->d_iatom.bytes() + b->d_param.bytes() + b->d_unit.bytes() + b->d_ugrp.bytes() +
                b->d_usys.bytes() + b->d_ucen.bytes() + b->d_uref.bytes() + b->d_place.bytes() + b->d_unit_at.bytes() +
                b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
-               b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_spos.bytes() + b->d_spar.bytes() + b->d_mc_cell.bytes() +
+               b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_sunit.bytes() + b->d_spos.bytes() + b->d_spar.bytes() + b->d_mc_cell.bytes() +
                b->d_mc_sys.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() + b->d_build.bytes() + b->d_nbr.bytes() +
                b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_e_unit.bytes() + b->d_energy.bytes() +
                b->d_body0.bytes() + b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() +

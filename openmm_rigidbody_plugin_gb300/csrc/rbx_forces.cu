@@ -155,6 +155,7 @@ __device__ __forceinline__ void settle(const FFDev& D, const DevBuf& B, int prec
     D.place[u] = p;
     D.unit_at[p] = u;
     D.sgrp[p] = D.ugrp[u];
+    D.sunit[p] = kn;
     D.uref[u] = c;
 }
 
@@ -514,24 +515,59 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 // table in shared memory, else from the atoms' own parameters by Lorentz-Berthelot.
 // The pair term is OpenMM's CutoffPeriodic form: reaction-field Coulomb and unshifted LJ.
 //
-// Bound: instruction issue (64 % of the slots used), the L1 data pipe (67 %) and load latency, not HBM
-// (6 %). Measured on 256 boxes of 64 to 4096 bodies of the water/tetrahedron/ring mix (1.07e6 atoms):
-// 0.82 ms per step with list builds and integrator, against 1.22 for one warp per rigid body with its
-// atoms in shared memory, neighbours expanded atom by atom through a queue, and the neighbours'
-// records in list order. What made the difference: the unit's atoms in registers (no shared-memory
-// load per pair), one listed unit per lane instead of one atom (a third of the entry work), records in
-// cell order and by atom slot (contiguous lanes read contiguous records: a quarter fewer L1
-// wavefronts), and no Lennard-Jones term for the atoms that have none. Not kept, all within 3 %: 80
-// registers and 24 warps per SM, blocks of 4, 16 or 32 warps, two atoms at a time in packed FP32
-// instructions (the FMA pipe takes as long; 5 % slower).
-constexpr int kFW = 8;    // warps (units) per block
+// Bound: instruction issue (62 % of the slots used), the L1 data pipe (53 to 67 %) and load latency, not
+// HBM (6 %). Measured per step of 256 boxes of 64 to 4096 bodies of the water/tetrahedron/ring mix
+// (1.07e6 atoms), list builds and integrator included: 0.75 ms, against 1.22 for one warp per rigid
+// body with its atoms in shared memory, neighbours expanded atom by atom through a queue, and the
+// neighbours' records in list order. What made the difference: the unit's atoms in registers (no
+// shared-memory load per pair), one listed unit per lane instead of one atom (a third of the entry
+// work), records in cell order and by atom slot (contiguous lanes read contiguous records: a quarter
+// fewer L1 wavefronts), no Lennard-Jones term for the atoms that have none; then (17.5 -> 16.3 ms per
+// 20 steps) all that a place names fetched at once, predicated sums, halving sums over the lanes and
+// blocks of 4 warps (8: 16.7). Energies are added three pairs at a time to the compensated sum, without
+// branches (forces of 40 boxes with solutes 0.98 -> 0.80 ms). Not kept: 40 warps per SM at 48 registers
+// (19.2 ms); 24 at 80, with (20.5) or without (equal) the next atoms fetched before these are paired;
+// two atoms at a time in packed FP32 instructions (the FMA pipe takes as long; 5 % slower).
+constexpr int kFW = 4;    // warps (units) per block
 constexpr int kRing = 64;  // packed list entries per warp
 
 struct UnitTask {
     int p, s, n, lane;        // place, system, list entries
+    int k0;                   // the unit's first interacting atom
+    int q0, q1;               // the lane's first two list entries (before clamping to n)
     float4 c;                 // centroid and radius
     float4* ring;
 };
+
+// Sums of N values over the warp, each in one lane: at every step a lane hands half of its values to its
+// partner and takes the partner's share of the other half, so the work halves (N = 9: 12 shuffles
+// instead of 45). Returns the index of the value that the lane ends with, in v[0], or -1. Lanes that
+// differ in bit 0 end with the same value; the even one has it.
+template <int M, int O, int N> __device__ __forceinline__ void join_step(float (&v)[N], int lane, int& first, int& count) {
+    if constexpr (O > 0) {
+        constexpr int K = (M + 1) / 2;
+        if constexpr (M == 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+            if (lane & O) count = 0;
+        } else {
+            const bool up = (lane & O) != 0;
+#pragma unroll
+            for (int i = 0; i < K; i++) {
+                const float hi = i + K < M ? v[i + K] : 0.0f;
+                const float give = up ? v[i] : hi, keep = up ? hi : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+            }
+            first += up ? K : 0;
+            count = up ? count - K : min(count, K);
+        }
+        join_step<K, O / 2>(v, lane, first, count);
+    }
+}
+template <int N> __device__ __forceinline__ int join_lanes(float (&v)[N], int lane) {
+    int first = 0, count = N;
+    join_step<N, 16>(v, lane, first, count);
+    return count > 0 ? first : -1;
+}
 
 // NI atoms of the unit, the first NL with Lennard-Jones (the others Coulomb only: their pairs skip it,
 // and the unit's charge is applied once, to the sum). JS: atom records per place. RELAX: coincident
@@ -564,19 +600,15 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
         }
     }
     ESum en;
-    // the atoms of one listed unit (place q, shift sh) against the unit's own
-    auto stream = [&](float4 e, bool full) {
-        const int q = __float_as_int(e.w);
-        float4 xq[JS];
-#pragma unroll
-        for (int b = 0; b < JS; b++) xq[b] = full ? D.spos[b][q] : make_float4(kFar, kFar, kFar, 0.0f);
+    // the atoms xq of one listed unit (place and shift e) against the unit's own
+    auto pairs = [&](const float4 (&xq)[JS], float4 e) {
 #pragma unroll
         for (int b = 0; b < JS; b++) {
             const float xj = xq[b].x + e.x, yj = xq[b].y + e.y, zj = xq[b].z + e.z;
             const int tj = __float_as_int(xq[b].w);
-            float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!PT && full) pj = D.spar[b][q];
-            float qj = 0.0f;
+            float4 pj;
+            if (!PT) pj = D.spar[b][__float_as_int(e.w)];
+            float qj = 0.0f, eb = 0.0f;
             // K q_i q_j, 12 C12, 6 C6 of the pair (and, from the table, the streamed atom's charge)
             auto coefficients = [&](int a) {
                 float4 t;
@@ -604,74 +636,101 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                     const float inv_r6 = inv_r2 * inv_r2 * inv_r2;
                     const float lj = inv_r6 * fmaf(t.y, inv_r6, -t.z);  // 12 C12 r^-12 - 6 C6 r^-6
                     gf = fmaf(t.x, rf, lj * inv_r2);
-                    if (ENERGY && in)
-                        en.add(t.x * (inv_r + S.krf * r2 - S.crf) +
-                               inv_r6 * (t.y * (1.0f / 12.0f) * inv_r6 - t.z * (1.0f / 6.0f)));
+                    if (ENERGY) {
+                        const float ep = t.x * (inv_r + S.krf * r2 - S.crf) +
+                                         inv_r6 * (t.y * (1.0f / 12.0f) * inv_r6 - t.z * (1.0f / 6.0f));
+                        eb += in ? ep : 0.0f;
+                    }
                 } else {
                     gf = qj * rf;
-                    if (ENERGY && in) en.add(qi[a] * qj * (inv_r + S.krf * r2 - S.crf));
+                    if (ENERGY) eb += in ? qi[a] * qj * (inv_r + S.krf * r2 - S.crf) : 0.0f;
                 }
-                gf = in ? gf : 0.0f;
-                f[a][0] = fmaf(gf, d.x, f[a][0]);
-                f[a][1] = fmaf(gf, d.y, f[a][1]);
-                f[a][2] = fmaf(gf, d.z, f[a][2]);
+                if (in) {
+                    f[a][0] = fmaf(gf, d.x, f[a][0]);
+                    f[a][1] = fmaf(gf, d.y, f[a][1]);
+                    f[a][2] = fmaf(gf, d.z, f[a][2]);
+                }
             }
+            if (ENERGY) en.add(eb);
         }
     };
-    const float reach = sqrtf(rc2) + c.w + 1e-6f;
+    const float reach = S.rc + c.w + 1e-6f;
+    const int slot = D.iatom[T.k0 + min(lane / 3, NI - 1)];
     int head = 0, held = 0;  // the ring's first entry and length
     // list entries and their centroids are fetched a batch ahead of their use
+    // (entries past the list's end, whatever the memory holds, become the system's first place)
     const int last = max(T.n - 1, 0);
-    int q0 = T.n ? u0 + (int)nb[min(lane, last)] : u0, q1 = T.n ? u0 + (int)nb[min(32 + lane, last)] : u0;
+    int q0 = u0 + (lane < T.n ? T.q0 : 0), q1 = u0 + (lane + 32 < T.n ? T.q1 : 0);
     float4 c0 = D.scen[q0];
-    for (int e0 = 0; e0 < T.n; e0 += 32) {
-        const int q = q0;
-        const float4 cj = c0;
-        q0 = q1;
-        c0 = D.scen[q1];
-        q1 = u0 + (int)nb[min(e0 + 64 + lane, last)];
-        const float dx = cj.x - c.x, dy = cj.y - c.y, dz = cj.z - c.z;
-        const float4 e = make_float4(-S.L * rintf(dx * S.invL), -S.L * rintf(dy * S.invL), -S.L * rintf(dz * S.invL),
-                                     __int_as_float(q));
-        const float ex = dx + e.x, ey = dy + e.y, ez = dz + e.z;
-        const float lim = reach + cj.w;
-        const bool keep = e0 + lane < T.n && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < lim * lim;
-        const unsigned int m = __ballot_sync(kAll, keep);
-        if (keep) T.ring[(head + held + __popc(m & ((1u << lane) - 1u))) & (kRing - 1)] = e;
-        held += __popc(m);
-        __syncwarp();
-        if (held >= 32) {
-            stream(T.ring[(head + lane) & (kRing - 1)], true);
-            head += 32;
-            held -= 32;
+    for (int e0 = 0;;) {
+        while (held < 32 && e0 < T.n) {
+            const int q = q0;
+            const float4 cj = c0;
+            q0 = q1;
+            c0 = D.scen[q1];
+            q1 = u0 + (int)nb[min(e0 + 64 + lane, last)];
+            const float dx = cj.x - c.x, dy = cj.y - c.y, dz = cj.z - c.z;
+            const float4 e = make_float4(-S.L * rintf(dx * S.invL), -S.L * rintf(dy * S.invL), -S.L * rintf(dz * S.invL),
+                                         __int_as_float(q));
+            const float ex = dx + e.x, ey = dy + e.y, ez = dz + e.z;
+            const float lim = reach + cj.w;
+            const bool keep = e0 + lane < T.n && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < lim * lim;
+            const unsigned int m = __ballot_sync(kAll, keep);
+            if (keep) T.ring[(head + held + __popc(m & ((1u << lane) - 1u))) & (kRing - 1)] = e;
+            held += __popc(m);
+            e0 += 32;
             __syncwarp();
         }
-    }
-    if (held) stream(lane < held ? T.ring[(head + lane) & (kRing - 1)] : make_float4(0.f, 0.f, 0.f, 0.f), lane < held);
-    // join the lanes (every lane ends with the same sums); lane 3 a + c stores component c of atom a
-    const int u = D.unit_at[T.p];
-    const int k0 = D.unit[u].x;
-    float mine = 0.0f;
+        if (held == 0) break;
+        float4 x[JS], e = make_float4(0.f, 0.f, 0.f, __int_as_float(u0));
+        if (lane < held) {
+            e = T.ring[(head + lane) & (kRing - 1)];
 #pragma unroll
-    for (int a = 0; a < NI; a++) {
-        const float w = a < NL ? 1.0f : qi[a];
+            for (int b = 0; b < JS; b++) x[b] = D.spos[b][__float_as_int(e.w)];
+        } else {
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) f[a][k] += __shfl_xor_sync(kAll, f[a][k], o);
-            f[a][k] *= w;
+            for (int b = 0; b < JS; b++) x[b] = make_float4(kFar, kFar, kFar, 0.0f);
         }
-        const float cap = force_scale(D, f[a][0], f[a][1], f[a][2]);
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            if (lane == 3 * a + k) mine = f[a][k] * cap;
+        head += 32;
+        held = max(held - 32, 0);
+        pairs(x, e);
+        __syncwarp();
     }
-    if (lane < 3 * NI) store_force(D, force + D.iatom[k0 + lane / 3] + (size_t)(lane % 3) * stride, mine, T.s);
+    // join the lanes; every component of every atom's force is stored by one lane
+#pragma unroll
+    for (int a = NL; a < NI; a++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) f[a][k] *= qi[a];
+    float v[3 * NI];
+    if (RELAX) {  // every lane ends with all sums, for the cap on an atom's force
+        float mine = 0.0f;
+#pragma unroll
+        for (int a = 0; a < NI; a++) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) f[a][k] += __shfl_xor_sync(kAll, f[a][k], o);
+            }
+            const float cap = force_scale(D, f[a][0], f[a][1], f[a][2]);
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (lane == 3 * a + k) mine = f[a][k] * cap;
+        }
+        if (lane < 3 * NI) store_force(D, force + slot + (size_t)(lane % 3) * stride, mine, T.s);
+    } else {
+#pragma unroll
+        for (int a = 0; a < NI; a++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) v[3 * a + k] = f[a][k];
+        const int at = join_lanes(v, lane);
+        const int to = __shfl_sync(kAll, slot, max(at, 0) / 3 * 3);
+        if (at >= 0) store_force(D, force + to + (size_t)(at % 3) * stride, v[0], T.s);
+    }
     if (ENERGY) {
         double e = en.value();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(kAll, e, o);
-        if (lane == 0) D.e_unit[u] = 0.5 * e;
+        if (lane == 0) D.e_unit[D.unit_at[T.p]] = 0.5 * e;
     }
 }
 
@@ -689,14 +748,13 @@ __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, co
     unit_forces<JS, 1, 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
 }
 
-// Blocks per SM: 64 registers for the pass of every step, 80 for the larger variants (with 128, forces
-// of 40 boxes with 64-type solutes took 1.09 ms instead of 0.98).
-template <int JS, bool ENERGY, bool PT> constexpr int force_blocks() {
-    return JS <= 2 || (JS == 3 && PT && !ENERGY) ? 4 : 3;
-}
+// Blocks per SM: 64 registers a thread (32 warps per SM); 80 for units of four atoms. The larger variants
+// then spill a little and still gain: forces of 40 boxes with 64-type solutes take 1.09 ms at 128
+// registers, 0.98 at 80 and 0.97 at 64.
+constexpr int force_blocks(int records) { return records <= 3 ? 8 : 6; }
 
 template <int JS, bool ENERGY, bool PT, bool RELAX>
-__global__ void __launch_bounds__(32 * kFW, (force_blocks<JS, ENERGY, PT>())) ff_force(FFDev D, long long* __restrict__ force, int stride) {
+__global__ void __launch_bounds__(32 * kFW, force_blocks(JS)) ff_force(FFDev D, long long* __restrict__ force, int stride) {
     extern __shared__ float4 stab[];  // PT: the type-pair table
     __shared__ float4 ring[kFW][kRing];
     chain_release();
@@ -714,11 +772,22 @@ __global__ void __launch_bounds__(32 * kFW, (force_blocks<JS, ENERGY, PT>())) ff
     const FFSys S = D.sys[T.s];
     chain_wait();
     if (!on) return;
-    T.c = D.scen[T.p];
     T.ring = ring[warp];
-    T.n = D.build[T.s] ? build_list(D, S, T.p, T.s, T.c, T.lane) : D.ncnt[T.p];
+    // all that the place names is fetched at once: a warp's chain of dependent loads is short
+    T.c = D.scen[T.p];
+    T.n = D.ncnt[T.p];
+    const int2 kn = D.sunit[T.p];
+    const unsigned int* nb = D.nbr + (size_t)T.p * D.cap;
+    T.q0 = (int)nb[T.lane];
+    T.q1 = (int)nb[min(32 + T.lane, D.cap - 1)];
+    if (D.build[T.s]) {
+        T.n = build_list(D, S, T.p, T.s, T.c, T.lane);
+        T.q0 = (int)nb[T.lane];
+        T.q1 = (int)nb[min(32 + T.lane, D.cap - 1)];
+    }
     if (T.p == S.u0 && T.lane == 0) D.moved[T.s] = 0;  // for the next evaluation's ff_check
-    const int nn = D.unit[D.unit_at[T.p]].y, ni = nn & 0xff, nl = nn >> 8;
+    T.k0 = kn.x;
+    const int ni = kn.y & 0xff, nl = kn.y >> 8;
     if (S.pair_image)
         unit_dispatch<JS, ENERGY, PT, RELAX, true>(D, S, T, ni, nl, force, stride);
     else

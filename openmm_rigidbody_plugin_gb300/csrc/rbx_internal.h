@@ -113,16 +113,16 @@ constexpr int kEnergyChunk = 2048;  // units per chunk of the potential energies
 // Cells (of units, by centroid) of all systems are numbered consecutively. Units are numbered as
 // listed (index u) and, from every list build on, by place in cell order (p), system by system.
 constexpr int kMaxUnit = 4;
-struct FFSys {
-    int a0, a1;   // device slots of the system's atoms
-    int i0, i1;   // its interacting atoms, as a range of the interacting-atom list
+struct alignas(16) FFSys {
     int u0, u1;   // its units (as indices u, and as places p)
     int c0, nc;   // first cell and cells per box edge of the list build (1: one cell, all pairs)
-    float L, invL, rc2, krf, crf;
+    float L, invL, rc, rc2;
+    float krf, crf;
     float rl;          // cutoff + skin: units are listed when their centroids lie within rl + both radii
     float half_skin2;  // (skin/2)^2: a centroid moved this far since the build invalidates the lists
     int pair_image;    // 1: cutoff + two radii may reach half the box; the force pass takes the
                        // minimum image per pair (else one shift per listed unit)
+    int pad[3];
 };
 struct FFDev {
     int S, n_int, n_units, n_cells;
@@ -141,6 +141,7 @@ struct FFDev {
     int* cell_cursor;     // [n_cells]
     float4* scen;         // [n_units] p: centroid and radius
     int* sgrp;            // [n_units] p: group
+    int2* sunit;          // [n_units] p: the unit's entry of `unit`
     // p: atom records x, y, z (at the image nearest the unit's centroid), type: record a of place p at
     // spos[a][p] (a < slots; those past the unit's atoms lie far outside every cutoff)
     float4* spos[kMaxUnit];
