@@ -752,9 +752,13 @@ __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, co
 // then spill a little and still gain: forces of 40 boxes with 64-type solutes take 1.09 ms at 128
 // registers, 0.98 at 80 and 0.97 at 64.
 constexpr int force_blocks(int records) { return records <= 3 ? 8 : 6; }
+// Batches of at most kFewUnits units (two warps per scheduler) leave the SMs nearly empty: a warp's own
+// chain of instructions is then the time, and 128 registers let more of it overlap (512 waters, 20 steps
+// with energies and a frame: 475 against 537 us; at 2600 units, 683 against 662).
+constexpr int kFewUnits = 8 * kSMs, kFewBlocks = 4;
 
-template <int JS, bool ENERGY, bool PT, bool RELAX>
-__global__ void __launch_bounds__(32 * kFW, force_blocks(JS)) ff_force(FFDev D, long long* __restrict__ force, int stride) {
+template <int JS, bool ENERGY, bool PT, bool RELAX, int BLOCKS>
+__global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long* __restrict__ force, int stride) {
     extern __shared__ float4 stab[];  // PT: the type-pair table
     __shared__ float4 ring[kFW][kRing];
     chain_release();
@@ -797,10 +801,12 @@ __global__ void __launch_bounds__(32 * kFW, force_blocks(JS)) ff_force(FFDev D, 
 template <int JS, bool ENERGY, bool RELAX>
 cudaError_t launch_force_kernel(const FFDev& D, long long* f, int stride, cudaStream_t st) {
     const int grid = (D.n_units + kFW - 1) / kFW;
-    if (D.ntypes)
-        return launch_chained(ff_force<JS, ENERGY, true, RELAX>, grid, 32 * kFW, sizeof(float4) * D.ntypes * D.ntypes, st,
-                              D, f, stride);
-    return launch_chained(ff_force<JS, ENERGY, false, RELAX>, grid, 32 * kFW, 0, st, D, f, stride);
+    if (!D.ntypes)
+        return launch_chained(ff_force<JS, ENERGY, false, RELAX, force_blocks(JS)>, grid, 32 * kFW, 0, st, D, f, stride);
+    const size_t table = sizeof(float4) * D.ntypes * D.ntypes;
+    if (!RELAX && D.n_units <= kFewUnits)
+        return launch_chained(ff_force<JS, ENERGY, true, RELAX, kFewBlocks>, grid, 32 * kFW, table, st, D, f, stride);
+    return launch_chained(ff_force<JS, ENERGY, true, RELAX, force_blocks(JS)>, grid, 32 * kFW, table, st, D, f, stride);
 }
 
 // A capped relaxation forms no energies.
