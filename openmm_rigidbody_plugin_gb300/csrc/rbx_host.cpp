@@ -350,11 +350,13 @@ void pack_tiles(rbx_integrator* h) {
     // system that fits one wave of resident tiles (3 per SM; 6 of the narrow shape) is spread over all
     // of it: the step is then a chain of latencies, shorter with fewer bodies per tile. Single/mixed,
     // part1 + fused + part2: 333 bodies 30.4 -> 23.3 us, 21,017 bodies 34.8 -> 32.8; twice as many tiles
-    // than fit cost 45 us there. Double precision is bound by each SM's FP64 pipe, so more and smaller
-    // tiles even the SMs out as long as warps stay full: 50,118 bodies 606 us in tiles of up to 512
-    // atoms, 575 at 3 tiles per SM, 503 at 6, 822 in half-empty warps.
+    // than fit cost 45 us there. Double precision is bound by each SM's FP64 pipe, so somewhat smaller
+    // tiles even the SMs out: exact rotation of 50,118 bodies of the mix 346 us in tiles of up to 512
+    // atoms, 340 at 3 tiles per SM, 326 at 4, 370 at 6 (a tile of 64 bodies holds 45 asymmetric tops, which
+    // take two warps as 64 would); of 50,000 waters 322 at 3, 265 at 4, 268 at 6. NO-SQUISH, 10 substeps,
+    // 50,118 bodies 534 at 3, 577 at 4, 555 at 6.
     const int nb = h->nb, TA = tile_atoms(h->prec, h->tile_threads);
-    const int wave = h->prec == PREC_DOUBLE ? 6 * kSMs : 3 * kSMs * (kThreadsF / h->tile_threads);
+    const int wave = h->prec == PREC_DOUBLE ? (h->mode == 0 ? 4 : 3) * kSMs : 3 * kSMs * (kThreadsF / h->tile_threads);
     const int per_tile = std::max(1, (nb + 32 * wave - 1) / (32 * wave)) * 32;
     const int TB = std::min(tile_bodies(h->prec, h->tile_threads), per_tile);
     h->tile_body0.assign(1, 0);

@@ -207,8 +207,10 @@ __global__ void sync_positions_kernel(DevSys S, DevBuf B) {
         const double* d = (const double*)S.d;
         const V3<double> r = v3<double>(st[b], st[b + nbp], st[b + 2 * nbp]);
         const Q4<double> q = q4<double>(st[b + 6 * nbp], st[b + 7 * nbp], st[b + 8 * nbp], st[b + 9 * nbp]);
+        double m[9];
+        rotation_matrix(q, m);
         for (int k = a0; k < a1; k++) {
-            const V3<double> delta = rotate_to_space(q, v3<double>(d[k], d[k + S.nba_pad], d[k + 2 * S.nba_pad]));
+            const V3<double> delta = mat_vec(m, v3<double>(d[k], d[k + S.nba_pad], d[k + 2 * S.nba_pad]));
             PosIO<P>::store(B, S.atom_loc[k], r, delta);
         }
     } else {

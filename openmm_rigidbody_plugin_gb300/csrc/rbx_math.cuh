@@ -75,6 +75,15 @@ template <class T> RBX_HD T tmin(T a, T b) { return a < b ? a : b; }
 template <class T> RBX_HD T tmax(T a, T b) { return a > b ? a : b; }
 template <class T> RBX_HD T tabs(T a) { return a < T(0) ? -a : a; }
 
+// x^(-1/2).
+template <class T> RBX_HD T inv_sqrt(T x) {
+#ifdef __CUDA_ARCH__
+    return rsqrt(x);
+#else
+    return T(1) / std::sqrt(x);
+#endif
+}
+
 // sin x and cos x. Rotation angles of one step are small: for |x| <= 1/4 the Maclaurin series to
 // x^13 and x^14 (truncation below 3e-21 relative, under FP64 rounding) replaces the general-range
 // functions, whose argument reduction is costly on GB300's narrow FP64 pipe; larger arguments take
@@ -161,7 +170,12 @@ template <class T> RBX_HD void symmetric_top_rotation(int k, T invIp, T invIk, V
 // RigidBody.cpp:241-308, evaluated in increment form for FP64 on GB300, whose FP64 rate is 1/64 of
 // FP32. The closed form spends dozens of FP64 divisions and square roots per body in its Carlson
 // iterations (RF, RJ) and AGM, and loses accuracy to cancellation at small rotations (its
-// third-kind integrals are differenced). This form spends about a dozen, 5.7x faster per step.
+// third-kind integrals are differenced). A division or square root costs about a dozen FP64
+// instructions, so this form is arranged to spend 17 and 7 of them: the quadrature nodes carry their
+// Jacobi functions and angular momentum as homogeneous coordinates (numerators over a common
+// denominator) and divide once each, and |L|, which the motion conserves, is not recomputed there.
+// With about 75 (a division per duplication, addition theorem, norm and rate) 50,118 bodies of a
+// mix took 497 us per part1 + fused + part2 instead of 376.
 // Against RK4 of the Euler equations in long double it is within 4e-16 (the closed form: 1.4e-11).
 // - L(t) in the body frame: the Jacobi functions at u0 + h from their values at u0, which the
 //   state fixes, by the addition theorem (Abramowitz & Stegun 16.17). The functions of the small
@@ -173,6 +187,51 @@ template <class T> RBX_HD void symmetric_top_rotation(int k, T invIp, T invIk, V
 //   about 4e-13 (wp dt)^10 of phi.
 // ---------------------------------------------------------------------------------------------
 
+// sn(h), cn(h) - 1, dn(h) - 1 of parameter m for |h| <= 1/32: Maclaurin series.
+template <class T> RBX_HD void jacobi_series(T h, T m, T& sn, T& cm1, T& dm1) {
+    const T u2 = h * h, m2 = m * m, m3 = m2 * m;
+    sn = h * (T(1) + u2 * (-(T(1) + m) * T(1.0 / 6) +
+                           u2 * ((T(1) + T(14) * m + m2) * T(1.0 / 120) +
+                                 u2 * (-(T(1) + T(135) * m + T(135) * m2 + m3) * T(1.0 / 5040) +
+                                       u2 * (T(1) + T(1228) * m + T(5478) * m2 + T(1228) * m3 + m2 * m2) *
+                                           T(1.0 / 362880)))));
+    cm1 = u2 * (T(-0.5) + u2 * ((T(1) + T(4) * m) * T(1.0 / 24) +
+                                u2 * (-(T(1) + T(44) * m + T(16) * m2) * T(1.0 / 720) +
+                                      u2 * (T(1) + T(408) * m + T(912) * m2 + T(64) * m3) * T(1.0 / 40320))));
+    dm1 = m * u2 * (T(-0.5) + u2 * ((T(4) + m) * T(1.0 / 24) +
+                                    u2 * (-(T(16) + T(44) * m + m2) * T(1.0 / 720) +
+                                          u2 * (T(64) + T(912) * m + T(408) * m2 + m3) * T(1.0 / 40320))));
+}
+
+// The three functions in homogeneous coordinates, sn = s/n, cn = c/n, dn = d/n, for any argument of
+// at most 2^60/32: no division in the duplications.
+template <class T> RBX_HD void jacobi_homogeneous(T h, T m, T& s, T& c, T& d, T& n) {
+    int k = 0;
+    while (tabs(h) > T(0.03125) && k < 60) {
+        h *= T(0.5);
+        k++;
+    }
+    jacobi_series(h, m, s, c, d);
+    c += T(1);
+    d += T(1);
+    n = T(1);
+    for (int i = 0; i < k; i++) {
+        const T s2 = s * s, c2 = c * c, d2 = d * d, n2 = n * n;
+        const T sn = T(2) * (s * c) * (d * n), cn = c2 * n2 - s2 * d2, dn = d2 * n2 - m * (s2 * c2);
+        n = n2 * n2 - m * (s2 * s2);
+        s = sn;
+        c = cn;
+        d = dn;
+        if (i % 4 == 3) {  // keep the common factor near 1 over many duplications
+            const T f = T(1) / n;
+            s *= f;
+            c *= f;
+            d *= f;
+            n = T(1);
+        }
+    }
+}
+
 // sn(h), cn(h) - 1, dn(h) - 1 of parameter m for a small argument.
 template <class T> RBX_HD void jacobi_small_t(T h, T m, T& sn, T& cm1, T& dm1) {
     int k = 0;
@@ -180,17 +239,7 @@ template <class T> RBX_HD void jacobi_small_t(T h, T m, T& sn, T& cm1, T& dm1) {
         h *= T(0.5);
         k++;
     }
-    const T u2 = h * h, m2 = m * m, m3 = m2 * m;
-    sn = h * (T(1) + u2 * (-(T(1) + m) / T(6) +
-                           u2 * ((T(1) + T(14) * m + m2) / T(120) +
-                                 u2 * (-(T(1) + T(135) * m + T(135) * m2 + m3) / T(5040) +
-                                       u2 * (T(1) + T(1228) * m + T(5478) * m2 + T(1228) * m3 + m2 * m2) / T(362880)))));
-    cm1 = u2 * (T(-0.5) + u2 * ((T(1) + T(4) * m) / T(24) +
-                                u2 * (-(T(1) + T(44) * m + T(16) * m2) / T(720) +
-                                      u2 * (T(1) + T(408) * m + T(912) * m2 + T(64) * m3) / T(40320))));
-    dm1 = m * u2 * (T(-0.5) + u2 * ((T(4) + m) / T(24) +
-                                    u2 * (-(T(16) + T(44) * m + m2) / T(720) +
-                                          u2 * (T(64) + T(912) * m + T(408) * m2 + m3) / T(40320))));
+    jacobi_series(h, m, sn, cm1, dm1);
     for (int i = 0; i < k; i++) {  // sn(2h) = 2 s c d / D, cn(2h) - 1 = -2 s^2 d^2 / D, dn(2h) - 1 = -2 m s^2 c^2 / D
         const T c = T(1) + cm1, d = T(1) + dm1, s2 = sn * sn;
         const T inv = T(1) / (T(1) - m * s2 * s2);
@@ -228,23 +277,26 @@ template <class T> RBX_HD void exact_rotation_increment(V3<T> I, V3<T> invI, Q4<
         // L^2 - 2K I2 and 2K I0 - L^2 as sums of non-negative terms
         const T r1 = Iw.x * Iw.x * (g02 * invI.x) + Iw.y * Iw.y * (g12 * invI.y);
         const T r3 = Iw.y * Iw.y * (g01 * invI.y) + Iw.z * Iw.z * (g02 * invI.z);
-        const T l1 = r1 * invI.y / g12, l3 = r3 * invI.y / g01;
-        const bool case1 = l1 < l3;  // L = I a (cn, sn, dn); otherwise I a (dn, sn, cn)
-        const T lmin = case1 ? l1 : l3, lmax = case1 ? l3 : l1;
+        // L = I a (cn, sn, dn) when r1/g12 < r3/g01 (case1); otherwise I a (dn, sn, cn)
+        const T p1 = r1 * g01, p3 = r3 * g12;
+        const bool case1 = p1 < p3;
+        const T m = case1 ? p1 / p3 : p3 / p1;
         const T c13 = T(1) / g02;
-        V3<T> a = v3<T>(sqrt(r1 * invI.x * c13), sqrt(lmin), sqrt(r3 * invI.z * c13));
-        if (w0.x < T(0)) a.x = -a.x;
-        if (w0.z < T(0)) a.z = -a.z;
-        const T m = lmin / lmax;
-        const T wp = -invI.y * a.x * a.z / (a.y * c13);
-        T s0 = w0.y / a.y;
+        // squares of the amplitudes a, their inverse roots, and the amplitudes
+        const V3<T> a2 = v3<T>(r1 * invI.x * c13, (case1 ? r1 : r3) * invI.y / (case1 ? g12 : g01), r3 * invI.z * c13);
+        V3<T> ia = v3<T>(inv_sqrt(a2.x), inv_sqrt(a2.y), inv_sqrt(a2.z));
+        if (w0.x < T(0)) ia.x = -ia.x;
+        if (w0.z < T(0)) ia.z = -ia.z;
+        const V3<T> a = mul(a2, ia);
+        const T wp = -invI.y * a.x * a.z * ia.y * g02;
+        T s0 = w0.y * ia.y;
         s0 = tmin(T(1), tmax(T(-1), s0));
-        const T cx = w0.x / a.x, cz = w0.z / a.z;
+        const T cx = w0.x * ia.x, cz = w0.z * ia.z;
         const T c0 = case1 ? cx : cz, d0 = case1 ? cz : cx;
         const V3<T> Ia = mul(I, a);
         const T ms0s0 = m * s0 * s0;
-        const T Lm = sqrt(Lsq);
-        const V3<T> n0 = Iw * (T(1) / Lm);
+        const T iLm = inv_sqrt(Lsq), Lm = Lsq * iLm;
+        const V3<T> n0 = Iw * iLm;
         auto dL = [&](T t) {  // L(t) - L(0)
             T sh, cm1, dm1;
             jacobi_small_t(wp * t, m, sh, cm1, dm1);
@@ -262,29 +314,38 @@ template <class T> RBX_HD void exact_rotation_increment(V3<T> I, V3<T> invI, Q4<
                           T(0.236926885056189087514264040720)};
         T phi = T(0);
         for (int i = 0; i < 5; i++) {
-            const V3<T> L = Iw + dL(T(0.5) * dt * (T(1) + glx[i]));
-            const V3<T> n = L * (T(1) / sqrt(dot(L, L)));
-            phi += glw[i] * dot(mul(invI, L), n + n0) / (T(1) + dot(n, n0));
+            // D L(t) by the addition theorem, D its denominator; with |L| = Lm the rate is
+            // (omega . L + Lm omega . n0) / (Lm + L . n0)
+            T s, c, d, n;
+            jacobi_homogeneous(wp * (T(0.5) * dt * (T(1) + glx[i])), m, s, c, d, n);
+            const T D = n * n - ms0s0 * (s * s);
+            const T S = s0 * (c * d) + (s * n) * (c0 * d0);
+            const T C = c0 * (c * n) - (s0 * d0) * (s * d), E = d0 * (d * n) - (m * s0 * c0) * (s * c);
+            const V3<T> L = case1 ? v3<T>(Ia.x * C, Ia.y * S, Ia.z * E) : v3<T>(Ia.x * E, Ia.y * S, Ia.z * C);
+            const V3<T> om = mul(invI, L);
+            const T LmD = Lm * D;
+            phi += glw[i] * (dot(om, L) + LmD * dot(om, n0)) / (D * (LmD + dot(L, n0)));
         }
         phi *= T(0.5) * dt;
         const V3<T> dLt = dL(dt);
         Lt = Iw + dLt;
-        const T Ltn = sqrt(dot(Lt, Lt));
+        const T Lt2 = dot(Lt, Lt), iLtn = inv_sqrt(Lt2), Ltn = Lt2 * iLtn;
         const T dLn = (T(2) * dot(Iw, dLt) + dot(dLt, dLt)) / (Ltn + Lm);  // |L(t)| - |L(0)|
-        const V3<T> dn = (dLt - n0 * dLn) * (T(1) / Ltn);                   // n - n0 without cancellation
+        const V3<T> dn = (dLt - n0 * dLn) * iLtn;                          // n - n0 without cancellation
         const T dn2 = dot(dn, dn);
-        const T mu0 = sqrt(tmax(T(1) - T(0.25) * dn2, T(0)));
-        const V3<T> nv = cross(dn, n0) * (T(0.5) / tmax(mu0, T(1e-300)));
-        const Q4<T> dmu = q4<T>(T(-0.25) * dn2 / (T(1) + mu0), nv.x, nv.y, nv.z);
+        const T mu2 = tmax(T(1) - T(0.25) * dn2, T(1e-300)), imu = inv_sqrt(mu2);
+        const V3<T> nv = cross(dn, n0) * (T(0.5) * imu);
+        const Q4<T> dmu = q4<T>(T(-0.25) * dn2 / (T(1) + mu2 * imu), nv.x, nv.y, nv.z);
         const Q4<T> de = axis_angle_increment(n0, phi);
         dr = de + dmu + qmul(de, dmu);
-        Lt = Lt * (Lm / Ltn);  // |L| is invariant: remove the rounding of its length
+        Lt = Lt * (Lm * iLtn);  // |L| is invariant: remove the rounding of its length
     }
     q = q + qmul(q, dr);
-    q = q * (T(1) / sqrt(dot(q, q)));
+    q = q * inv_sqrt(dot(q, q));
     // pi = 2 B(q) L(t) / |q|^2, so that Bt(q, pi) / 2 gives back L(t) exactly whatever the rounding of
     // the normalisation; without the division L and the energy drift by |q|^2 - 1 each step
-    pi = qB(q, Lt * (T(2) / dot(q, q)));
+    // (1/x = 2 - x to (1 - x)^2, about 1e-31 here)
+    pi = qB(q, Lt * (T(2) * (T(2) - dot(q, q))));
 }
 
 // Mode-0 free rotation for any body: closed forms for the degenerate classes, the elliptic

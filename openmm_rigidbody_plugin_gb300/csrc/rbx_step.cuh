@@ -156,11 +156,11 @@ static __device__ __noinline__ void flag_failure(unsigned int* status, uint8_t* 
     atomicAdd(status, 1u);
 }
 
-// Shared memory of the double-precision step kernel: sF, sT, sX 3*TA each; sQ 4*TB; sRb 3*TB
+// Shared memory of the double-precision step kernel: sF, sT, sX 3*TA each; sM 9*TB; sRb 3*TB
 // (double); sW 3*TB; sBody TA (uint16); sBig one word per warp.
 constexpr size_t step_smem_d() {
     constexpr int TA = kTileAtomsD, TB = kTileBodies;
-    return (size_t)3 * 3 * TA * sizeof(double) + 4 * TB * sizeof(double) + 3 * TB * sizeof(double) +
+    return (size_t)3 * 3 * TA * sizeof(double) + 9 * TB * sizeof(double) + 3 * TB * sizeof(double) +
            3 * TB * sizeof(double) + TA * sizeof(unsigned short) + (kThreads / 32) * sizeof(unsigned) + 64;
 }
 
@@ -314,9 +314,22 @@ __device__ __forceinline__ int block_tile(const DevSys& S) {
     return tile_of_block((int)blockIdx.x, S.n_body_tiles, S.n_free_tiles);
 }
 
+// At(q) as a row-major 3x3 matrix (homogeneous quadratic form, equal to Ct(q, B(q, .))).
+template <class T> __device__ __forceinline__ void rotation_matrix(Q4<T> q, T* m) {
+    const T ww = q.w * q.w, xx = q.x * q.x, yy = q.y * q.y, zz = q.z * q.z;
+    const T xy = q.x * q.y, xz = q.x * q.z, yz = q.y * q.z, wx = q.w * q.x, wy = q.w * q.y, wz = q.w * q.z;
+    m[0] = ww + xx - yy - zz; m[1] = T(2) * (xy - wz); m[2] = T(2) * (xz + wy);
+    m[3] = T(2) * (xy + wz); m[4] = ww - xx + yy - zz; m[5] = T(2) * (yz - wx);
+    m[6] = T(2) * (xz - wy); m[7] = T(2) * (yz + wx); m[8] = ww - xx - yy + zz;
+}
+template <class T> __device__ __forceinline__ V3<T> mat_vec(const T* m, V3<T> d) {
+    return v3<T>(fma(m[0], d.x, fma(m[1], d.y, m[2] * d.z)), fma(m[3], d.x, fma(m[4], d.y, m[5] * d.z)),
+                 fma(m[6], d.x, fma(m[7], d.y, m[8] * d.z)));
+}
+
 // Shared-memory carve-up common to both step kernels.
 template <class A> struct StepSmem {
-    A *sF, *sT, *sX, *sQ, *sW;
+    A *sF, *sT, *sX, *sM, *sW;  // sM: At(q) of each body
     double* sRb;
     unsigned short* sBody;
     unsigned* sBig;  // large-body ballots, one word per warp
@@ -324,8 +337,8 @@ template <class A> struct StepSmem {
         sF = (A*)smem;
         sT = sF + 3 * TA;
         sX = sT + 3 * TA;
-        sQ = sX + 3 * TA;
-        sRb = (double*)(sQ + 4 * TB);
+        sM = sX + 3 * TA;
+        sRb = (double*)(sM + 9 * TB);
         sW = (A*)(sRb + 3 * TB);
         sBody = (unsigned short*)(sW + 3 * TB);
         sBig = (unsigned*)(sBody + TA);
@@ -360,8 +373,7 @@ __device__ __forceinline__ void atom_forces(const DevSys& S, const DevBuf& B, co
         const int a = threadIdx.x + i * kThreads;
         if (a < nat) {
             const int t = sm.sBody[a];
-            Q4<A> q = q4<A>(sm.sQ[4 * t], sm.sQ[4 * t + 1], sm.sQ[4 * t + 2], sm.sQ[4 * t + 3]);
-            V3<A> delta = rotate_to_space(q, d[i]);
+            V3<A> delta = mat_vec(sm.sM + 9 * t, d[i]);
             V3<A> tau = cross(delta, F[i]);
             sm.sF[3 * a] = F[i].x; sm.sF[3 * a + 1] = F[i].y; sm.sF[3 * a + 2] = F[i].z;
             sm.sT[3 * a] = tau.x; sm.sT[3 * a + 1] = tau.y; sm.sT[3 * a + 2] = tau.z;
@@ -458,6 +470,9 @@ __device__ __forceinline__ void atom_velocities(const DevSys& S, const DevBuf& B
 
 // ------------------------------------------------------------------------------------------
 // Double precision: FP64 throughout, the plugin's formulas (RigidBody.cpp, rigidbodyintegrator.cu).
+// Bound: the FP64 pipe (two lanes per clock and SM), so the design spares FP64 instructions: a body's
+// rotation matrix once per phase (9 multiply-adds per atom instead of two quaternion products), few
+// divisions (rbx_math.cuh), warps of one rotation class.
 // ------------------------------------------------------------------------------------------
 // Free rotation of (q, pi) by dt in the integrator's rotation mode (double precision).
 template <bool EXACT>
@@ -495,10 +510,25 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
     double* st = (double*)S.state;
     chain_wait();
 
+    // The exact rotation takes the tile's bodies by rotation class (SORT): a warp executes the path of
+    // every class among its bodies, and an asymmetric top costs several times the others. 50,118 bodies of
+    // the mix, part1 + fused + part2: 326 against 376 us.
+    constexpr bool SORT = EXACT && KIND != STEP_PART2;
+    __shared__ unsigned short perm[SORT ? TB : 1], count[SORT ? kThreads / 32 : 1][4];
+    int cls = -1, rank = 0;
+    if (SORT) {
+        if (tid < nbt) cls = __ldg(S.cls + b0 + tid);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+            if (cls == c) rank = __popc(m & ((1u << (tid & 31)) - 1u));
+            if ((tid & 31) == 0) count[tid >> 5][c] = (unsigned short)__popc(m);
+        }
+    }
     bool big = false;
     if (tid < nbt) {
         const int b = b0 + tid;
-        for (int c = 0; c < 4; c++) sm.sQ[4 * tid + c] = st[b + (6 + c) * nbp];
+        rotation_matrix(q4<double>(st[b + 6 * nbp], st[b + 7 * nbp], st[b + 8 * nbp], st[b + 9 * nbp]), sm.sM + 9 * tid);
         const int s = __ldg(S.atom0 + b) - a0, e = __ldg(S.atom0 + b + 1) - a0;
         for (int j = s; j < e; j++) sm.sBody[j] = (unsigned short)tid;
         big = e - s > kWarpBody;
@@ -508,6 +538,12 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
         if ((tid & 31) == 0) sm.sBig[tid >> 5] = m;
     }
     __syncthreads();
+    if (SORT && tid < nbt) {
+        for (int c = 0; c <= cls; c++)
+            for (int w = 0; w < kThreads / 32; w++)
+                if (c < cls || w < (tid >> 5)) rank += count[w][c];
+        perm[rank] = (unsigned short)tid;
+    }
     atom_forces<P, KIND, double, double>(S, B, sm, a0, nat);
     __syncthreads();
     if (LARGE && count_large<kThreads / 32>(sm.sBig)) {
@@ -516,12 +552,12 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
         __syncthreads();
     }
     if (tid < nbt) {
-        const int b = b0 + tid;
+        const int t = SORT ? perm[tid] : tid, b = b0 + t;
         V3<double> Fa, Ta;
         const int s = __ldg(S.atom0 + b) - a0, e = __ldg(S.atom0 + b + 1) - a0;
         if (LARGE && e - s > kWarpBody) {
-            Fa = v3<double>(sm.sRb[3 * tid], sm.sRb[3 * tid + 1], sm.sRb[3 * tid + 2]);
-            Ta = v3<double>(sm.sW[3 * tid], sm.sW[3 * tid + 1], sm.sW[3 * tid + 2]);
+            Fa = v3<double>(sm.sRb[3 * t], sm.sRb[3 * t + 1], sm.sRb[3 * t + 2]);
+            Ta = v3<double>(sm.sW[3 * t], sm.sW[3 * t + 1], sm.sW[3 * t + 2]);
         } else {
             body_sums(sm, s, e, Fa, Ta);
         }
@@ -543,8 +579,8 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
         st[b + 3 * nbp] = v.x; st[b + 4 * nbp] = v.y; st[b + 5 * nbp] = v.z;
         if (KIND == STEP_PART2) {
             V3<double> ws = rotate_to_space(q, mul(invI, qBt(q, pi)) * 0.5);
-            sm.sRb[3 * tid] = v.x; sm.sRb[3 * tid + 1] = v.y; sm.sRb[3 * tid + 2] = v.z;
-            sm.sW[3 * tid] = ws.x; sm.sW[3 * tid + 1] = ws.y; sm.sW[3 * tid + 2] = ws.z;
+            sm.sRb[3 * t] = v.x; sm.sRb[3 * t + 1] = v.y; sm.sRb[3 * t + 2] = v.z;
+            sm.sW[3 * t] = ws.x; sm.sW[3 * t + 1] = ws.y; sm.sW[3 * t + 2] = ws.z;
             if (REF) {
                 // end of the stencils at t+h (rigidbodyintegrator.cu:380-384) and the body's terms of
                 // refinedKineticEnergies / potentialEnergyRefinement (:433-469), as corrections:
@@ -583,8 +619,8 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
                 rs[b + 3 * nbp] = sq.w; rs[b + 4 * nbp] = sq.x; rs[b + 5 * nbp] = sq.y; rs[b + 6 * nbp] = sq.z;
             }
             st[b] = r.x; st[b + nbp] = r.y; st[b + 2 * nbp] = r.z;
-            sm.sRb[3 * tid] = r.x; sm.sRb[3 * tid + 1] = r.y; sm.sRb[3 * tid + 2] = r.z;
-            sm.sQ[4 * tid] = q.w; sm.sQ[4 * tid + 1] = q.x; sm.sQ[4 * tid + 2] = q.y; sm.sQ[4 * tid + 3] = q.z;
+            sm.sRb[3 * t] = r.x; sm.sRb[3 * t + 1] = r.y; sm.sRb[3 * t + 2] = r.z;
+            rotation_matrix(q, sm.sM + 9 * t);
             st[b + 6 * nbp] = q.w; st[b + 7 * nbp] = q.x; st[b + 8 * nbp] = q.y; st[b + 9 * nbp] = q.z;
         }
         st[b + 10 * nbp] = pi.w; st[b + 11 * nbp] = pi.x; st[b + 12 * nbp] = pi.y; st[b + 13 * nbp] = pi.z;
@@ -599,8 +635,7 @@ __global__ void __launch_bounds__(kThreads, REF ? 1 : EXACT ? 2 : 3) step_kernel
         for (int a = tid; a < nat; a += kThreads) {
             const int t = sm.sBody[a];
             const int loc = __ldg(S.atom_loc + a0 + a);
-            Q4<double> q = q4<double>(sm.sQ[4 * t], sm.sQ[4 * t + 1], sm.sQ[4 * t + 2], sm.sQ[4 * t + 3]);
-            V3<double> delta = rotate_to_space(q, v3<double>(sm.sX[3 * a], sm.sX[3 * a + 1], sm.sX[3 * a + 2]));
+            V3<double> delta = mat_vec(sm.sM + 9 * t, v3<double>(sm.sX[3 * a], sm.sX[3 * a + 1], sm.sX[3 * a + 2]));
             PosIO<P>::store(B, loc, v3<double>(sm.sRb[3 * t], sm.sRb[3 * t + 1], sm.sRb[3 * t + 2]), delta);
         }
     }
@@ -623,19 +658,6 @@ template <int NT> struct FSmem {
     static constexpr int SG = SB + TA / 2;    // one word per warp: large-body ballots
     static constexpr int WORDS = SG + NT / 32;
 };
-
-// At(q) as a row-major 3x3 matrix (homogeneous quadratic form, equal to Ct(q, B(q, .))).
-__device__ __forceinline__ void rotation_matrix(Q4<float> q, float* m) {
-    const float ww = q.w * q.w, xx = q.x * q.x, yy = q.y * q.y, zz = q.z * q.z;
-    const float xy = q.x * q.y, xz = q.x * q.z, yz = q.y * q.z, wx = q.w * q.x, wy = q.w * q.y, wz = q.w * q.z;
-    m[0] = ww + xx - yy - zz; m[1] = 2.0f * (xy - wz); m[2] = 2.0f * (xz + wy);
-    m[3] = 2.0f * (xy + wz); m[4] = ww - xx + yy - zz; m[5] = 2.0f * (yz - wx);
-    m[6] = 2.0f * (xz - wy); m[7] = 2.0f * (yz + wx); m[8] = ww - xx - yy + zz;
-}
-__device__ __forceinline__ V3<float> mat_vec(const float* m, V3<float> d) {
-    return v3<float>(fmaf(m[0], d.x, fmaf(m[1], d.y, m[2] * d.z)), fmaf(m[3], d.x, fmaf(m[4], d.y, m[5] * d.z)),
-                     fmaf(m[6], d.x, fmaf(m[7], d.y, m[8] * d.z)));
-}
 
 // FP32 rotation increment dr (q <- q (x) (1 + dr)) for body angular momentum L over dt.
 template <bool EXACT>
