@@ -27,9 +27,8 @@ namespace {
 
 constexpr double kOne4PiEps0 = 138.935456;  // kJ nm / (mol e^2)
 // Neighbour-list skin (nm, of unit centroids). A longer list costs the force pass one distance test
-// per entry, a shorter one more builds: 256 boxes of the mix at 750 K take 19.7, 18.8, 18.3 and 17.9 ms
-// per 20 steps at 0.06, 0.09, 0.12 and 0.15 nm, 66,666 waters at 1100 K 7.5, 7.1, 7.2 and 7.0; at 300 K,
-// where lists last longer, the shorter ones gain, and their memory grows with the cube.
+// per entry, a shorter one more builds. 20 steps at 0.06, 0.08, 0.10, 0.12 and 0.14 nm: 256 boxes of the
+// mix at 750 K 15.1, 15.0, 15.0, 14.7 and 14.7 ms, 66,666 waters at 1100 K 4.62, 4.55, 4.52, 4.41 and 4.46.
 constexpr double kSkin = 0.12;
 
 #define BATCH_TRY(call)                                                                             \
@@ -107,10 +106,11 @@ struct rbx_batch {
     // force field
     DevArray<FFSys> d_sys;
     DevArray<int> d_iatom, d_ugrp, d_usys, d_place, d_unit_at, d_cell_count, d_cell_start, d_cell_cursor;
-    DevArray<int> d_sgrp, d_mc_cell, d_mc_sys, d_ncnt, d_atype;
+    DevArray<int> d_sgrp, d_ncnt, d_atype;
     DevArray<int2> d_unit, d_sunit;
     DevArray<float4> d_param, d_ucen, d_uref, d_scen, d_spos, d_spar, d_types;
     DevArray<unsigned char> d_moved, d_build;
+    DevArray<unsigned int> d_skey;      // FFDev::skey
     DevArray<unsigned int> d_nbr;       // neighbour lists of units (FFDev::nbr)
     DevArray<unsigned int> d_rebuilds;  // list builds per system (FFDev::rebuilds)
     // host copies for the set-up with a state: systems, cells allocated per system, unit layout
@@ -172,13 +172,19 @@ namespace {
 
 int check(const rbx_batch* b) { return b ? RBX_OK : set_error(RBX_ERR_INVALID_ARGUMENT, "null batch handle"); }
 
+// Cells of at least `edge` per box edge L, at most 256 and at most `most` in the box.
+int cells_per_edge(double L, double edge, int most) {
+    int nc = (int)std::min(256.0, std::floor(L / edge));
+    while (nc > 1 && (long long)nc * nc * nc > most) nc--;
+    return nc;
+}
+
 // Neighbour-list geometry for a state (host positions, user order): each unit's radius about its
 // centroid (constant for a rigid body), and from the largest radius of each system its list cells
 // (at least cutoff + skin + two radii per edge), the cell work list and the list capacity.
 int setup_lists(rbx_batch* b, const double* x) {
     const int S = b->S;
     std::vector<FFSys> sys = b->sys_h;
-    std::vector<int> mc_cell, mc_sys;
     std::vector<double> rho(S, 0.0);  // largest atom distance from a unit centroid
     for_each_system(sys, [&](int s) {
         const FFSys& f = sys[s];
@@ -211,16 +217,15 @@ int setup_lists(rbx_batch* b, const double* x) {
         // the device forms the radii in FP32: a margin of 1e-3 nm keeps its ones within the cells
         const double edge = (double)f.rl + 2.0 * rho_max + 1e-3;
         f.pair_image = std::sqrt((double)f.rc2) + 2.0 * rho_max + 1e-3 >= 0.5 * L ? 1 : 0;
-        int nc = (int)std::floor(L / edge);
-        if (nc > b->cells_alloc[s]) nc = b->cells_alloc[s];
-        if (nc < 3) nc = 1;
-        f.nc = nc;
-        if (nc > 1)
-            for (int c = 0; c < nc * nc * nc; c++) {
-                mc_cell.push_back(f.c0 + c);
-                mc_sys.push_back(s);
-            }
         const int U = f.u1 - f.u0;
+        // cells of half the reach where the box has five of them and they are not mostly empty, else of
+        // the whole reach, else one cell
+        const int half = cells_per_edge(L, 0.5 * edge, b->cells_alloc[s]), whole = cells_per_edge(L, edge, b->cells_alloc[s]);
+        const bool fine = half >= 5 && (long long)half * half * half <= 2LL * U;
+        const int nc = fine ? half : whole >= 3 ? whole : 1;
+        f.nc = nc;
+        f.win = fine ? 2 : 1;
+        f.reach = (float)((double)f.rl + rho_max + 1e-3);
         most_units = std::max<long long>(most_units, U);
         most_cells = std::max<long long>(most_cells, (long long)nc * nc * nc);
         const double reach = (double)f.rl + 2.0 * rho_max;
@@ -232,15 +237,10 @@ int setup_lists(rbx_batch* b, const double* x) {
     if (b->d_nbr.n < entries && b->d_nbr.alloc(entries) != cudaSuccess)
         return set_error(RBX_ERR_CUDA, "cudaMalloc of the neighbour lists failed (%d entries per unit)", cap);
     BATCH_TRY(cudaMemcpy(b->d_sys.p, sys.data(), sizeof(FFSys) * (size_t)S, cudaMemcpyHostToDevice));
-    if (!mc_cell.empty()) {
-        BATCH_TRY(cudaMemcpy(b->d_mc_cell.p, mc_cell.data(), sizeof(int) * mc_cell.size(), cudaMemcpyHostToDevice));
-        BATCH_TRY(cudaMemcpy(b->d_mc_sys.p, mc_sys.data(), sizeof(int) * mc_sys.size(), cudaMemcpyHostToDevice));
-    }
     FFDev& D = b->ff;
     const bool small = prep_limit(most_units, most_cells);
     D.prep_units = small ? (int)most_units : 0;
     D.prep_cells = small ? (int)most_cells : 0;
-    D.n_mc = (int)mc_cell.size();
     D.cap = cap;
     D.nbr = b->d_nbr.p;
     return RBX_OK;
@@ -471,13 +471,16 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         f.half_skin2 = (float)(0.25 * kSkin * kSkin);
         f.pair_image = 1;  // until the radii are known (rbx_batch_set_state)
         // cells for the largest grid any set of radii allows (the radii, known with the positions,
-        // can only make the cells larger and fewer)
-        int nc = (int)std::floor(L / (rc_s + kSkin));
-        if (nc < 3) nc = 1;
-        if (nc > 256) nc = 256;
+        // can only make the cells larger and fewer): of the whole reach, or of half of it while there
+        // are at most two per unit
+        const long long units_s = f.u1 - f.u0;
+        const int whole = cells_per_edge(L, rc_s + kSkin, 1 << 24), half = cells_per_edge(L, 0.5 * (rc_s + kSkin), 1 << 24);
+        const long long room = std::max<long long>((long long)whole * whole * whole,
+                                                   std::min((long long)half * half * half, 2 * units_s));
+        b->cells_alloc.push_back((int)std::max(1LL, room));
         f.c0 = cells;
-        f.nc = nc;
-        cells += nc * nc * nc;
+        f.nc = 1;
+        cells += b->cells_alloc[s];
         f.L = (float)L;
         f.invL = (float)(1.0 / L);
         f.rc = (float)rc_s;
@@ -487,8 +490,6 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         f.crf = (float)(1.0 / rc_s + krf * rc_s * rc_s);
     }
     b->sys_h = sys;
-    b->cells_alloc.resize(num_systems);
-    for (int s = 0; s < num_systems; s++) b->cells_alloc[s] = sys[s].nc;
     b->iatom_h = iatom;
     b->unit_h = unit;
     b->box_h.assign(box_edges, box_edges + num_systems);
@@ -545,8 +546,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
                 b->d_spos.alloc(records) != cudaSuccess || b->d_spar.alloc(types.empty() ? records : 0) != cudaSuccess ||
                 b->d_cell_count.alloc(cells) != cudaSuccess || b->d_cell_start.alloc(cells + 1) != cudaSuccess ||
                 b->d_cell_cursor.alloc(cells) != cudaSuccess || b->d_e_unit.alloc(u1) != cudaSuccess ||
-                b->d_mc_cell.alloc(std::max(cells, 1)) != cudaSuccess ||
-                b->d_mc_sys.alloc(std::max(cells, 1)) != cudaSuccess ||
+                b->d_skey.alloc(u1) != cudaSuccess ||
                 b->d_energy.alloc(num_systems) != cudaSuccess || b->d_ke.alloc(2 * (size_t)num_systems) != cudaSuccess ||
                 b->d_user.alloc(3 * (size_t)N) != cudaSuccess || b->d_sys_status.alloc(num_systems) != cudaSuccess ||
                 b->d_moved.alloc(num_systems) != cudaSuccess || b->d_build.alloc(num_systems) != cudaSuccess ||
@@ -607,9 +607,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.ntypes = (int)types.size();
     D.prep_units = 0;
     D.prep_cells = 0;
-    D.n_mc = 0;
-    D.mc_cell = b->d_mc_cell.p;
-    D.mc_sys = b->d_mc_sys.p;
+    D.skey = b->d_skey.p;
     // the owned OpenMM-layout buffers (forces of non-interacting atoms stay zero)
     rbx_buffers rb;
     if ((rc = rbx_context_buffers(b->integ, &rb))) { delete b; return rc; }
@@ -828,13 +826,14 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
     if (rc) return rc;
     if (!bytes) return set_error(RBX_ERR_INVALID_ARGUMENT, "null output");
     size_t n = b->d_sys.bytes() + b->d_iatom.bytes() + b->d_param.bytes() + b->d_unit.bytes() + b->d_ugrp.bytes() +
-               b->d_usys.bytes() + b->d_ucen.bytes() + b->d_uref.bytes() + b->d_place.bytes() + b->d_unit_at.bytes() +
-               b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
-               b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_sunit.bytes() + b->d_spos.bytes() + b->d_spar.bytes() + b->d_mc_cell.bytes() +
-               b->d_mc_sys.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() + b->d_build.bytes() + b->d_nbr.bytes() +
-               b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_e_unit.bytes() + b->d_energy.bytes() +
-               b->d_body0.bytes() + b->d_free0.bytes() + b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() +
-               b->ke_chunks.bytes() + b->e_chunks.bytes();
+               b->d_usys.bytes() + b->d_ucen.bytes() + b->d_uref.bytes() + b->d_place.bytes() +
+               b->d_unit_at.bytes() + b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
+               b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_sunit.bytes() + b->d_spos.bytes() + b->d_spar.bytes() +
+               b->d_skey.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() +
+               b->d_build.bytes() + b->d_nbr.bytes() + b->d_ncnt.bytes() + b->d_rebuilds.bytes() +
+               b->d_e_unit.bytes() + b->d_energy.bytes() + b->d_body0.bytes() + b->d_free0.bytes() +
+               b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() + b->ke_chunks.bytes() +
+               b->e_chunks.bytes();
     *bytes = n + (b->integ ? device_bytes(b->integ) : 0);
     return RBX_OK;
 }

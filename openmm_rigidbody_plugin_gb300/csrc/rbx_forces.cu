@@ -18,7 +18,7 @@
 //               build; lists that stay get their atoms' records at their places in cell order, the
 //               others a new cell order first (cells of at least cutoff + skin + twice the largest
 //               radius per edge, counted, scanned and sorted in shared memory)
-// and the others the same in kernels over all units (ff_check, ff_bin, ff_scan, ff_scatter, ff_sort,
+// and the others the same in kernels over all units (ff_check, ff_bin, ff_scan, ff_scatter,
 // ff_place; those after ff_check return at once for systems whose lists stay). Then
 //   ff_force    one warp per unit (all systems). Where the lists are to be rebuilt the warp first
 //               builds its own: the units in range among the 27 cells around it (or, in a
@@ -159,6 +159,30 @@ __device__ __forceinline__ void settle(const FFDev& D, const DevBuf& B, int prec
     D.uref[u] = c;
 }
 
+// Exclusive scan of n counts by a block: each thread a run of them, the runs' sums by warp shuffles.
+// put(i, start) receives every start; count(i) is read once. Returns nothing; ends without a barrier.
+template <class Count, class Put>
+__device__ __forceinline__ void block_scan(int n, int* wsum, const Count& count, const Put& put) {
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int per = (n + nthr - 1) / nthr, i0 = min(tid * per, n), i1 = min(i0 + per, n);
+    int sum = 0;
+    for (int i = i0; i < i1; i++) sum += count(i);
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((tid & 31) >= o) incl += v;
+    }
+    if ((tid & 31) == 31) wsum[tid >> 5] = incl;
+    __syncthreads();
+    int at = incl - sum;
+    for (int w = 0; w < (tid >> 5); w++) at += wsum[w];
+    for (int i = i0; i < i1; i++) {
+        const int c = count(i);
+        put(i, at);
+        at += c;
+    }
+}
+
 // Everything before the force pass for one system, in one block. The cell counts and the keys of the
 // system's units, in cell order, are in shared memory. Within a cell units are ranked by key (all
 // different), so the order does not depend on the order of the atomics.
@@ -199,25 +223,11 @@ __global__ void __launch_bounds__(1024) ff_prep(FFDev D, DevBuf B, int prec) {
     __syncthreads();
     for (int u = S.u0 + tid; u < S.u1; u += nthr) atomicAdd(cell + cell_index(S, D.ucen[u]), 1);
     __syncthreads();
-    // exclusive scan of the counts: each thread a run of cells, the runs' sums by warp shuffles
-    const int per = (ncell + nthr - 1) / nthr, i0 = min(tid * per, ncell), i1 = min(i0 + per, ncell);
-    int sum = 0;
-    for (int i = i0; i < i1; i++) sum += cell[i];
-    int incl = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((tid & 31) >= o) incl += v;
-    }
-    if ((tid & 31) == 31) wsum[tid >> 5] = incl;
-    __syncthreads();
-    int at = incl - sum;
-    for (int w = 0; w < (tid >> 5); w++) at += wsum[w];
-    for (int i = i0; i < i1; i++) {
-        const int n = cell[i];
-        cell[i] = at;
-        D.cell_start[S.c0 + i] = S.u0 + at;
-        at += n;
-    }
+    block_scan(ncell, wsum, [&](int i) { return cell[i]; },
+               [&](int i, int at) {
+                   cell[i] = at;
+                   D.cell_start[S.c0 + i] = S.u0 + at;
+               });
     if (tid == 0) D.cell_start[S.c0 + ncell] = S.u1;
     __syncthreads();
     for (int u = S.u0 + tid; u < S.u1; u += nthr) {
@@ -268,44 +278,32 @@ __global__ void ff_bin(FFDev D) {
     if (S.nc > 1) atomicAdd(D.cell_count + S.c0 + cell_index(S, D.ucen[u]), 1);
 }
 
-// Exclusive scan of one system's cell counts, in chunks of blockDim.x; the counts are reset.
-__global__ void ff_scan(FFDev D) {
-    __shared__ int s[256];
+// One block per system: its cells' starts, the counts reset, and whether its lists are rebuilt.
+__global__ void __launch_bounds__(1024) ff_scan(FFDev D) {
+    __shared__ int wsum[32];
     chain_release();
     chain_wait();
-    const bool build = rebuilding(D, blockIdx.x);
+    const int s = blockIdx.x;
+    const bool build = rebuilding(D, s);
     if (threadIdx.x == 0) {
-        D.build[blockIdx.x] = build;
-        if (build) D.rebuilds[blockIdx.x]++;
+        D.build[s] = build;
+        if (build) D.rebuilds[s]++;
     }
     if (!build) return;
-    const FFSys S = D.sys[blockIdx.x];
-    const int ncell = S.nc * S.nc * S.nc;
+    const FFSys S = D.sys[s];
     if (S.nc == 1) return;
-    int base = S.u0;
-    for (int c0 = 0; c0 < ncell; c0 += blockDim.x) {
-        const int c = c0 + threadIdx.x;
-        const int v = c < ncell ? D.cell_count[S.c0 + c] : 0;
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < (int)blockDim.x; o <<= 1) {  // Hillis-Steele inclusive scan
-            const int t = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (c < ncell) {
-            const int start = base + s[threadIdx.x] - v;
-            D.cell_start[S.c0 + c] = start;
-            D.cell_cursor[S.c0 + c] = start;
-            D.cell_count[S.c0 + c] = 0;
-        }
-        base += s[blockDim.x - 1];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) D.cell_start[S.c0 + ncell] = base;  // equals S.u1
+    const int ncell = S.nc * S.nc * S.nc;
+    int* count = D.cell_count + S.c0;
+    block_scan(ncell, wsum, [&](int i) { return count[i]; },
+               [&](int i, int at) {
+                   D.cell_start[S.c0 + i] = S.u0 + at;
+                   D.cell_cursor[S.c0 + i] = S.u0 + at;
+                   count[i] = 0;
+               });
+    if (threadIdx.x == 0) D.cell_start[S.c0 + ncell] = S.u1;
 }
 
+// Keys of the units of multi-cell boxes, cell by cell (in the order of the atomics).
 __global__ void ff_scatter(FFDev D) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     chain_release();
@@ -314,156 +312,149 @@ __global__ void ff_scatter(FFDev D) {
     const int s = D.usys[u];
     if (!rebuilding(D, s)) return;
     const FFSys S = D.sys[s];
-    if (S.nc == 1) {
-        D.unit_at[u] = u;  // one cell: unit order
-        return;
-    }
+    if (S.nc == 1) return;
     const float4 c = D.ucen[u];
-    D.unit_at[atomicAdd(D.cell_cursor + S.c0 + cell_index(S, c), 1)] = (int)cell_key(S, c, u);
+    D.skey[atomicAdd(D.cell_cursor + S.c0 + cell_index(S, c), 1)] = cell_key(S, c, u);
 }
 
-// Sort each cell of a multi-cell box by its units' keys, so that every cell, and so every list, is in
-// a fixed order. One warp per cell: the cell is staged in shared memory and each lane ranks its
-// entries against all of them (the entries are distinct, so the ranks are a permutation); a cell
-// larger than the stage falls back to an insertion sort by one lane.
-constexpr int kSortWarps = 4, kSortStage = 512;
-__global__ void __launch_bounds__(32 * kSortWarps) ff_sort(FFDev D) {
-    __shared__ unsigned int stage[kSortWarps][kSortStage];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int w = blockIdx.x * kSortWarps + warp;
-    chain_release();
-    chain_wait();
-    if (w >= D.n_mc) return;
-    const int sy = D.mc_sys[w];
-    if (!rebuilding(D, sy)) return;
-    const int c = D.mc_cell[w], u0 = D.sys[sy].u0;
-    const int b = D.cell_start[c], e = D.cell_start[c + 1], n = e - b;
-    unsigned int* key = (unsigned int*)D.unit_at + b;
-    unsigned int* s = stage[warp];
-    if (n <= kSortStage) {
-        for (int i = lane; i < n; i += 32) s[i] = key[i];
-        __syncwarp();
-        for (int i = lane; i < n; i += 32) {
-            const unsigned int v = s[i];
-            int rank = 0;
-            for (int j = 0; j < n; j++) rank += s[j] < v;
-            key[rank] = u0 + (v & kKeyUnit);
-        }
-    } else if (lane == 0) {
-        for (int i = 1; i < n; i++) {
-            const unsigned int v = key[i];
-            int j = i - 1;
-            while (j >= 0 && key[j] > v) {
-                key[j + 1] = key[j];
-                j--;
-            }
-            key[j + 1] = v;
-        }
-        for (int i = 0; i < n; i++) key[i] = u0 + (key[i] & kKeyUnit);
-    }
-}
-
+// Every unit of the rebuilt systems at its place: in its cell, by rank of its key (single-cell boxes:
+// unit order).
 __global__ void ff_place(FFDev D, DevBuf B, int prec) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     chain_release();
     chain_wait();
-    if (p >= D.n_units) return;
-    const int s = D.usys[p];  // places [u0, u1) belong to the system of unit p
-    if (rebuilding(D, s)) settle(D, B, prec, D.sys[s], D.unit_at[p], p);
+    if (i >= D.n_units) return;
+    const int s = D.usys[i];  // places [u0, u1) belong to the system of unit i
+    if (!rebuilding(D, s)) return;
+    const FFSys S = D.sys[s];
+    if (S.nc == 1) return settle(D, B, prec, S, i, i);
+    const unsigned int key = D.skey[i];
+    const int u = S.u0 + (int)(key & kKeyUnit);
+    const int* start = D.cell_start + S.c0 + cell_index(S, D.ucen[u]);
+    const int b = start[0], e = start[1];
+    int rank = 0;
+    for (int j = b; j < e; j++) rank += D.skey[j] < key;
+    settle(D, B, prec, S, u, b + rank);
 }
 
-// Lists, a warp per unit: the lanes test 32 candidates at a time (their centroids and groups lie in place
-// order, so a row of neighbour cells is one contiguous run) and append the ones in range in order, a
-// ballot giving each its slot. Against one thread per unit of a cell walking the 27 cells staged in
-// shared memory, no lane idles (a cell holds about 48 units of 128 threads) and the list is written
-// coalesced. A full list marks the system as failed (the capacity is sized from the densest system with
-// a wide margin, so this does not happen in a liquid).
-// Bound: load latency. The bounds of all runs are fetched at once, a run per lane, and kAhead chunks of
-// candidates are in flight. Measured per 20 steps: 512 waters 548, 528 and 531 us with 1, 2 and 4 chunks,
-// 256 boxes of the mix 18.4, 18.1 and 18.3 ms. Built by the force pass itself: a kernel of its own, which
-// has nothing to do in most steps, cost 588 us and 19.0 ms.
-// Returns the length of the list of the unit at place p with centroid c.
-__device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p, int s, float4 c, int lane) {
+// Lists, a warp per unit: the lanes test 32 candidates at a time and append the ones in range in order,
+// a ballot giving each its slot (coalesced). The candidates are the units of the cells within reach,
+// row of cells by row: in place order a row is one contiguous run (two where it crosses the box's
+// edge), trimmed to the chord of the reach through the row, and the runs are taken as one sequence, so
+// that the lanes stay full however short they are. A full list marks the system as failed (the capacity
+// is sized from the densest system with a wide margin, so this does not happen in a liquid).
+// Bound: load latency and issue. Cells of half the reach, trimmed, leave about 650 candidates of a
+// water's 214 entries; cells of the whole reach (27 of them, untrimmed) had 1600. 20 steps with energies
+// and a frame: 66,666 waters 5.0 -> 4.4 ms, 256 boxes of the mix 16.3 -> 14.7; forces of 15,001 bodies
+// 0.32 -> 0.26. kAhead chunks of
+// candidates are in flight. Built by the force pass itself: a kernel of its own, which has nothing to do
+// in most steps, cost 588 against 531 us per 20 steps of 512 waters.
+// Returns the length of the list of the unit at place p with centroid c; runs: scratch of 32 records.
+__device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p, int s, float4 c, int lane, float4* runs) {
     constexpr unsigned int kAll = 0xffffffffu;
     constexpr int kAhead = 2;
     const int grp = D.sgrp[p];
     unsigned int* list = D.nbr + (size_t)p * D.cap;
-    // lane's run of places [r0, r1) and its periodic shift: the whole box (minimum image per pair) or, of
-    // the cells around the unit's own, a row of up to three inside the box (lanes 0 to 8) or the one
-    // across its edge (9 to 17). The shifts are exact for units in range: a cell edge is at least
-    // cutoff + skin + twice the largest radius, and there are at least three per edge.
-    const bool image = S.nc == 1;
-    int r0 = 0, r1 = 0, runs = 1;
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    if (image) {
-        r0 = S.u0;
-        r1 = S.u1;
-    } else {
-        const int nc = S.nc;
-        const int cx = wrap_cell(c.x, S.invL, nc), cy = wrap_cell(c.y, S.invL, nc), cz = wrap_cell(c.z, S.invL, nc);
-        const bool edge = cx == 0 || cx == nc - 1;
-        runs = edge ? 18 : 9;
-        if (lane < runs) {
-            int z = cz + lane % 9 / 3 - 1, y = cy + lane % 3 - 1;
-            sz = z < 0 ? -S.L : (z >= nc ? S.L : 0.f);
-            z = z < 0 ? z + nc : (z >= nc ? z - nc : z);
-            sy = y < 0 ? -S.L : (y >= nc ? S.L : 0.f);
-            y = y < 0 ? y + nc : (y >= nc ? y - nc : y);
-            const int* row = D.cell_start + S.c0 + (z * nc + y) * nc;
-            const int x0 = lane < 9 ? max(cx - 1, 0) : (cx == 0 ? nc - 1 : 0);
-            const int x1 = lane < 9 ? min(cx + 1, nc - 1) : x0;
-            sx = lane < 9 ? 0.f : (cx == 0 ? -S.L : S.L);
-            r0 = row[x0];
-            r1 = row[x1 + 1];
+    const bool image = S.nc == 1;  // one run, the whole box: minimum image per pair
+    const int nc = S.nc, w = S.win, side = 2 * w + 1;
+    const int cx = wrap_cell(c.x, S.invL, nc), cy = wrap_cell(c.y, S.invL, nc), cz = wrap_cell(c.z, S.invL, nc);
+    // the lane's row of cells: the cells xa to xb of it are within reach, in an unwrapped count
+    int xa = 0, xb = -1;
+    const int* row = nullptr;
+    float sy = 0.f, sz = 0.f;
+    if (!image && lane < side * side) {
+        int z = cz + lane / side - w, y = cy + lane % side - w;
+        const float e = S.L / (float)nc, ie = S.invL * (float)nc, reach = S.reach + c.w;
+        const float tz = fmaxf(fmaxf((float)z * e - c.z, c.z - (float)(z + 1) * e), 0.0f);
+        const float ty = fmaxf(fmaxf((float)y * e - c.y, c.y - (float)(y + 1) * e), 0.0f);
+        const float h2 = reach * reach - fmaf(ty, ty, tz * tz);
+        if (h2 > 0.0f) {
+            const float h = sqrtf(h2);
+            xa = max((int)floorf((c.x - h) * ie), cx - w);
+            xb = min((int)floorf((c.x + h) * ie), cx + w);
         }
+        sz = z < 0 ? -S.L : (z >= nc ? S.L : 0.f);
+        z = z < 0 ? z + nc : (z >= nc ? z - nc : z);
+        sy = y < 0 ? -S.L : (y >= nc ? S.L : 0.f);
+        y = y < 0 ? y + nc : (y >= nc ? y - nc : y);
+        row = D.cell_start + S.c0 + (z * nc + y) * nc;
     }
-    int run = 0, n = 0, q0 = __shfl_sync(kAll, r0, 0), q1 = __shfl_sync(kAll, r1, 0);
-    float hx = __shfl_sync(kAll, sx, 0), hy = __shfl_sync(kAll, sy, 0), hz = __shfl_sync(kAll, sz, 0);
-    bool more = true;  // chunks left: the next begins at q0 of the run that ends at q1
-    auto settle_run = [&]() {
-        while (q0 >= q1) {
-            if (++run >= runs) {
-                more = false;
-                return;
+    int n = 0;
+    // the parts of the rows inside the box, then the parts across its edge. The periodic shifts are exact
+    // for units in range: there are at least 2 w + 1 cells per edge.
+    const int parts = !image && (cx < w || cx >= nc - w) ? 2 : 1;
+    for (int part = 0; part < parts; part++) {
+        int r0 = 0, r1 = 0;
+        float sx = 0.f;
+        if (image) {
+            if (lane == 0) {
+                r0 = S.u0;
+                r1 = S.u1;
             }
-            q0 = __shfl_sync(kAll, r0, run);
-            q1 = __shfl_sync(kAll, r1, run);
-            hx = __shfl_sync(kAll, sx, run);
-            hy = __shfl_sync(kAll, sy, run);
-            hz = __shfl_sync(kAll, sz, run);
+        } else {
+            int a = xa, b = xb;
+            if (part == 0) {
+                a = max(a, 0);
+                b = min(b, nc - 1);
+            } else if (cx < w) {
+                sx = -S.L;
+                a += nc;
+                b = min(b, -1) + nc;
+            } else {
+                sx = S.L;
+                a = max(a, nc) - nc;
+                b -= nc;
+            }
+            if (a <= b) {
+                r0 = row[a];
+                r1 = row[b + 1];
+            }
         }
-    };
-    settle_run();
-    while (more) {
-        int q[kAhead], gq[kAhead];
-        float4 cq[kAhead];
+        // the runs that hold anything, packed: run k covers the sequence from first[k] on
+        int first = r1 - r0;
+        const bool any = first > 0;
+        const int len = first;
 #pragma unroll
-        for (int k = 0; k < kAhead; k++) {
-            q[k] = more && q0 + lane < q1 ? q0 + lane : -1;
-            cq[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            gq[k] = grp;
-            if (q[k] >= 0) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kAll, first, o);
+            if (lane >= o) first += v;
+        }
+        const int total = __shfl_sync(kAll, first, 31);
+        first -= len;
+        const unsigned int held = __ballot_sync(kAll, any);
+        __syncwarp();
+        if (any) runs[__popc(held & ((1u << lane) - 1u))] = make_float4(__int_as_float(r0 - first), sy, sz, 0.0f);
+        __syncwarp();
+        int before = 0;  // runs that begin before the chunk
+        for (int f0 = 0; f0 < total; f0 += 32 * kAhead) {
+            int q[kAhead], gq[kAhead];
+            float4 cq[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; k++) {
+                const int f = f0 + 32 * k, at = first - f;
+                const unsigned int begins = __reduce_or_sync(kAll, any && at >= 0 && at < 32 ? 1u << at : 0u);
+                const int r = before + __popc(begins & (0xffffffffu >> (31 - lane))) - 1;
+                before += __popc(begins);
+                const float4 run = runs[max(r, 0)];
+                const bool on = f + lane < total;
+                q[k] = on ? __float_as_int(run.x) + f + lane : S.u0;
                 cq[k] = D.scen[q[k]];
-                gq[k] = D.sgrp[q[k]];
+                gq[k] = on ? D.sgrp[q[k]] : grp;
+                cq[k].x += sx;
+                cq[k].y += run.y;
+                cq[k].z += run.z;
             }
-            cq[k].x += hx;
-            cq[k].y += hy;
-            cq[k].z += hz;
-            if (more) {
-                q0 += 32;
-                settle_run();
-            }
-        }
 #pragma unroll
-        for (int k = 0; k < kAhead; k++) {
-            float3 d = make_float3(c.x - cq[k].x, c.y - cq[k].y, c.z - cq[k].z);
-            if (image) d = min_image(d.x, d.y, d.z, S);
-            const float lim = S.rl + c.w + cq[k].w;
-            const bool hit = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) < lim * lim && gq[k] != grp;
-            const unsigned int m = __ballot_sync(kAll, hit);
-            const int at = n + __popc(m & ((1u << lane) - 1u));
-            if (hit && at < D.cap) list[at] = (unsigned int)(q[k] - S.u0);
-            n += __popc(m);
+            for (int k = 0; k < kAhead; k++) {
+                float3 d = make_float3(c.x - cq[k].x, c.y - cq[k].y, c.z - cq[k].z);
+                if (image) d = min_image(d.x, d.y, d.z, S);
+                const float lim = S.rl + c.w + cq[k].w;
+                const bool hit = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) < lim * lim && gq[k] != grp;
+                const unsigned int m = __ballot_sync(kAll, hit);
+                const int at = n + __popc(m & ((1u << lane) - 1u));
+                if (hit && at < D.cap) list[at] = (unsigned int)(q[k] - S.u0);
+                n += __popc(m);
+            }
         }
     }
     if (lane == 0) {
@@ -750,8 +741,10 @@ __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, co
 
 // Blocks per SM: 64 registers a thread (32 warps per SM); 80 for units of four atoms. The larger variants
 // then spill a little and still gain: forces of 40 boxes with 64-type solutes take 1.09 ms at 128
-// registers, 0.98 at 80 and 0.97 at 64.
+// registers, 0.98 at 80 and 0.97 at 64 (later, with the list build's code, 0.75 at 80 and 0.77 at 64: the
+// form without the type-pair table takes 80).
 constexpr int force_blocks(int records) { return records <= 3 ? 8 : 6; }
+constexpr int kUntypedBlocks = 6;
 // Batches of at most kFewUnits units (two warps per scheduler) leave the SMs nearly empty: a warp's own
 // chain of instructions is then the time, and 128 registers let more of it overlap (512 waters, 20 steps
 // with energies and a frame: 475 against 537 us; at 2600 units, 683 against 662).
@@ -785,7 +778,7 @@ __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long*
     T.q0 = (int)nb[T.lane];
     T.q1 = (int)nb[min(32 + T.lane, D.cap - 1)];
     if (D.build[T.s]) {
-        T.n = build_list(D, S, T.p, T.s, T.c, T.lane);
+        T.n = build_list(D, S, T.p, T.s, T.c, T.lane, T.ring);
         T.q0 = (int)nb[T.lane];
         T.q1 = (int)nb[min(32 + T.lane, D.cap - 1)];
     }
@@ -802,7 +795,7 @@ template <int JS, bool ENERGY, bool RELAX>
 cudaError_t launch_force_kernel(const FFDev& D, long long* f, int stride, cudaStream_t st) {
     const int grid = (D.n_units + kFW - 1) / kFW;
     if (!D.ntypes)
-        return launch_chained(ff_force<JS, ENERGY, false, RELAX, force_blocks(JS)>, grid, 32 * kFW, 0, st, D, f, stride);
+        return launch_chained(ff_force<JS, ENERGY, false, RELAX, kUntypedBlocks>, grid, 32 * kFW, 0, st, D, f, stride);
     const size_t table = sizeof(float4) * D.ntypes * D.ntypes;
     if (!RELAX && D.n_units <= kFewUnits)
         return launch_chained(ff_force<JS, ENERGY, true, RELAX, kFewBlocks>, grid, 32 * kFW, table, st, D, f, stride);
@@ -863,9 +856,8 @@ int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* 
     } else {
         put(launch_chained(ff_check, gg, t, 0, st, D, B, prec));
         put(launch_chained(ff_bin, gg, t, 0, st, D));
-        put(launch_chained(ff_scan, D.S, 256, 0, st, D));
+        put(launch_chained(ff_scan, D.S, 1024, 0, st, D));
         put(launch_chained(ff_scatter, gg, t, 0, st, D));
-        if (D.n_mc) put(launch_chained(ff_sort, (D.n_mc + kSortWarps - 1) / kSortWarps, 32 * kSortWarps, 0, st, D));
         put(launch_chained(ff_place, gg, t, 0, st, D, B, prec));
     }
     long long* f = const_cast<long long*>(B.force);

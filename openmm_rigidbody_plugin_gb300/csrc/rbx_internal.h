@@ -122,7 +122,10 @@ struct alignas(16) FFSys {
     float half_skin2;  // (skin/2)^2: a centroid moved this far since the build invalidates the lists
     int pair_image;    // 1: cutoff + two radii may reach half the box; the force pass takes the
                        // minimum image per pair (else one shift per listed unit)
-    int pad[3];
+    float reach;       // rl + the system's largest radius (and a margin): a unit's list lies within this
+                       // + its own radius
+    int win;           // cells on either side of a unit's own that may hold listed units (1 or 2)
+    int pad;
 };
 struct FFDev {
     int S, n_int, n_units, n_cells;
@@ -139,6 +142,7 @@ struct FFDev {
     int* cell_count;      // [n_cells], zero between evaluations
     int* cell_start;      // [n_cells + 1] (entry c0 + nc^3 of each system ends it)
     int* cell_cursor;     // [n_cells]
+    unsigned int* skey;   // [n_units] keys of the units, cell by cell (cell_key)
     float4* scen;         // [n_units] p: centroid and radius
     int* sgrp;            // [n_units] p: group
     int2* sunit;          // [n_units] p: the unit's entry of `unit`
@@ -174,10 +178,6 @@ struct FFDev {
     // the largest system's units and list cells, where every system is small enough for one block
     // (prep_limit); prep_units = 0 otherwise
     int prep_units, prep_cells;
-    // work list of the cell sort (set with the state): every cell of the multi-cell boxes with its system
-    int n_mc;
-    const int* mc_cell;
-    const int* mc_sys;
 };
 constexpr int kMaxTypes = 32;  // atom types of the type-pair table (FFDev::types)
 // Interacting atoms of one system (a limit of this interface: list entries are 32-bit words).

@@ -2,7 +2,8 @@
 the force pass changes form: bodies of 1 to 4 atoms (one unit of neighbour lists), 5, 8, 13 and 45
 (several units), bodies with and without Lennard-Jones on their last atoms, atoms without any
 interaction between them, few atom types (pair table) and more than 32, boxes of one list cell (with
-and without the minimum image per pair) and of many.
+and without the minimum image per pair), of cells of half the reach (five an edge and more) and, where
+sparse, of the whole reach (three and more).
 
 Tolerances, as in test_gpu_forces.py: FP32 pair terms and sums from FP32 positions hold 99.9 % of the
 atoms to 2e-5 of the largest force, and a pair within rounding of the cutoff, which may count on one
@@ -48,6 +49,8 @@ def _box(rng, sizes, edge, types):
     ("threes", [3] * 400, 4.4, 0.8),
     ("fours", [4] * 300, 4.6, 0.9),
     ("many", [1] * 90 + [2] * 60 + [3] * 120 + [4] * 40 + [5] * 30 + [8] * 20 + [13] * 6 + [45] * 2, 5.2, 0.85),
+    ("sparse", [3] * 60, 7.0, 0.8),
+    ("sparse, three cells an edge", [1] * 30 + [3] * 30 + [8] * 4, 4.0, 0.9),
     ("one body and one atom", [45, 1], 2.2, 0.9)])
 def test_forces_of_bodies_of_every_size(oracle_mod, name, sizes, edge, cutoff, types):
     from openmm_rigidbody_plugin_gb300 import batch, build
