@@ -666,9 +666,21 @@ __device__ __forceinline__ Q4<float> rotation_increment(const DevSys& S, int b, 
     return nosquish_increment(L, R, R.invI.z != 0.0f, dt, S.rot_n);
 }
 
+// qBt with its roundings written out: which product of a pair the compiler fuses may change with the
+// code around it (it did for NO-SQUISH, from one instantiation and one version of the kernel to the
+// next), and positions are kept to 48 bits.
+__device__ __forceinline__ V3<float> body_momentum2(Q4<float> q, Q4<float> y) {
+    const float x0 = __fmaf_rn(-q.x, y.w, __fmul_rn(q.w, y.x));
+    const float y0 = __fmaf_rn(-q.y, y.w, -__fmul_rn(q.z, y.x));
+    const float z0 = __fmaf_rn(q.y, y.x, -__fmul_rn(q.z, y.w));
+    return v3<float>(__fmaf_rn(-q.y, y.z, __fmaf_rn(q.z, y.y, x0)), __fmaf_rn(q.x, y.z, __fmaf_rn(q.w, y.y, y0)),
+                     __fmaf_rn(q.w, y.z, __fmaf_rn(-q.x, y.y, z0)));
+}
+
 template <int P, int KIND, bool EXACT, bool REF, int NT, bool LARGE>
 __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B, double dt_d) {
     using FSmem = rbx::FSmem<NT>;
+    constexpr bool kWritten = !EXACT && !REF && !(LARGE && P == PREC_MIXED);  // the forms that round so
     constexpr int APT = 4;  // body atoms per thread in phase 1
     chain_release();
     const int tile = block_tile(S);
@@ -828,7 +840,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
                 const Q4<float> drf = rotation_increment<EXACT>(S, b, qBt(qh, ph + Ctau) * 0.5f, R, dt);
                 Q4<float> qd = qmul(qh - dqn, drb) * 0.5f + dqn * 2.5f + qmul(qh, drf);
                 qd = qd - qh * dot(qd, qh);
-                const V3<float> L = qBt(qh, ph) * 0.5f;
+                const V3<float> L = (kWritten ? body_momentum2(qh, ph) : qBt(qh, ph)) * 0.5f;
                 const float dkr = dot(qd, ph) / (6.0f * dt) - 0.5f * dot(L, mul(R.invI, L));
                 const V3<float> tb = rotate_to_body(qh, Ta);
                 const float u = dot(Fa, Fa) * invm + dot(tb, mul(R.invI, tb));
@@ -837,7 +849,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
         } else {
 #pragma unroll
             for (int c = 0; c < 3; c++) x[c] = ff_acc(x[c], fmaf(x[3 + c].hi, dt, x[3 + c].lo * dt));  // drift
-            const V3<float> L = qBt(qh, ph) * 0.5f;
+            const V3<float> L = (kWritten ? body_momentum2(qh, ph) : qBt(qh, ph)) * 0.5f;
             const Q4<float> dr = rotation_increment<EXACT>(S, b, L, R, dt);
             const Q4<float> dq = qmul(qh, dr), dp = qmul(ph, dr);
             x[6] = ff_acc(x[6], dq.w); x[7] = ff_acc(x[7], dq.x); x[8] = ff_acc(x[8], dq.y); x[9] = ff_acc(x[9], dq.z);
