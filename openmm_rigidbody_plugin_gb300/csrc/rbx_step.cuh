@@ -143,6 +143,20 @@ template <> struct PosIO<PREC_DOUBLE> {
 };
 
 
+// A body atom's velocity in the OpenMM layout of each precision. velm.w (1/m) is left untouched and not
+// read: x, y in one store, z in another.
+template <int P> __device__ __forceinline__ void store_velocity(const DevBuf& b, int loc, V3<double> v) {
+    if (P == PREC_SINGLE) {
+        float* to = (float*)b.velm + 4 * (size_t)loc;
+        *(float2*)to = make_float2((float)v.x, (float)v.y);
+        to[2] = (float)v.z;
+    } else {
+        double* to = (double*)b.velm + 4 * (size_t)loc;
+        *(double2*)to = make_double2(v.x, v.y);
+        to[2] = v.z;
+    }
+}
+
 // Failure detector: the new state of a body or free atom is checked for a non-finite value (NaN
 // or infinity; the check is one sum of already loaded values); a failing unit gets its flag byte
 // and the status counter one increment. Finite values never take the branch.
@@ -452,19 +466,14 @@ template <int NW> __device__ __forceinline__ int count_large(const unsigned* mas
 // Phase 3, part2: atom velocities v + omega_space x delta.
 template <int P, class A>
 __device__ __forceinline__ void atom_velocities(const DevSys& S, const DevBuf& B, const StepSmem<A>& sm, int a0, int nat) {
-    using V4 = typename Tr<P>::V4;
-    V4* vel = (V4*)B.velm;
     for (int a = threadIdx.x; a < nat; a += kThreads) {
         const int t = sm.sBody[a];
         const int loc = __ldg(S.atom_loc + a0 + a);
         V3<A> x = v3<A>(sm.sX[3 * a], sm.sX[3 * a + 1], sm.sX[3 * a + 2]);
         V3<A> w = v3<A>(sm.sW[3 * t], sm.sW[3 * t + 1], sm.sW[3 * t + 2]);
         V3<A> rel = cross(w, x);
-        V4 vm = vel[loc];
-        vm.x = sm.sRb[3 * t] + (double)rel.x;
-        vm.y = sm.sRb[3 * t + 1] + (double)rel.y;
-        vm.z = sm.sRb[3 * t + 2] + (double)rel.z;
-        vel[loc] = vm;
+        store_velocity<P>(B, loc, v3<double>(sm.sRb[3 * t] + (double)rel.x, sm.sRb[3 * t + 1] + (double)rel.y,
+                                             sm.sRb[3 * t + 2] + (double)rel.z));
     }
 }
 
@@ -677,8 +686,18 @@ __device__ __forceinline__ V3<float> body_momentum2(Q4<float> q, Q4<float> y) {
                      __fmaf_rn(q.w, y.z, __fmaf_rn(-q.x, y.y, z0)));
 }
 
+// State rows that a step of this kind leaves as they are: r and q in part2.
+template <int KIND> __device__ __forceinline__ constexpr bool kept_by(int c) {
+    return KIND == STEP_PART2 && (c < 3 || (c >= 6 && c < 10));
+}
+
+// Threads per SM: 768 at 80 registers; part2, which rotates nothing, 1024 at 64 (1e6 bodies and 1e5 free
+// atoms: 115 against 122 us a launch; 1280 at 48 registers is slower). With r and q neither stored nor
+// read whole, part2 moves 574 MB of DRAM traffic instead of 720: 130 -> 115 us, 74 % of measured HBM.
+template <int KIND, bool REF> constexpr int step_threads() { return KIND == STEP_PART2 && !REF ? 1024 : 768; }
+
 template <int P, int KIND, bool EXACT, bool REF, int NT, bool LARGE>
-__global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B, double dt_d) {
+__global__ void __launch_bounds__(NT, (step_threads<KIND, REF>() / NT)) step_kernel_f(DevSys S, DevBuf B, double dt_d) {
     using FSmem = rbx::FSmem<NT>;
     constexpr bool kWritten = !EXACT && !REF && !(LARGE && P == PREC_MIXED);  // the forms that round so
     constexpr int APT = 4;  // body atoms per thread in phase 1
@@ -773,9 +792,10 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
     // Phase 2: kicks, drift and rotation on the float-float state
     if (tid < nbt) {
         const int b = b0 + tid;
+        // (part2 moves neither r nor q: it reads their high words only and stores neither)
         ff x[14];
 #pragma unroll
-        for (int c = 0; c < 14; c++) x[c] = ff{ghi[b + c * nbp], glo[b + c * nbp]};
+        for (int c = 0; c < 14; c++) x[c] = ff{ghi[b + c * nbp], kept_by<KIND>(c) ? 0.0f : glo[b + c * nbp]};
         const float* bc = S.bconst;
         const float invm = __ldg(bc + b), invm_lo = __ldg(bc + b + 7 * nbp);
         Rotor R;
@@ -840,7 +860,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
                 const Q4<float> drf = rotation_increment<EXACT>(S, b, qBt(qh, ph + Ctau) * 0.5f, R, dt);
                 Q4<float> qd = qmul(qh - dqn, drb) * 0.5f + dqn * 2.5f + qmul(qh, drf);
                 qd = qd - qh * dot(qd, qh);
-                const V3<float> L = (kWritten ? body_momentum2(qh, ph) : qBt(qh, ph)) * 0.5f;
+                const V3<float> L = qBt(qh, ph) * 0.5f;
                 const float dkr = dot(qd, ph) / (6.0f * dt) - 0.5f * dot(L, mul(R.invI, L));
                 const V3<float> tb = rotate_to_body(qh, Ta);
                 const float u = dot(Fa, Fa) * invm + dot(tb, mul(R.invI, tb));
@@ -905,7 +925,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
         }
 #pragma unroll
         for (int c = 0; c < 14; c++) {
-            const bool normed = KIND != STEP_PART2 && (c < 3 || (c >= 6 && c < 10));
+            if (kept_by<KIND>(c)) continue;
+            const bool normed = c < 3 || (c >= 6 && c < 10);
             const ff y = normed ? x[c] : ff_norm(x[c]);
             ghi[b + c * nbp] = y.hi;
             glo[b + c * nbp] = y.lo;
@@ -922,15 +943,9 @@ __global__ void __launch_bounds__(NT, 768 / NT) step_kernel_f(DevSys S, DevBuf B
         const int k = a0 + a;
         const V3<float> x = v3<float>(__ldg(dg3 + k), __ldg(dg3 + k + S.nba_pad), __ldg(dg3 + k + 2 * S.nba_pad));
         if (KIND == STEP_PART2) {
-            using V4 = typename Tr<P>::V4;
             const V3<float> rel = cross(v3<float>(sW[3 * t], sW[3 * t + 1], sW[3 * t + 2]), mat_vec(sM + 9 * t, x));
             const double* v = (const double*)(sR + 6 * t);
-            V4* vel = (V4*)B.velm;
-            V4 vm = vel[loc];
-            vm.x = v[0] + (double)rel.x;
-            vm.y = v[1] + (double)rel.y;
-            vm.z = v[2] + (double)rel.z;
-            vel[loc] = vm;
+            store_velocity<P>(B, loc, v3<double>(v[0] + (double)rel.x, v[1] + (double)rel.y, v[2] + (double)rel.z));
         } else {
             const V3<float> delta = mat_vec(sM + 9 * t, x);
             const float* rf = sR + 6 * t;
