@@ -188,9 +188,9 @@ class BatchedSystems:
         _lib.check(self._lib.rbx_batch_set_graph_steps(self._h, int(k)))
 
     def autotune(self, dt=0.002, trial_steps=3, stream=None):
-        """Pick the step kernel's tile shape, the cell list-build kernel's block size and the steps per
-        captured graph by timing them on this batch; the state is restored exactly afterwards.
-        Returns the choice."""
+        """Pick the step kernel's tile shape and the steps per captured graph by timing them on this
+        batch; the state is restored exactly afterwards. Returns the choice ("cell_threads", once a
+        list-build block size, no longer changes the schedule)."""
         out = np.zeros(2, dtype=np.int32)
         _lib.check(self._lib.rbx_batch_autotune(self._h, _stream(stream), float(dt), int(trial_steps),
                                                 out.ctypes.data_as(ctypes.POINTER(ctypes.c_int))))

@@ -508,7 +508,7 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 //
 // Bound: instruction issue (62 % of the slots used), the L1 data pipe (53 to 67 %) and load latency, not
 // HBM (6 %). Measured per step of 256 boxes of 64 to 4096 bodies of the water/tetrahedron/ring mix
-// (1.07e6 atoms), list builds and integrator included: 0.75 ms, against 1.22 for one warp per rigid
+// (1.07e6 atoms), list builds and integrator included: 0.73 ms, against 1.22 for one warp per rigid
 // body with its atoms in shared memory, neighbours expanded atom by atom through a queue, and the
 // neighbours' records in list order. What made the difference: the unit's atoms in registers (no
 // shared-memory load per pair), one listed unit per lane instead of one atom (a third of the entry
