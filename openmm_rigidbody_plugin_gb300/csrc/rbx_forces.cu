@@ -502,9 +502,8 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 // Atoms sit at their images nearest their own unit's centroid, so the unit shift gives the minimum
 // image of every pair within the cutoff when cutoff + two radii < L/2; systems of smaller boxes
 // (FFSys::pair_image) take the minimum image per pair as well.
-// With at most kMaxTypes atom types each pair's (K q_i q_j, 12 C12, 6 C6) comes from a type-pair table, in
-// shared memory (kShared) or, of more than kSharedTypes types, through L1 (kGlobal: a solvent's few types
-// keep their entries there), else from the atoms' own parameters by Lorentz-Berthelot (kUntyped).
+// With at most kMaxTypes atom types (PT) each pair's (K q_i q_j, 12 C12, 6 C6) comes from a type-pair
+// table in shared memory, else from the atoms' own parameters by Lorentz-Berthelot.
 // The pair term is OpenMM's CutoffPeriodic form: reaction-field Coulomb and unshifted LJ.
 //
 // Bound: instruction issue (62 % of the slots used), the L1 data pipe (53 to 67 %) and load latency, not
@@ -520,7 +519,6 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 // branches (forces of 40 boxes with solutes 0.98 -> 0.80 ms). Not kept: 40 warps per SM at 48 registers
 // (19.2 ms); 24 at 80, with (20.5) or without (equal) the next atoms fetched before these are paired;
 // two atoms at a time in packed FP32 instructions (the FMA pipe takes as long; 5 % slower).
-constexpr int kUntyped = 0, kShared = 1, kGlobal = 2;  // PT
 constexpr int kFW = 4;    // warps (units) per block
 constexpr int kRing = 64;  // packed list entries per warp
 
@@ -565,19 +563,18 @@ template <int N> __device__ __forceinline__ int join_lanes(float (&v)[N], int la
 // NI atoms of the unit, the first NL with Lennard-Jones (the others Coulomb only: their pairs skip it,
 // and the unit's charge is applied once, to the sum). JS: atom records per place. RELAX: coincident
 // atoms have no direction and add nothing. PI: the minimum image per pair.
-template <int JS, int NI, int NL, bool ENERGY, int PT, bool RELAX, bool PI>
+template <int JS, int NI, int NL, bool ENERGY, bool PT, bool RELAX, bool PI>
 __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, const UnitTask& T, long long* __restrict__ force,
                                             int stride) {
     constexpr unsigned int kAll = 0xffffffffu;
-    extern __shared__ float4 stab[];
+    extern __shared__ float4 stab[];  // PT: the type-pair table
     const int lane = T.lane, nt = D.ntypes;
     const unsigned int* nb = D.nbr + (size_t)T.p * D.cap;
     const int u0 = S.u0;
     const float4 c = T.c;
     const float two_krf = 2.0f * S.krf, rc2 = S.rc2;
     float xi[NI][3], f[NI][3], qi[NI];
-    const float4* row[NI];  // the atom's row of the type-pair table (PT == kShared)
-    int at_row[NI];         // its first entry (PT == kGlobal)
+    const float4* row[NI];  // the atom's row of the type-pair table
     float4 pi[NI];
 #pragma unroll
     for (int a = 0; a < NI; a++) {
@@ -586,12 +583,9 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
         xi[a][1] = x.y;
         xi[a][2] = x.z;
         f[a][0] = f[a][1] = f[a][2] = 0.0f;
-        if (PT == kShared) {
+        if (PT) {
             row[a] = stab + __float_as_int(x.w) * nt;
             qi[a] = stab[__float_as_int(x.w)].w;
-        } else if (PT == kGlobal) {
-            at_row[a] = __float_as_int(x.w) * nt;
-            qi[a] = D.types[__float_as_int(x.w)].w;
         } else {
             pi[a] = D.spar[a][T.p];
         }
@@ -610,7 +604,7 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
             auto coefficients = [&](int a) {
                 float4 t;
                 if (PT) {
-                    t = PT == kShared ? row[a][tj] : __ldg(D.types + at_row[a] + tj);
+                    t = row[a][tj];
                     qj = t.w;
                 } else {
                     const float sig = pi[a].y + pj.y, sig2 = sig * sig, sig6 = sig2 * sig2 * sig2;
@@ -733,7 +727,7 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
 
 // The unit's exact size (the same choice for every lane): 3 atoms of which one has LJ is a 3-site
 // water; other units take the full term for every atom.
-template <int JS, bool ENERGY, int PT, bool RELAX, bool PI>
+template <int JS, bool ENERGY, bool PT, bool RELAX, bool PI>
 __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, const UnitTask& T, int ni, int nl,
                                               long long* force, int stride) {
     if (JS >= 4 && ni == 4) return unit_forces<JS, JS >= 4 ? 4 : 1, JS >= 4 ? 4 : 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
@@ -745,25 +739,24 @@ __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, co
     unit_forces<JS, 1, 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
 }
 
-// Blocks per SM: 64 registers a thread (32 warps per SM); 80 for units of four atoms and without the table
-// in shared memory. The larger variants then spill a little and still gain: forces of 40 boxes with 64-type
-// solutes without a table take 1.09 ms at 128 registers, 0.98 at 80 and 0.97 at 64 (later, with the list
-// build's code, 0.75 at 80 and 0.77 at 64). With the table through L1 they take 0.71 at 80 and 0.725 at 64,
-// and 20 steps of these boxes 5.95 ms without it, 5.26 at 80 and 5.49 at 64.
+// Blocks per SM: 64 registers a thread (32 warps per SM); 80 for units of four atoms. The larger variants
+// then spill a little and still gain: forces of 40 boxes with 64-type solutes take 1.09 ms at 128
+// registers, 0.98 at 80 and 0.97 at 64 (later, with the list build's code, 0.75 at 80 and 0.77 at 64: the
+// form without the type-pair table takes 80).
 constexpr int force_blocks(int records) { return records <= 3 ? 8 : 6; }
-constexpr int kUntypedBlocks = 6, kGlobalBlocks = 6;
+constexpr int kUntypedBlocks = 6;
 // Batches of at most kFewUnits units (two warps per scheduler) leave the SMs nearly empty: a warp's own
 // chain of instructions is then the time, and 128 registers let more of it overlap (512 waters, 20 steps
 // with energies and a frame: 475 against 537 us; at 2600 units, 683 against 662).
 constexpr int kFewUnits = 8 * kSMs, kFewBlocks = 4;
 
-template <int JS, bool ENERGY, int PT, bool RELAX, int BLOCKS>
+template <int JS, bool ENERGY, bool PT, bool RELAX, int BLOCKS>
 __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long* __restrict__ force, int stride) {
-    extern __shared__ float4 stab[];  // PT == kShared: the type-pair table
+    extern __shared__ float4 stab[];  // PT: the type-pair table
     __shared__ float4 ring[kFW][kRing];
     chain_release();
     const int nt = D.ntypes;
-    if (PT == kShared) {
+    if (PT) {
         for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) stab[t] = D.types[t];
         __syncthreads();
     }
@@ -804,15 +797,14 @@ __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long*
 template <int JS, bool ENERGY, bool RELAX>
 cudaError_t launch_force_kernel(const FFDev& D, long long* f, int stride, cudaStream_t st) {
     const int grid = (D.n_units + kFW - 1) / kFW;
-    const size_t table = D.ntypes <= kSharedTypes ? sizeof(float4) * D.ntypes * D.ntypes : 0;
+    const size_t table = sizeof(float4) * D.ntypes * D.ntypes;
     auto launch = [&](int blocks, void (*kernel)(FFDev, long long*, int)) {
         const size_t block_shared = sizeof(float4) * kFW * kRing + table + 1024;
         return launch_chained_l1<FFDev, long long*, int>(blocks * block_shared, kernel, grid, 32 * kFW, table, st, D, f, stride);
     };
-    if (!D.ntypes) return launch(kUntypedBlocks, ff_force<JS, ENERGY, kUntyped, RELAX, kUntypedBlocks>);
-    if (D.ntypes > kSharedTypes) return launch(kGlobalBlocks, ff_force<JS, ENERGY, kGlobal, RELAX, kGlobalBlocks>);
-    if (!RELAX && D.n_units <= kFewUnits) return launch(kFewBlocks, ff_force<JS, ENERGY, kShared, RELAX, kFewBlocks>);
-    return launch(force_blocks(JS), ff_force<JS, ENERGY, kShared, RELAX, force_blocks(JS)>);
+    if (!D.ntypes) return launch(kUntypedBlocks, ff_force<JS, ENERGY, false, RELAX, kUntypedBlocks>);
+    if (!RELAX && D.n_units <= kFewUnits) return launch(kFewBlocks, ff_force<JS, ENERGY, true, RELAX, kFewBlocks>);
+    return launch(force_blocks(JS), ff_force<JS, ENERGY, true, RELAX, force_blocks(JS)>);
 }
 
 // A capped relaxation forms no energies.

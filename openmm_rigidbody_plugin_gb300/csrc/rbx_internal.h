@@ -179,11 +179,7 @@ struct FFDev {
     // (prep_limit); prep_units = 0 otherwise
     int prep_units, prep_cells;
 };
-// Most atom types whose pair table (FFDev::types) the force pass copies to shared memory (16 KB), and most
-// of a table at all: larger ones are read through L1. 20 steps of 40 boxes of 700 to 3100 waters of T
-// charges each, without a table, with one: T = 64 4.54, 3.96 ms; 128 4.54, 4.05; 256 4.54, 4.11; 512 4.54,
-// 4.19; 1024 4.54, 4.35, where the table (16 MB, formed on the host) no longer pays for its set-up.
-constexpr int kSharedTypes = 32, kMaxTypes = 256;
+constexpr int kMaxTypes = 32;  // atom types of the type-pair table (FFDev::types)
 // Interacting atoms of one system (a limit of this interface: list entries are 32-bit words).
 constexpr int kMaxSystemAtoms = 1 << 26;
 // Whether the set-up of a system of this many units and list cells is left to one block (ff_prep): a
