@@ -35,6 +35,7 @@
 
 #include <cstdint>
 
+#include "rbx_cells.h"
 #include "rbx_internal.h"
 #include "rbx_launch.cuh"
 
@@ -55,20 +56,7 @@ __device__ __forceinline__ float3 atom_position(const DevBuf& B, int prec, int s
     return make_float3(p.x, p.y, p.z);
 }
 
-__device__ __forceinline__ int wrap_cell(float x, float invL, int nc) {
-    float f = x * invL;
-    f -= floorf(f);
-    int c = (int)(f * (float)nc);
-    return c < 0 ? 0 : (c >= nc ? nc - 1 : c);
-}
-
-// Position of an interacting atom wrapped into [0, L) and its minimum-image displacement.
-__device__ __forceinline__ float3 wrap_box(float3 x, const FFSys& S) {
-    x.x -= S.L * floorf(x.x * S.invL);
-    x.y -= S.L * floorf(x.y * S.invL);
-    x.z -= S.L * floorf(x.z * S.invL);
-    return x;
-}
+// Minimum-image displacement.
 __device__ __forceinline__ float3 min_image(float dx, float dy, float dz, const FFSys& S) {
     return make_float3(dx - S.L * rintf(dx * S.invL), dy - S.L * rintf(dy * S.invL), dz - S.L * rintf(dz * S.invL));
 }
@@ -76,13 +64,32 @@ __device__ __forceinline__ float3 min_image(float dx, float dy, float dz, const 
 // Coordinate of the unused atom records of a place: outside every cutoff, its square finite.
 constexpr float kFar = 1e10f;
 
-// Centroid of a unit (the mean of its atoms' minimum-image displacements from the first, wrapped
-// into the box) and its radius.
-__device__ __forceinline__ float4 unit_centroid(const FFDev& D, const DevBuf& B, int prec, const FFSys& S, int k0, int n,
-                                                float3 (&x)[kMaxUnit]) {
+// The unit's atoms at their images nearest its centroid c; returns the largest squared distance from it.
+__device__ __forceinline__ float atoms_about(const FFSys& S, int n, float4 c, float3 (&x)[kMaxUnit]) {
+    float rho2 = 0.f;
+#pragma unroll
+    for (int a = 0; a < kMaxUnit; a++) {
+        if (a >= n) break;
+        const float3 d = min_image(x[a].x - c.x, x[a].y - c.y, x[a].z - c.z, S);
+        rho2 = fmaxf(rho2, fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)));
+        x[a] = make_float3(c.x + d.x, c.y + d.y, c.z + d.z);
+    }
+    return rho2;
+}
+
+// Positions of a unit's atoms.
+__device__ __forceinline__ void unit_positions(const FFDev& D, const DevBuf& B, int prec, int k0, int n,
+                                               float3 (&x)[kMaxUnit]) {
 #pragma unroll
     for (int a = 0; a < kMaxUnit; a++)
         if (a < n) x[a] = atom_position(B, prec, D.iatom[k0 + a]);
+}
+
+// Centroid of a unit (the mean of its atoms' minimum-image displacements from the first, wrapped
+// into the box) and its radius; x: its atoms about it.
+__device__ __forceinline__ float4 unit_centroid(const FFDev& D, const DevBuf& B, int prec, const FFSys& S, int k0, int n,
+                                                float3 (&x)[kMaxUnit]) {
+    unit_positions(D, B, prec, k0, n, x);
     float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
     for (int a = 1; a < kMaxUnit; a++) {
@@ -93,16 +100,11 @@ __device__ __forceinline__ float4 unit_centroid(const FFDev& D, const DevBuf& B,
         sz += d.z;
     }
     const float inv = 1.0f / (float)n;
-    const float3 c = wrap_box(make_float3(x[0].x + sx * inv, x[0].y + sy * inv, x[0].z + sz * inv), S);
-    float rho2 = 0.f;
-#pragma unroll
-    for (int a = 0; a < kMaxUnit; a++) {
-        if (a >= n) break;
-        const float3 d = min_image(x[a].x - c.x, x[a].y - c.y, x[a].z - c.z, S);
-        rho2 = fmaxf(rho2, fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)));
-        x[a] = make_float3(c.x + d.x, c.y + d.y, c.z + d.z);  // at the image nearest the centroid
-    }
-    return make_float4(c.x, c.y, c.z, sqrtf(rho2));
+    float4 c = make_float4(wrap_coordinate(fmaf(sx, inv, x[0].x), S.L, S.invL),
+                           wrap_coordinate(fmaf(sy, inv, x[0].y), S.L, S.invL),
+                           wrap_coordinate(fmaf(sz, inv, x[0].z), S.L, S.invL), 0.0f);
+    c.w = sqrtf(atoms_about(S, n, c, x));
+    return c;
 }
 
 // A unit's records at place p: centroid, and its atoms (at their images nearest the centroid, so that
@@ -119,7 +121,7 @@ __device__ __forceinline__ void write_place(const FFDev& D, int p, int k0, int n
 
 // Cell of a centroid in its system.
 __device__ __forceinline__ int cell_index(const FFSys& S, float4 c) {
-    return (wrap_cell(c.z, S.invL, S.nc) * S.nc + wrap_cell(c.y, S.invL, S.nc)) * S.nc + wrap_cell(c.x, S.invL, S.nc);
+    return (cell_of(c.z, S.invL, S.nc) * S.nc + cell_of(c.y, S.invL, S.nc)) * S.nc + cell_of(c.x, S.invL, S.nc);
 }
 
 // Key of a unit in the order within its cell: its place on a 4 x 4 x 4 grid of the cell in Z-order,
@@ -143,12 +145,14 @@ __device__ __forceinline__ bool moved_too_far(const FFDev& D, const FFSys& S, in
     return fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) > S.half_skin2;
 }
 
-// Unit u at its new place p: records, group, build centroid.
+// Unit u at its new place p: records, group, build centroid (the one that its cell was taken from).
 __device__ __forceinline__ void settle(const FFDev& D, const DevBuf& B, int prec, const FFSys& S, int u, int p) {
     const int2 kn = D.unit[u];
     const int k0 = kn.x, n = kn.y & 0xff;
     float3 x[kMaxUnit];
-    const float4 c = unit_centroid(D, B, prec, S, k0, n, x);
+    const float4 c = D.ucen[u];
+    unit_positions(D, B, prec, k0, n, x);
+    atoms_about(S, n, c, x);
     write_place(D, p, k0, n, c, x);
     if (!D.ntypes)
         for (int a = 0; a < D.slots; a++) D.spar[a][p] = a < n ? D.param[k0 + a] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -357,7 +361,7 @@ __device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p,
     unsigned int* list = D.nbr + (size_t)p * D.cap;
     const bool image = S.nc == 1;  // one run, the whole box: minimum image per pair
     const int nc = S.nc, w = S.win, side = 2 * w + 1;
-    const int cx = wrap_cell(c.x, S.invL, nc), cy = wrap_cell(c.y, S.invL, nc), cz = wrap_cell(c.z, S.invL, nc);
+    const int cx = cell_of(c.x, S.invL, nc), cy = cell_of(c.y, S.invL, nc), cz = cell_of(c.z, S.invL, nc);
     // the lane's row of cells: the cells xa to xb of it are within reach, in an unwrapped count
     int xa = 0, xb = -1;
     const int* row = nullptr;
