@@ -21,10 +21,41 @@ RBX_HD inline float wrap_coordinate(float x, float L, float invL) {
     return x >= L ? x - L : x;
 }
 
-// Cell, of nc per edge, of a wrapped coordinate.
+// Cell, of nc per edge, of a wrapped coordinate (of any other the nearest one, of a NaN the first).
 RBX_HD inline int cell_of(float x, float invL, int nc) {
-    const int c = (int)(x * invL * (float)nc);
-    return c < 0 ? 0 : (c >= nc ? nc - 1 : c);
+    return (int)fminf(fmaxf(x * invL * (float)nc, 0.0f), (float)(nc - 1));
+}
+
+// Cells a to b (none when a > b).
+struct CellRange {
+    int a, b;
+};
+
+// The cells that [x - h, x + h] meets along one edge, `per_length` cells per unit of length, among the w
+// cells on either side of cell c, in an unwrapped count (from -w to nc - 1 + w). Any x and h, not finite ones
+// too, stay inside that window: the limits are applied before the conversion to whole numbers.
+RBX_HD inline CellRange cells_within(float x, float h, float per_length, int c, int w) {
+    const float lo = (float)(c - w), hi = (float)(c + w);
+    CellRange r;
+    r.a = (int)fminf(fmaxf(floorf((x - h) * per_length), lo), hi + 1.0f);
+    r.b = (int)fmaxf(fminf(floorf((x + h) * per_length), hi), lo - 1.0f);
+    return r;
+}
+
+// The part of such a range inside the box (part 0), or across the edge that cell c is near (part 1), as cells
+// from 0 to nc - 1. At least 2 w + 1 cells per edge: a range crosses one edge at most.
+RBX_HD inline CellRange range_part(CellRange r, int part, int c, int w, int nc) {
+    if (part == 0) {
+        r.a = r.a > 0 ? r.a : 0;
+        r.b = r.b < nc - 1 ? r.b : nc - 1;
+    } else if (c < w) {
+        r.a += nc;
+        r.b = (r.b < -1 ? r.b : -1) + nc;
+    } else {
+        r.a = (r.a > nc ? r.a : nc) - nc;
+        r.b -= nc;
+    }
+    return r;
 }
 
 }  // namespace rbx

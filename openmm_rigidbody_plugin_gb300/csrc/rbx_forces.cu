@@ -362,8 +362,8 @@ __device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p,
     const bool image = S.nc == 1;  // one run, the whole box: minimum image per pair
     const int nc = S.nc, w = S.win, side = 2 * w + 1;
     const int cx = cell_of(c.x, S.invL, nc), cy = cell_of(c.y, S.invL, nc), cz = cell_of(c.z, S.invL, nc);
-    // the lane's row of cells: the cells xa to xb of it are within reach, in an unwrapped count
-    int xa = 0, xb = -1;
+    // the lane's row of cells and those of it within reach, in an unwrapped count
+    CellRange within = {0, -1};
     const int* row = nullptr;
     float sy = 0.f, sz = 0.f;
     if (!image && lane < side * side) {
@@ -372,11 +372,7 @@ __device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p,
         const float tz = fmaxf(fmaxf((float)z * e - c.z, c.z - (float)(z + 1) * e), 0.0f);
         const float ty = fmaxf(fmaxf((float)y * e - c.y, c.y - (float)(y + 1) * e), 0.0f);
         const float h2 = reach * reach - fmaf(ty, ty, tz * tz);
-        if (h2 > 0.0f) {
-            const float h = sqrtf(h2);
-            xa = max((int)floorf((c.x - h) * ie), cx - w);
-            xb = min((int)floorf((c.x + h) * ie), cx + w);
-        }
+        if (h2 > 0.0f) within = cells_within(c.x, sqrtf(h2), ie, cx, w);
         sz = z < 0 ? -S.L : (z >= nc ? S.L : 0.f);
         z = z < 0 ? z + nc : (z >= nc ? z - nc : z);
         sy = y < 0 ? -S.L : (y >= nc ? S.L : 0.f);
@@ -396,22 +392,11 @@ __device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p,
                 r1 = S.u1;
             }
         } else {
-            int a = xa, b = xb;
-            if (part == 0) {
-                a = max(a, 0);
-                b = min(b, nc - 1);
-            } else if (cx < w) {
-                sx = -S.L;
-                a += nc;
-                b = min(b, -1) + nc;
-            } else {
-                sx = S.L;
-                a = max(a, nc) - nc;
-                b -= nc;
-            }
-            if (a <= b) {
-                r0 = row[a];
-                r1 = row[b + 1];
+            const CellRange in = range_part(within, part, cx, w, nc);
+            if (part == 1) sx = cx < w ? -S.L : S.L;
+            if (in.a <= in.b) {
+                r0 = row[in.a];
+                r1 = row[in.b + 1];
             }
         }
         // the runs that hold anything, packed: run k covers the sequence from first[k] on

@@ -44,6 +44,75 @@ def wrap(tmp_path_factory):
     return call
 
 
+RANGES = r"""
+#include <cstdio>
+#include "rbx_cells.h"
+int main() {  // lines of: x h L nc w -> the ranges of the parts that the search takes
+    float x, h, L;
+    int nc, w;
+    while (scanf("%f %f %f %d %d", &x, &h, &L, &nc, &w) == 5) {
+        const float invL = 1.0f / L;
+        const int c = rbx::cell_of(x, invL, nc);
+        const rbx::CellRange r = rbx::cells_within(x, h, invL * (float)nc, c, w);
+        const int parts = c < w || c >= nc - w ? 2 : 1;
+        printf("%d %d", c, parts);
+        for (int p = 0; p < 2; p++) {
+            const rbx::CellRange in = p < parts ? rbx::range_part(r, p, c, w, nc) : rbx::CellRange{0, -1};
+            printf(" %d %d", in.a, in.b);
+        }
+        printf("\n");
+    }
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def ranges(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not found")
+    d = tmp_path_factory.mktemp("ranges")
+    src, exe = d / "ranges.cpp", d / "ranges"
+    src.write_text(RANGES)
+    csrc = os.path.join(ROOT, "openmm_rigidbody_plugin_gb300", "csrc")
+    # signed overflow and conversions out of range end the program
+    subprocess.run([gxx, "-std=c++17", "-O1", "-Wall", "-Werror", "-fsanitize=undefined,float-cast-overflow",
+                    "-fno-sanitize-recover=all", "-I", csrc, str(src), "-o", str(exe)], check=True)
+
+    def call(cases):
+        lines = "".join(" ".join(str(v) for v in c) + "\n" for c in cases)
+        out = subprocess.run([str(exe)], input=lines, check=True, capture_output=True, text=True).stdout
+        return np.array([[int(v) for v in line.split()] for line in out.splitlines()])
+    return call
+
+
+def test_cells_in_reach_are_taken_once_each(ranges):
+    rng = np.random.default_rng(3)
+    cases = []
+    for _ in range(3000):
+        w = int(rng.integers(1, 3))
+        nc = int(rng.integers(2 * w + 1, 14))
+        edge = float(rng.uniform(0.3, 2.0))
+        cases.append((float(np.float32(rng.uniform(0, nc * edge * (1 - 1e-6)))), rng.uniform(0.0, w * edge), nc * edge, nc, w))
+    out = ranges(cases)
+    for (x, h, L, nc, w), (c, _, a0, b0, a1, b1) in zip(cases, out):
+        taken = list(range(a0, b0 + 1)) + list(range(a1, b1 + 1))
+        assert len(taken) == len(set(taken)) and all(0 <= k < nc for k in taken)
+        edge, slack = L / nc, 1e-4
+        met = {int(np.floor(t / edge)) % nc for t in np.arange(x - h + slack, x + h - slack, 0.01 * edge)}
+        assert met <= set(taken), (x, h, L, nc, w, taken, met)
+
+
+def test_coordinates_without_a_place_in_the_box_stay_in_the_cell_table(ranges):
+    values = [s * v for s in (-1, 1) for v in (1e5, 1e8, 1.5e9, 2.2e9, 3e12, 1e30, 3e38, float("inf"))]
+    reaches = [0.5, 1e6, 1e20, float("inf")]
+    cases = [(x, h, L, nc, w) for x in values for h in reaches for L, nc, w in ((4.4, 7, 2), (3.0, 3, 1), (5.0, 5, 2))]
+    for case, (c, _, a0, b0, a1, b1) in zip(cases, ranges(cases)):
+        for a, b in ((a0, b0), (a1, b1)):
+            assert a > b or (0 <= a and b < case[3]), (case, a, b)
+
+
 def test_wrapped_coordinates_lie_in_their_cells(wrap):
     rng = np.random.default_rng(2)
     x, L, nc = [], [], []
