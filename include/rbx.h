@@ -351,11 +351,15 @@ int rbx_last_launch_count(const rbx_integrator* h);
  * freedom.
  * Forces come from neighbour lists of units of at most four atoms (a rigid body is cut into units;
  * a free atom is one): two units of different bodies are listed together when their centroids lie
- * within cutoff + a skin of 0.12 nm + both units' radii. Each system rebuilds its lists when one of its centroids has
- * moved half the skin, and every list is rebuilt for the state a step call ends in (and for the
+ * within cutoff + a skin of 0.12 nm + both units' radii. rbx_batch_set_state gives every system room for
+ * its longest list in that state and a fifth more (never less than its mean density asks for); a
+ * unit with more neighbours than that, in a system that has become far denser since, is paired with
+ * all units of its system instead: the same forces, more slowly. Each system rebuilds its lists when one of
+ * its centroids has moved half the skin, and every list is rebuilt for the state a step call ends in (and for the
  * first evaluation after rbx_batch_set_state or rbx_batch_restore), so the forces and energy at a
  * call's start and end depend on the positions alone: a system's results are a function of its own
- * state and of the lengths of the calls that step it.
+ * state, of the positions last given to rbx_batch_set_state and of the lengths of the calls that step
+ * it.
  */
 typedef struct rbx_batch rbx_batch;
 /* rbx_batch_set_state builds every body from the given positions and velocities (as

@@ -9,11 +9,13 @@
 
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <map>
 #include <new>
+#include <numeric>
 #include <thread>
 #include <vector>
 
@@ -113,11 +115,12 @@ struct rbx_batch {
     DevArray<unsigned int> d_skey;      // FFDev::skey
     DevArray<unsigned int> d_nbr;       // neighbour lists of units (FFDev::nbr)
     DevArray<unsigned int> d_rebuilds;  // list builds per system (FFDev::rebuilds)
+    DevArray<int> d_most;               // longest list per system, and builds that are not the user's
     // host copies for the set-up with a state: systems, cells allocated per system, unit layout
     std::vector<FFSys> sys_h;
     std::vector<int> cells_alloc, iatom_h;
     std::vector<int2> unit_h;
-    std::vector<double> box_h;
+    std::vector<double> box_h, list_expect;  // list_expect: list lengths at the mean density
     DevArray<double> d_e_unit, d_energy;
     FFDev ff{};
     // per-system reductions
@@ -181,7 +184,8 @@ int cells_per_edge(double L, double edge, int most) {
 
 // Neighbour-list geometry for a state (host positions, user order): each unit's radius about its
 // centroid (constant for a rigid body), and from the largest radius of each system its list cells
-// (at least cutoff + skin + two radii per edge), the cell work list and the list capacity.
+// (at least cutoff + skin + two radii per edge, or half of that). The lists themselves are sized by
+// size_lists, once the state is on the device.
 int setup_lists(rbx_batch* b, const double* x) {
     const int S = b->S;
     std::vector<FFSys> sys = b->sys_h;
@@ -209,7 +213,7 @@ int setup_lists(rbx_batch* b, const double* x) {
         }
         rho[s] = std::sqrt(rho_max);
     });
-    double cap_need = 1.0;
+    b->list_expect.assign(S, 0.0);
     long long most_units = 0, most_cells = 0;
     for (int s = 0; s < S; s++) {
         FFSys& f = sys[s];
@@ -229,20 +233,14 @@ int setup_lists(rbx_batch* b, const double* x) {
         most_units = std::max<long long>(most_units, U);
         most_cells = std::max<long long>(most_cells, (long long)nc * nc * nc);
         const double reach = (double)f.rl + 2.0 * rho_max;
-        const double expect = 4.18879 * reach * reach * reach * (double)U / (L * L * L);
-        cap_need = std::max(cap_need, std::min((double)std::max(U - 1, 1), 1.35 * expect + 32.0));
+        b->list_expect[s] = 4.18879 * reach * reach * reach * (double)U / (L * L * L);
     }
-    const int cap = std::max(32, ((int)std::ceil(cap_need) + 31) / 32 * 32);
-    const size_t entries = (size_t)std::max(b->ff.n_units, 1) * (size_t)cap;
-    if (b->d_nbr.n < entries && b->d_nbr.alloc(entries) != cudaSuccess)
-        return set_error(RBX_ERR_CUDA, "cudaMalloc of the neighbour lists failed (%d entries per unit)", cap);
     BATCH_TRY(cudaMemcpy(b->d_sys.p, sys.data(), sizeof(FFSys) * (size_t)S, cudaMemcpyHostToDevice));
+    b->sys_h = sys;
     FFDev& D = b->ff;
     const bool small = prep_limit(most_units, most_cells);
     D.prep_units = small ? (int)most_units : 0;
     D.prep_cells = small ? (int)most_cells : 0;
-    D.cap = cap;
-    D.nbr = b->d_nbr.p;
     return RBX_OK;
 }
 
@@ -278,6 +276,45 @@ DevBuf buffers(rbx_batch* b) {
     d.force = rb.force;
     d.stride = rb.stride;
     return d;
+}
+
+// List memory for the state on the device. The longest list of each system is counted there, not estimated
+// from the mean density: bodies cut into units, clusters and droplets make lists many times longer than that.
+// A fifth and 32 entries are left for what the motion adds, and no system gets less than its mean density
+// asks for. A list that outgrows its room all the same costs time, not pairs (FFDev::ncnt).
+// Every system has a capacity of its own, so that its results do not depend on the others.
+int size_lists(rbx_batch* b, void* stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    const int S = b->S;
+    std::vector<int> most(S, 0);
+    FFDev D = b->ff;
+    D.rebuilds = (unsigned int*)(b->d_most.p + S);  // these are no builds of the user's steps
+    if (launch_list_lengths(D, b->prec, buffers(b), b->d_most.p, stream) < 0)
+        return set_error(RBX_ERR_CUDA, "list length kernels failed: %s", cudaGetErrorString(cudaGetLastError()));
+    BATCH_TRY(cudaMemcpyAsync(most.data(), b->d_most.p, sizeof(int) * (size_t)S, cudaMemcpyDeviceToHost, st));
+    BATCH_TRY(cudaStreamSynchronize(st));
+    int most_units = 1;
+    for (const FFSys& f : b->sys_h) most_units = std::max(most_units, f.u1 - f.u0);
+    std::vector<unsigned int> every((most_units + 31) / 32 * 32);
+    std::iota(every.begin(), every.end(), 0u);
+    long long rows = (long long)every.size() / 32;  // of 32 entries
+    for (int s = 0; s < S; s++) {
+        FFSys& f = b->sys_h[s];
+        const int U = f.u1 - f.u0;
+        const double need = std::max(1.35 * b->list_expect[s], 1.2 * most[s]) + 32.0;
+        f.cap = ((int)std::ceil(std::min((double)std::max(U - 1, 1), need)) + 31) / 32 * 32;
+        f.list0 = (int)rows;
+        rows += (long long)U * (f.cap / 32);
+        if (rows > INT_MAX) return set_error(RBX_ERR_CUDA, "neighbour lists of more than 2^36 entries");
+    }
+    const size_t entries = 32 * (size_t)rows;
+    if (b->d_nbr.n < entries && b->d_nbr.alloc(entries) != cudaSuccess)
+        return set_error(RBX_ERR_CUDA, "cudaMalloc of the neighbour lists failed (%zu entries)", entries);
+    b->ff.nbr = b->d_nbr.p;
+    BATCH_TRY(cudaMemcpyAsync(b->d_nbr.p, every.data(), sizeof(unsigned int) * every.size(), cudaMemcpyHostToDevice, st));
+    BATCH_TRY(cudaMemcpyAsync(b->d_sys.p, b->sys_h.data(), sizeof(FFSys) * (size_t)S, cudaMemcpyHostToDevice, st));
+    BATCH_TRY(cudaStreamSynchronize(st));
+    return RBX_OK;
 }
 
 // Event pair around one launch group when timing is on (never inside a stream capture).
@@ -468,7 +505,8 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
         // the box: an image within the cutoff (below half the box) is always the minimum image, and
         // its unit pair is always listed.
         f.rl = (float)(rc_s + kSkin);
-        f.half_skin2 = (float)(0.25 * kSkin * kSkin);
+        f.cap = 32;  // until the lists are sized (rbx_batch_set_state)
+        f.list0 = 0;
         f.pair_image = 1;  // until the radii are known (rbx_batch_set_state)
         // cells for the largest grid any set of radii allows (the radii, known with the positions,
         // can only make the cells larger and fewer): of the whole reach, or of half of it while there
@@ -550,13 +588,14 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
                 b->d_energy.alloc(num_systems) != cudaSuccess || b->d_ke.alloc(2 * (size_t)num_systems) != cudaSuccess ||
                 b->d_user.alloc(3 * (size_t)N) != cudaSuccess || b->d_sys_status.alloc(num_systems) != cudaSuccess ||
                 b->d_moved.alloc(num_systems) != cudaSuccess || b->d_build.alloc(num_systems) != cudaSuccess ||
-                b->d_rebuilds.alloc(num_systems) != cudaSuccess))
+                b->d_rebuilds.alloc(num_systems) != cudaSuccess || b->d_most.alloc(2 * (size_t)num_systems) != cudaSuccess))
         rc = set_error(RBX_ERR_CUDA, "cudaMalloc of force-field arrays failed");
     if (!rc && (cudaMemset(b->d_sys_status.p, 0, sizeof(unsigned int) * (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_cell_count.p, 0, sizeof(int) * (size_t)cells) != cudaSuccess ||
                 cudaMemset(b->d_moved.p, 0, (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_build.p, 0, (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_rebuilds.p, 0, sizeof(unsigned int) * (size_t)num_systems) != cudaSuccess ||
+                cudaMemset(b->d_most.p, 0, sizeof(int) * 2 * (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_ncnt.p, 0, sizeof(int) * u1) != cudaSuccess ||
                 cudaMemset(b->d_place.p, 0, sizeof(int) * u1) != cudaSuccess ||
                 cudaMemset(b->d_unit_at.p, 0, sizeof(int) * u1) != cudaSuccess))
@@ -599,9 +638,9 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.moved = b->d_moved.p;
     D.build = b->d_build.p;
     D.rebuilds = b->d_rebuilds.p;
-    D.nbr = nullptr;  // allocated with the state (its capacity follows the units' radii)
+    D.nbr = nullptr;  // allocated with the state (size_lists)
     D.ncnt = b->d_ncnt.p;
-    D.cap = 0;
+    D.half_skin2 = (float)(0.25 * kSkin * kSkin);
     D.types = b->d_types.p;
     D.atype = b->d_atype.p;
     D.ntypes = (int)types.size();
@@ -628,6 +667,7 @@ int rbx_batch_set_state(rbx_batch* b, void* stream, const double* positions, con
     if (!positions || !velocities) return set_error(RBX_ERR_INVALID_ARGUMENT, "null positions or velocities");
     BATCH_TRY(cudaSetDevice(b->device));
     BATCH_TRY(cudaStreamSynchronize((cudaStream_t)stream));  // no force pass in flight on the old lists
+    b->d_body0.release();  // no state, until all of the new one is in place
     if ((rc = setup_lists(b, positions))) return rc;
     // positions and velocities into the device buffers, bodies built there (no host round trip)
     if ((rc = rbx_context_load(b->integ, stream, positions, velocities))) return rc;
@@ -637,6 +677,7 @@ int rbx_batch_set_state(rbx_batch* b, void* stream, const double* positions, con
     // body atoms start where the body state puts them (the step kernels' arithmetic), so that a
     // system's trajectory is a function of its body state alone, in or out of a batch
     if ((rc = rbx_context_sync_bodies(b->integ, stream))) return rc;
+    if ((rc = size_lists(b, stream))) return rc;
     if ((rc = sync_host_dof(b->integ))) return rc;
     std::vector<int> body0, free0;
     if ((rc = system_ranges(b->integ, b->offsets, body0, free0, b->dof))) return rc;
@@ -830,7 +871,7 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
                b->d_unit_at.bytes() + b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
                b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_sunit.bytes() + b->d_spos.bytes() + b->d_spar.bytes() +
                b->d_skey.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() +
-               b->d_build.bytes() + b->d_nbr.bytes() + b->d_ncnt.bytes() + b->d_rebuilds.bytes() +
+               b->d_build.bytes() + b->d_nbr.bytes() + b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_most.bytes() +
                b->d_e_unit.bytes() + b->d_energy.bytes() + b->d_body0.bytes() + b->d_free0.bytes() +
                b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() + b->ke_chunks.bytes() +
                b->e_chunks.bytes();

@@ -142,7 +142,7 @@ __device__ __forceinline__ unsigned int cell_key(const FFSys& S, float4 c, int u
 __device__ __forceinline__ bool moved_too_far(const FFDev& D, const FFSys& S, int u, float4 c) {
     const float4 r = D.uref[u];
     const float3 d = min_image(c.x - r.x, c.y - r.y, c.z - r.z, S);
-    return fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) > S.half_skin2;
+    return fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) > D.half_skin2;
 }
 
 // Unit u at its new place p: records, group, build centroid (the one that its cell was taken from).
@@ -341,24 +341,29 @@ __global__ void ff_place(FFDev D, DevBuf B, int prec) {
     settle(D, B, prec, S, u, b + rank);
 }
 
+// The list of the unit at place p starts at entry 32 list_row.
+__device__ __forceinline__ int list_row(const FFSys& S, int p) { return S.list0 + (p - S.u0) * (S.cap >> 5); }
+
 // Lists, a warp per unit: the lanes test 32 candidates at a time and append the ones in range in order,
 // a ballot giving each its slot (coalesced). The candidates are the units of the cells within reach,
 // row of cells by row: in place order a row is one contiguous run (two where it crosses the box's
 // edge), trimmed to the chord of the reach through the row, and the runs are taken as one sequence, so
-// that the lanes stay full however short they are. A full list marks the system as failed (the capacity
-// is sized from the densest system with a wide margin, so this does not happen in a liquid).
+// that the lanes stay full however short they are. Entries past the list's capacity are counted, not stored
+// (the force pass then takes every unit of the system instead of the list).
 // Bound: load latency and issue. Cells of half the reach, trimmed, leave about 650 candidates of a
 // water's 214 entries; cells of the whole reach (27 of them, untrimmed) had 1600. 20 steps with energies
 // and a frame: 66,666 waters 5.0 -> 4.4 ms, 256 boxes of the mix 16.3 -> 14.7; forces of 15,001 bodies
 // 0.32 -> 0.26. kAhead chunks of
 // candidates are in flight. Built by the force pass itself: a kernel of its own, which has nothing to do
 // in most steps, cost 588 against 531 us per 20 steps of 512 waters.
-// Returns the length of the list of the unit at place p with centroid c; runs: scratch of 32 records.
-__device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p, int s, float4 c, int lane, float4* runs) {
+// Returns the length of the list of the unit at place p with centroid c; runs: scratch of 32 records. STORE:
+// the list and its length are stored.
+template <bool STORE>
+__device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p, float4 c, int lane, float4* runs) {
     constexpr unsigned int kAll = 0xffffffffu;
     constexpr int kAhead = 2;
     const int grp = D.sgrp[p];
-    unsigned int* list = D.nbr + (size_t)p * D.cap;
+    unsigned int* list = STORE ? D.nbr + (size_t)32 * list_row(S, p) : nullptr;
     const bool image = S.nc == 1;  // one run, the whole box: minimum image per pair
     const int nc = S.nc, w = S.win, side = 2 * w + 1;
     const int cx = cell_of(c.x, S.invL, nc), cy = cell_of(c.y, S.invL, nc), cz = cell_of(c.z, S.invL, nc);
@@ -441,17 +446,14 @@ __device__ __forceinline__ int build_list(const FFDev& D, const FFSys& S, int p,
                 const bool hit = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)) < lim * lim && gq[k] != grp;
                 const unsigned int m = __ballot_sync(kAll, hit);
                 const int at = n + __popc(m & ((1u << lane) - 1u));
-                if (hit && at < D.cap) list[at] = (unsigned int)(q[k] - S.u0);
+                if (STORE && hit && at < S.cap) list[at] = (unsigned int)(q[k] - S.u0);
                 n += __popc(m);
             }
         }
     }
-    if (lane == 0) {
-        D.ncnt[p] = min(n, D.cap);
-        if (n > D.cap && D.sys_status) atomicOr(D.sys_status + s, 2u);
-    }
+    if (STORE && lane == 0) D.ncnt[p] = n;
     __syncwarp();  // the lanes read each other's entries
-    return min(n, D.cap);
+    return n;
 }
 
 // Compensated FP32 accumulator (Knuth's two-sum): the running sum keeps its rounding error in `lo`.
@@ -464,6 +466,19 @@ struct ESum {
     }
     __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
+
+// The longest list of each system (most, zero before), a warp per unit.
+__global__ void __launch_bounds__(128) ff_list_lengths(FFDev D, int* most) {
+    __shared__ float4 runs[4][32];
+    chain_release();
+    chain_wait();
+    const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31, p = blockIdx.x * 4 + warp;
+    if (p >= D.n_units) return;
+    const int s = D.usys[p];
+    const FFSys S = D.sys[s];
+    const int n = build_list<false>(D, S, p, D.scen[p], lane, runs[warp]);
+    if (lane == 0) atomicMax(most + s, n);
+}
 
 // Relaxation: the factor that caps an atom's force.
 __device__ __forceinline__ float force_scale(const FFDev& D, float fx, float fy, float fz) {
@@ -513,6 +528,8 @@ constexpr int kRing = 64;  // packed list entries per warp
 
 struct UnitTask {
     int p, s, n, lane;        // place, system, list entries
+    int row;                  // the unit's list (list_row), or where more units are in range than it holds
+                              // -1 - its group: every place of the system (the list at row 0) but the group's
     int k0;                   // the unit's first interacting atom
     int q0, q1;               // the lane's first two list entries (before clamping to n)
     float4 c;                 // centroid and radius
@@ -558,7 +575,7 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
     constexpr unsigned int kAll = 0xffffffffu;
     extern __shared__ float4 stab[];  // PT: the type-pair table
     const int lane = T.lane, nt = D.ntypes;
-    const unsigned int* nb = D.nbr + (size_t)T.p * D.cap;
+    const unsigned int* nb = D.nbr + (size_t)32 * max(T.row, 0);
     const int u0 = S.u0;
     const float4 c = T.c;
     const float two_krf = 2.0f * S.krf, rc2 = S.rc2;
@@ -655,7 +672,8 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                                          __int_as_float(q));
             const float ex = dx + e.x, ey = dy + e.y, ez = dz + e.z;
             const float lim = reach + cj.w;
-            const bool keep = e0 + lane < T.n && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < lim * lim;
+            const bool keep = e0 + lane < T.n && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < lim * lim &&
+                              !(T.row < 0 && D.sgrp[q] == -1 - T.row);
             const unsigned int m = __ballot_sync(kAll, keep);
             if (keep) T.ring[(head + held + __popc(m & ((1u << lane) - 1u))) & (kRing - 1)] = e;
             held += __popc(m);
@@ -765,13 +783,20 @@ __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long*
     T.c = D.scen[T.p];
     T.n = D.ncnt[T.p];
     const int2 kn = D.sunit[T.p];
-    const unsigned int* nb = D.nbr + (size_t)T.p * D.cap;
+    T.row = list_row(S, T.p);
+    const unsigned int* nb = D.nbr + (size_t)32 * T.row;
     T.q0 = (int)nb[T.lane];
-    T.q1 = (int)nb[min(32 + T.lane, D.cap - 1)];
+    T.q1 = (int)nb[min(32 + T.lane, S.cap - 1)];
     if (D.build[T.s]) {
-        T.n = build_list(D, S, T.p, T.s, T.c, T.lane, T.ring);
+        T.n = build_list<true>(D, S, T.p, T.c, T.lane, T.ring);
         T.q0 = (int)nb[T.lane];
-        T.q1 = (int)nb[min(32 + T.lane, D.cap - 1)];
+        T.q1 = (int)nb[min(32 + T.lane, S.cap - 1)];
+    }
+    if (T.n > S.cap) {
+        T.n = S.u1 - S.u0;
+        T.row = -1 - D.sgrp[T.p];
+        T.q0 = T.lane;
+        T.q1 = 32 + T.lane;
     }
     if (T.p == S.u0 && T.lane == 0) D.moved[T.s] = 0;  // for the next evaluation's ff_check
     T.k0 = kn.x;
@@ -836,43 +861,70 @@ int launch_forces_to_user(const long long* force, int stride, int natoms, double
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
+namespace {
+
+// The launches of an evaluation; after an error the others are left out of the result, not undone.
+struct Chain {
+    int n = 0;
+    cudaError_t e = cudaSuccess;
+    void put(cudaError_t r) {
+        if (e == cudaSuccess) e = r;
+        n++;
+    }
+};
+
+// Everything before the force pass.
+void put_prep(Chain& chain, const FFDev& D, int prec, const DevBuf& B, cudaStream_t st) {
+    const int t = 256, gg = (D.n_units + t - 1) / t;
+    if (D.prep_units) {
+        const int threads = D.prep_units >= 1024 ? 1024 : (D.prep_units + 31) / 32 * 32;
+        chain.put(launch_chained(ff_prep, D.S, threads, sizeof(int) * (D.prep_units + D.prep_cells), st, D, B, prec));
+    } else {
+        chain.put(launch_chained(ff_check, gg, t, 0, st, D, B, prec));
+        chain.put(launch_chained(ff_bin, gg, t, 0, st, D));
+        chain.put(launch_chained(ff_scan, D.S, 1024, 0, st, D));
+        chain.put(launch_chained(ff_scatter, gg, t, 0, st, D));
+        chain.put(launch_chained(ff_place, gg, t, 0, st, D, B, prec));
+    }
+}
+
+}  // namespace
+
+int launch_list_lengths(const FFDev& D, int prec, const DevBuf& B, int* most, void* stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    Chain chain;
+    chain.put(cudaMemsetAsync(most, 0, sizeof(int) * (size_t)D.S, st));
+    if (D.n_units) {
+        FFDev all = D;
+        all.force_all = 1;
+        put_prep(chain, all, prec, B, st);
+        chain.put(launch_chained(ff_list_lengths, (D.n_units + 3) / 4, 128, 0, st, all, most));
+    }
+    return chain.e == cudaSuccess ? chain.n : -1;
+}
+
 int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (D.n_int == 0) return 0;
-    const int t = 256, gg = (D.n_units + t - 1) / t;
-    int n = 0;
-    cudaError_t e = cudaSuccess;
-    auto put = [&](cudaError_t r) {
-        if (e == cudaSuccess) e = r;
-        n++;
-    };
-    if (D.prep_units) {
-        const int threads = D.prep_units >= 1024 ? 1024 : (D.prep_units + 31) / 32 * 32;
-        put(launch_chained(ff_prep, D.S, threads, sizeof(int) * (D.prep_units + D.prep_cells), st, D, B, prec));
-    } else {
-        put(launch_chained(ff_check, gg, t, 0, st, D, B, prec));
-        put(launch_chained(ff_bin, gg, t, 0, st, D));
-        put(launch_chained(ff_scan, D.S, 1024, 0, st, D));
-        put(launch_chained(ff_scatter, gg, t, 0, st, D));
-        put(launch_chained(ff_place, gg, t, 0, st, D, B, prec));
-    }
+    Chain chain;
+    put_prep(chain, D, prec, B, st);
     long long* f = const_cast<long long*>(B.force);
     switch (D.slots) {
-        case 1: put(launch_force_pass<1>(D, energy, f, B.stride, st)); break;
-        case 2: put(launch_force_pass<2>(D, energy, f, B.stride, st)); break;
-        case 3: put(launch_force_pass<3>(D, energy, f, B.stride, st)); break;
-        default: put(launch_force_pass<4>(D, energy, f, B.stride, st));
+        case 1: chain.put(launch_force_pass<1>(D, energy, f, B.stride, st)); break;
+        case 2: chain.put(launch_force_pass<2>(D, energy, f, B.stride, st)); break;
+        case 3: chain.put(launch_force_pass<3>(D, energy, f, B.stride, st)); break;
+        default: chain.put(launch_force_pass<4>(D, energy, f, B.stride, st));
     }
     if (energy) {
         const SystemChunks& c = D.e_chunks;
         double* part = c.n == D.S ? D.energy : c.part;  // every system one chunk: its sum is the result
-        put(launch_chained(ff_energy, c.n, 256, 0, st, D, part));
+        chain.put(launch_chained(ff_energy, c.n, 256, 0, st, D, part));
         if (part != D.energy) {
             if (launch_join_chunks(part, c.chunk0, D.S, 1, D.energy, stream) < 0) return -1;
-            n++;
+            chain.n++;
         }
     }
-    return e == cudaSuccess ? n : -1;
+    return chain.e == cudaSuccess ? chain.n : -1;
 }
 
 }  // namespace rbx

@@ -119,13 +119,13 @@ struct alignas(16) FFSys {
     float L, invL, rc, rc2;
     float krf, crf;
     float rl;          // cutoff + skin: units are listed when their centroids lie within rl + both radii
-    float half_skin2;  // (skin/2)^2: a centroid moved this far since the build invalidates the lists
-    int pair_image;    // 1: cutoff + two radii may reach half the box; the force pass takes the
-                       // minimum image per pair (else one shift per listed unit)
     float reach;       // rl + the system's largest radius (and a margin): a unit's list lies within this
                        // + its own radius
+    int pair_image;    // 1: cutoff + two radii may reach half the box; the force pass takes the
+                       // minimum image per pair (else one shift per listed unit)
     int win;           // cells on either side of a unit's own that may hold listed units (1 or 2)
-    int pad;
+    int cap;           // list entries allocated per unit (a multiple of 32)
+    int list0;         // the system's first list entry, in units of 32 entries
 };
 struct FFDev {
     int S, n_int, n_units, n_cells;
@@ -161,9 +161,11 @@ struct FFDev {
                              // evaluations
     unsigned char* build;    // [S] this evaluation's force pass builds the system's lists
     unsigned int* rebuilds;  // [S] list builds of each system so far (a statistic)
-    unsigned int* nbr;       // entry e of place p at p * cap + e: the listed unit's place - u0
-    int* ncnt;               // [n_units] p: entries
-    int cap;                 // entries per unit allocated
+    unsigned int* nbr;       // entry e of place p at 32 list0 + (p - u0) cap + e: the listed unit's place - u0.
+                             // Before the lists 0, 1, 2, ...: the list of every place of a system
+    int* ncnt;               // [n_units] p: units in range at the last build; where that is more than cap the
+                             // list is not used, and the force pass looks at every unit of the system
+    float half_skin2;        // (skin/2)^2: a centroid moved this far since the build invalidates the lists
     // Atom types (ntypes > 0): the distinct (sqrt(K) q, sigma/2, sqrt(epsilon)) of the interacting
     // atoms; spos .w then holds the atom's type (int bits), and the force pass takes each pair's
     // coefficients from a table of type pairs: entry (i, j) is K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j
@@ -172,9 +174,8 @@ struct FFDev {
     int ntypes;
     double* energy;       // [S] potential energy per system (kJ/mol)
     float fcap;           // > 0: each atom's force is scaled down to at most this magnitude
-    unsigned int* sys_status;  // [S] bit 0: a force of the system is non-finite or beyond the
-                               // fixed-point range (never during a capped relaxation); bit 1: a list
-                               // outgrew its capacity
+    unsigned int* sys_status;  // [S] non-zero: a force of the system is non-finite or beyond the
+                               // fixed-point range (never during a capped relaxation)
     // the largest system's units and list cells, where every system is small enough for one block
     // (prep_limit); prep_units = 0 otherwise
     int prep_units, prep_cells;
@@ -188,6 +189,9 @@ constexpr int kMaxSystemAtoms = 1 << 26;
 // kernels over all units and 4.66 in a block each.
 inline bool prep_limit(long long units, long long cells) { return units <= 1024 && units + cells <= 12000; }
 int launch_forces(const FFDev& D, int prec, const DevBuf& B, bool energy, void* stream);
+// most[s]: the length of the longest neighbour list of system s at the current positions, for sizing the lists
+// (nothing is stored of them; D.rebuilds is counted up).
+int launch_list_lengths(const FFDev& D, int prec, const DevBuf& B, int* most, void* stream);
 // Fixed-point forces of slots [0, natoms) -> user-order doubles out[3*natoms] (kJ/mol/nm).
 int launch_forces_to_user(const long long* force, int stride, int natoms, double* out, void* stream);
 
