@@ -591,6 +591,8 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
                 b->d_rebuilds.alloc(num_systems) != cudaSuccess || b->d_most.alloc(2 * (size_t)num_systems) != cudaSuccess))
         rc = set_error(RBX_ERR_CUDA, "cudaMalloc of force-field arrays failed");
     if (!rc && (cudaMemset(b->d_sys_status.p, 0, sizeof(unsigned int) * (size_t)num_systems) != cudaSuccess ||
+                // (a batch without interacting atoms has no force evaluation to write its energies)
+                cudaMemset(b->d_energy.p, 0, sizeof(double) * (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_cell_count.p, 0, sizeof(int) * (size_t)cells) != cudaSuccess ||
                 cudaMemset(b->d_moved.p, 0, (size_t)num_systems) != cudaSuccess ||
                 cudaMemset(b->d_build.p, 0, (size_t)num_systems) != cudaSuccess ||
