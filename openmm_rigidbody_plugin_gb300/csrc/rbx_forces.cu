@@ -519,8 +519,9 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 // work), records in cell order and by atom slot (contiguous lanes read contiguous records: a quarter
 // fewer L1 wavefronts), no Lennard-Jones term for the atoms that have none; then (17.5 -> 16.3 ms per
 // 20 steps) all that a place names fetched at once, predicated sums, halving sums over the lanes and
-// blocks of 4 warps (8: 16.7). Energies are added three pairs at a time to the compensated sum, without
-// branches (forces of 40 boxes with solutes 0.98 -> 0.80 ms). Not kept: 40 warps per SM at 48 registers
+// blocks of 4 warps (8: 16.7). Every pair's energy is added to the compensated sum on its own, without
+// branches; the pairs of one streamed atom added up first, in plain FP32, were narrower and no faster (forces
+// of 40 boxes with solutes 739 us, now 728). Not kept: 40 warps per SM at 48 registers
 // (19.2 ms); 24 at 80, with (20.5) or without (equal) the next atoms fetched before these are paired;
 // two atoms at a time in packed FP32 instructions (the FMA pipe takes as long; 5 % slower).
 constexpr int kFW = 4;    // warps (units) per block
@@ -606,7 +607,7 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
             const int tj = __float_as_int(xq[b].w);
             float4 pj;
             if (!PT) pj = D.spar[b][__float_as_int(e.w)];
-            float qj = PT ? 0.0f : pj.x, eb = 0.0f;
+            float qj = PT ? 0.0f : pj.x;
             // K q_i q_j, 12 C12, 6 C6 of the pair (and, from the table, the streamed atom's charge)
             auto coefficients = [&](int a) {
                 float4 t;
@@ -637,11 +638,11 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                     if (ENERGY) {
                         const float ep = t.x * (inv_r + S.krf * r2 - S.crf) +
                                          inv_r6 * (t.y * (1.0f / 12.0f) * inv_r6 - t.z * (1.0f / 6.0f));
-                        eb += in ? ep : 0.0f;
+                        en.add(in ? ep : 0.0f);
                     }
                 } else {
                     gf = qj * rf;
-                    if (ENERGY) eb += in ? qi[a] * qj * (inv_r + S.krf * r2 - S.crf) : 0.0f;
+                    if (ENERGY) en.add(in ? qi[a] * qj * (inv_r + S.krf * r2 - S.crf) : 0.0f);
                 }
                 if (in) {
                     f[a][0] = fmaf(gf, d.x, f[a][0]);
@@ -649,7 +650,6 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                     f[a][2] = fmaf(gf, d.z, f[a][2]);
                 }
             }
-            if (ENERGY) en.add(eb);
         }
     };
     const float reach = S.rc + c.w + 1e-6f;
