@@ -6,6 +6,7 @@ rotations of four products each, and L(0) + dL before them, roundings of 2^-53 (
 1.6e-16 rms over the three components' largest error. Whatever else is rounded into it shows: two square
 roots (each rounded to half an ulp or worse, and their product) make it 2.0e-16. The bound lies between,
 1.85e-16, and the largest error at 1e-15. The quaternion is renormalised: 1.1e-16 rms, 4e-16 at most."""
+import math
 import os
 import shutil
 import subprocess
@@ -115,3 +116,60 @@ def test_error_of_one_step(tmp_path):
         assert mL < 1e-15, (dt, kind, mL)
     mean = (sum(r[5] ** 2 for r in rows) / len(rows)) ** 0.5
     assert mean < 1.85e-16, mean
+
+
+JACOBI = r"""
+#include <algorithm>
+#include <cstdio>
+#include "rbx_math.cuh"
+using namespace rbx;
+typedef long double LD;
+
+// sn, cn, dn by the arithmetic-geometric mean (Abramowitz & Stegun 16.4) in long double
+static void agm(LD u, LD m1, LD* f) {  // m1 = 1 - m
+    LD a[40], c[40], b = sqrtl(m1);
+    a[0] = 1; c[0] = sqrtl(1 - m1);
+    int n = 0;
+    while (fabsl(c[n]) > 1e-19L && n < 30) {
+        a[n + 1] = 0.5L * (a[n] + b);
+        c[n + 1] = 0.5L * (a[n] - b);
+        b = sqrtl(a[n] * b);
+        n++;
+    }
+    LD phi = ldexpl(a[n] * u, n);
+    for (; n > 0; n--) phi = 0.5L * (phi + asinl(c[n] / a[n] * sinl(phi)));
+    f[0] = sinl(phi); f[1] = cosl(phi);
+    f[2] = sqrtl(m1 + (1 - m1) * f[1] * f[1]);
+}
+
+int main() {
+    for (double m1 : {0.99, 0.5, 0.1, 0.01, 1e-4, 1e-6, 1e-10})
+        for (double h : {1e-3, 0.02, 0.031, 0.06, 0.12, 0.25, 0.4999, 0.5001, 0.9, 1.7, 3.0, 7.0, 20.0, 100.0, 600.0, 1e4, 1e6, 1e12}) {
+            const double m = 1.0 - m1;
+            LD f[3];
+            agm(h, 1.0L - (LD)m, f);
+            double s, c, d, n, sn, cm1, dm1;
+            jacobi_homogeneous(h, m, s, c, d, n);
+            jacobi_small_t(h, m, sn, cm1, dm1);
+            const double e = (double)std::max({fabsl(s / (LD)n - f[0]), fabsl(c / (LD)n - f[1]), fabsl(d / (LD)n - f[2])});
+            const double r = (double)std::max({fabsl(sn - f[0]), fabsl(1 + (LD)cm1 - f[1]), fabsl(1 + (LD)dm1 - f[2])});
+            printf("%g %g %g %g\n", m1, h, e, r);
+        }
+    return 0;
+}
+"""
+
+
+def test_jacobi_functions_in_homogeneous_coordinates(tmp_path):
+    """sn, cn, dn as the quadrature takes them, of any argument, also next to the separatrix (1 - m from 0.99 to
+    1e-10), against the arithmetic-geometric mean in long double. Each of the k duplications from below 1/32
+    doubles the roundings (2^-53) before it, 2^k x 2^-53; beyond an argument h of 1/2 the quadrature itself is
+    off by 4e-13 h^10, and the functions need be no better. They are finite wherever the form that divides at
+    each duplication is."""
+    rows = run(tmp_path, JACOBI)
+    assert len(rows) == 7 * 18
+    for m1, h, error, divided in rows:
+        k = max(0, math.ceil(math.log2(h * 32)))
+        assert error == error or divided != divided, (m1, h)
+        if h <= 3.0:
+            assert error <= max(2.0 ** (k - 53), 4e-13 * h ** 10), (m1, h, error)
