@@ -675,9 +675,10 @@ __device__ __forceinline__ Q4<float> rotation_increment(const DevSys& S, int b, 
     return nosquish_increment(L, R, R.invI.z != 0.0f, dt, S.rot_n);
 }
 
-// qBt with its roundings written out: which product of a pair the compiler fuses may change with the
-// code around it (it did for NO-SQUISH, from one instantiation and one version of the kernel to the
-// next), and positions are kept to 48 bits.
+// qBt with its roundings written out, for NO-SQUISH in every form of the kernel: which product of a pair the
+// compiler fuses may change with the code around it (it did, from one form and one version of the kernel to
+// the next), positions are kept to 48 bits, and a body's step must not depend on the form that another
+// body of the handle asks for.
 __device__ __forceinline__ V3<float> body_momentum2(Q4<float> q, Q4<float> y) {
     const float x0 = __fmaf_rn(-q.x, y.w, __fmul_rn(q.w, y.x));
     const float y0 = __fmaf_rn(-q.y, y.w, -__fmul_rn(q.z, y.x));
@@ -699,7 +700,6 @@ template <int KIND, bool REF> constexpr int step_threads() { return KIND == STEP
 template <int P, int KIND, bool EXACT, bool REF, int NT, bool LARGE>
 __global__ void __launch_bounds__(NT, (step_threads<KIND, REF>() / NT)) step_kernel_f(DevSys S, DevBuf B, double dt_d) {
     using FSmem = rbx::FSmem<NT>;
-    constexpr bool kWritten = !EXACT && !REF && !(LARGE && P == PREC_MIXED);  // the forms that round so
     constexpr int APT = 4;  // body atoms per thread in phase 1
     chain_release();
     const int tile = block_tile(S);
@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(NT, (step_threads<KIND, REF>() / NT)) step_ker
         } else {
 #pragma unroll
             for (int c = 0; c < 3; c++) x[c] = ff_acc(x[c], fmaf(x[3 + c].hi, dt, x[3 + c].lo * dt));  // drift
-            const V3<float> L = (kWritten ? body_momentum2(qh, ph) : qBt(qh, ph)) * 0.5f;
+            const V3<float> L = (EXACT ? qBt(qh, ph) : body_momentum2(qh, ph)) * 0.5f;
             const Q4<float> dr = rotation_increment<EXACT>(S, b, L, R, dt);
             const Q4<float> dq = qmul(qh, dr), dp = qmul(ph, dr);
             x[6] = ff_acc(x[6], dq.w); x[7] = ff_acc(x[7], dq.x); x[8] = ff_acc(x[8], dq.y); x[9] = ff_acc(x[9], dq.z);
