@@ -109,7 +109,7 @@ struct rbx_batch {
     DevArray<FFSys> d_sys;
     DevArray<int> d_iatom, d_ugrp, d_usys, d_place, d_unit_at, d_cell_count, d_cell_start, d_cell_cursor;
     DevArray<int> d_sgrp, d_ncnt, d_atype;
-    DevArray<int2> d_unit, d_sunit;
+    DevArray<int2> d_unit, d_sunit, d_sys_types;
     DevArray<float4> d_param, d_ucen, d_uref, d_scen, d_spos, d_spar, d_types;
     DevArray<unsigned char> d_moved, d_build;
     DevArray<unsigned int> d_skey;      // FFDev::skey
@@ -264,6 +264,38 @@ int unit_atoms(const std::vector<int>& group_sizes) {
         }
     }
     return best;
+}
+
+// The types of atoms [k0, k1): the distinct triples in order of appearance and each atom's index among them;
+// false (and no atom of a type) when there are more than kMaxTypes.
+bool atom_types(const std::vector<float4>& param, size_t k0, size_t k1, std::vector<float4>& types, std::vector<int>& type_of) {
+    std::map<std::array<float, 3>, int> seen;
+    types.clear();
+    for (size_t k = k0; k < k1; k++) {
+        const auto it = seen.emplace(std::array<float, 3>{param[k].x, param[k].y, param[k].z}, (int)types.size()).first;
+        if (it->second == (int)types.size()) {
+            if (it->second == kMaxTypes) {
+                std::fill(type_of.begin() + k0, type_of.begin() + k, 0);
+                return false;
+            }
+            types.push_back(param[k]);
+        }
+        type_of[k] = it->second;
+    }
+    return true;
+}
+
+// Type-pair table: (K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j) with C12 = 4 eps sig^12, C6 = 4 eps sig^6 and
+// Lorentz-Berthelot sig = (sig_i + sig_j)/2, eps = sqrt(eps_i eps_j), formed in FP64 from the
+// FP32 type values (the force is (12 C12 r^-6 - 6 C6) r^-8 r).
+void append_pair_table(const std::vector<float4>& types, std::vector<float4>& table) {
+    for (const float4& i : types)
+        for (const float4& j : types) {
+            const double sig = (double)i.y + (double)j.y, eps = (double)i.z * (double)j.z;
+            const double s6 = sig * sig * sig * sig * sig * sig;
+            table.push_back(make_float4((float)((double)i.x * (double)j.x), (float)(48.0 * eps * s6 * s6),
+                                        (float)(24.0 * eps * s6), j.x));
+        }
 }
 
 DevBuf buffers(rbx_batch* b) {
@@ -543,45 +575,40 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     std::vector<int> units_of(num_systems);
     for (int s = 0; s < num_systems; s++) units_of[s] = sys[s].u1 - sys[s].u0;
     if (!rc) rc = b->e_chunks.set(units_of, kEnergyChunk, 1);
-    // atom types: the distinct (scaled charge, sigma/2, sqrt(epsilon)) triples; with at most
-    // kMaxTypes of them the force pass reads one 16-byte record per neighbour (position and type)
-    // and takes each pair's coefficients from a table of type pairs
-    std::vector<float4> types;
-    std::vector<int> type_of(param.size(), -1);
-    {
-        std::map<std::array<float, 3>, int> seen;
-        for (size_t k = 0; k < param.size() && (int)types.size() <= kMaxTypes; k++) {
-            const std::array<float, 3> key{param[k].x, param[k].y, param[k].z};
-            auto it = seen.find(key);
-            if (it == seen.end()) {
-                it = seen.emplace(key, (int)types.size()).first;
-                types.push_back(make_float4(key[0], key[1], key[2], 0.0f));
+    // atom types: the distinct (scaled charge, sigma/2, sqrt(epsilon)) triples. A system of at most kMaxTypes
+    // types takes each pair's coefficients from a table of type pairs, whatever the systems beside it: one table
+    // for the batch where its types fit one together, else a table per such system
+    std::vector<float4> pair_table;
+    std::vector<int> type_of(param.size(), 0);
+    std::vector<int2> sys_types;
+    int nt = 0;
+    if (!param.empty()) {
+        std::vector<float4> types;
+        if (atom_types(param, 0, param.size(), types, type_of)) {
+            nt = (int)types.size();
+            append_pair_table(types, pair_table);
+        } else {
+            bool any = false;
+            auto first_atom = [&](int u) { return u < nunit ? (size_t)unit[u].x : param.size(); };
+            for (int s = 0; s < num_systems; s++) {
+                const bool typed = atom_types(param, first_atom(sys[s].u0), first_atom(sys[s].u1), types, type_of);
+                sys_types.push_back(typed ? make_int2((int)pair_table.size(), (int)types.size()) : make_int2(0, 0));
+                if (typed) append_pair_table(types, pair_table);
+                any = any || typed;
             }
-            type_of[k] = it->second;
+            if (!any) sys_types.clear();
         }
-        if ((int)types.size() > kMaxTypes) types.clear();
     }
-    if (types.empty()) type_of.clear();
-    // the type-pair table: (K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j) with C12 = 4 eps sig^12, C6 = 4 eps sig^6 and
-    // Lorentz-Berthelot sig = (sig_i + sig_j)/2, eps = sqrt(eps_i eps_j), formed in FP64 from the
-    // FP32 type values (the force is (12 C12 r^-6 - 6 C6) r^-8 r)
-    const int nt = (int)types.size();
-    std::vector<float4> pair_table((size_t)nt * nt);
-    for (int i = 0; i < nt; i++)
-        for (int j = 0; j < nt; j++) {
-            const double sig = (double)types[i].y + (double)types[j].y, eps = (double)types[i].z * (double)types[j].z;
-            const double s6 = sig * sig * sig * sig * sig * sig;
-            pair_table[(size_t)i * nt + j] = make_float4((float)((double)types[i].x * (double)types[j].x),
-                                                         (float)(48.0 * eps * s6 * s6), (float)(24.0 * eps * s6), types[j].x);
-        }
+    if (pair_table.empty()) type_of.clear();
     if (!rc) rc = upload_vec(b->d_types, pair_table);
     if (!rc) rc = upload_vec(b->d_atype, type_of);
+    if (!rc) rc = upload_vec(b->d_sys_types, sys_types);
     const size_t u1 = std::max(nunit, 1), records = u1 * slots;
     if (!rc && (b->d_place.alloc(u1) != cudaSuccess || b->d_unit_at.alloc(u1) != cudaSuccess ||
                 b->d_ucen.alloc(u1) != cudaSuccess ||
                 b->d_uref.alloc(u1) != cudaSuccess || b->d_scen.alloc(u1) != cudaSuccess ||
                 b->d_sgrp.alloc(u1) != cudaSuccess || b->d_sunit.alloc(u1) != cudaSuccess || b->d_ncnt.alloc(u1) != cudaSuccess ||
-                b->d_spos.alloc(records) != cudaSuccess || b->d_spar.alloc(types.empty() ? records : 0) != cudaSuccess ||
+                b->d_spos.alloc(records) != cudaSuccess || b->d_spar.alloc(nt ? 0 : records) != cudaSuccess ||
                 b->d_cell_count.alloc(cells) != cudaSuccess || b->d_cell_start.alloc(cells + 1) != cudaSuccess ||
                 b->d_cell_cursor.alloc(cells) != cudaSuccess || b->d_e_unit.alloc(u1) != cudaSuccess ||
                 b->d_skey.alloc(u1) != cudaSuccess ||
@@ -628,7 +655,7 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.sunit = b->d_sunit.p;
     for (int a = 0; a < kMaxUnit; a++) {
         D.spos[a] = a < slots ? b->d_spos.p + a * u1 : nullptr;
-        D.spar[a] = a < slots && types.empty() ? b->d_spar.p + a * u1 : nullptr;
+        D.spar[a] = a < slots && !nt ? b->d_spar.p + a * u1 : nullptr;
     }
     D.slots = slots;
     D.e_unit = b->d_e_unit.p;
@@ -645,7 +672,8 @@ int rbx_batch_create(rbx_batch** out, int num_systems, const int* atom_offsets, 
     D.half_skin2 = (float)(0.25 * kSkin * kSkin);
     D.types = b->d_types.p;
     D.atype = b->d_atype.p;
-    D.ntypes = (int)types.size();
+    D.ntypes = nt;
+    D.sys_types = b->d_sys_types.p;
     D.prep_units = 0;
     D.prep_cells = 0;
     D.skey = b->d_skey.p;
@@ -872,7 +900,7 @@ int rbx_batch_memory(const rbx_batch* b, size_t* bytes) {
                b->d_usys.bytes() + b->d_ucen.bytes() + b->d_uref.bytes() + b->d_place.bytes() +
                b->d_unit_at.bytes() + b->d_cell_count.bytes() + b->d_cell_start.bytes() + b->d_cell_cursor.bytes() +
                b->d_scen.bytes() + b->d_sgrp.bytes() + b->d_sunit.bytes() + b->d_spos.bytes() + b->d_spar.bytes() +
-               b->d_skey.bytes() + b->d_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() +
+               b->d_skey.bytes() + b->d_types.bytes() + b->d_sys_types.bytes() + b->d_atype.bytes() + b->d_moved.bytes() +
                b->d_build.bytes() + b->d_nbr.bytes() + b->d_ncnt.bytes() + b->d_rebuilds.bytes() + b->d_most.bytes() +
                b->d_e_unit.bytes() + b->d_energy.bytes() + b->d_body0.bytes() + b->d_free0.bytes() +
                b->d_sys_status.bytes() + b->d_ke.bytes() + b->d_user.bytes() + b->ke_chunks.bytes() +

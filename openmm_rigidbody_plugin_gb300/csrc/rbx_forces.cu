@@ -114,7 +114,7 @@ __device__ __forceinline__ void write_place(const FFDev& D, int p, int k0, int n
 #pragma unroll
     for (int a = 0; a < kMaxUnit; a++) {
         if (a >= D.slots) break;
-        D.spos[a][p] = a < n ? make_float4(x[a].x, x[a].y, x[a].z, D.ntypes ? __int_as_float(D.atype[k0 + a]) : 0.0f)
+        D.spos[a][p] = a < n ? make_float4(x[a].x, x[a].y, x[a].z, D.atype ? __int_as_float(D.atype[k0 + a]) : 0.0f)
                      : make_float4(kFar, kFar, kFar, 0.0f);
     }
 }
@@ -154,7 +154,7 @@ __device__ __forceinline__ void settle(const FFDev& D, const DevBuf& B, int prec
     unit_positions(D, B, prec, k0, n, x);
     atoms_about(S, n, c, x);
     write_place(D, p, k0, n, c, x);
-    if (!D.ntypes)
+    if (D.spar[0])
         for (int a = 0; a < D.slots; a++) D.spar[a][p] = a < n ? D.param[k0 + a] : make_float4(0.f, 0.f, 0.f, 0.f);
     D.place[u] = p;
     D.unit_at[p] = u;
@@ -506,8 +506,10 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 // Atoms sit at their images nearest their own unit's centroid, so the unit shift gives the minimum
 // image of every pair within the cutoff when cutoff + two radii < L/2; systems of smaller boxes
 // (FFSys::pair_image) take the minimum image per pair as well.
-// With at most kMaxTypes atom types (PT) each pair's (K q_i q_j, 12 C12, 6 C6) comes from a type-pair
-// table in shared memory, else from the atoms' own parameters by Lorentz-Berthelot.
+// In systems of at most kMaxTypes atom types each pair's (K q_i q_j, 12 C12, 6 C6) comes from a type-pair table, else
+// from the atoms' own parameters by Lorentz-Berthelot (the two round differently, so the form follows from the
+// system alone). The table is in shared memory where one holds the types of the whole batch, else the system's
+// own is read through L1.
 // The pair term is OpenMM's CutoffPeriodic form: reaction-field Coulomb and unshifted LJ.
 //
 // Bound: instruction issue (62 % of the slots used), the L1 data pipe (53 to 67 %) and load latency, not
@@ -527,12 +529,15 @@ __device__ __forceinline__ void store_force(const FFDev& D, long long* __restric
 constexpr int kFW = 4;    // warps (units) per block
 constexpr int kRing = 64;  // packed list entries per warp
 
+enum PairForm { kAtomParams, kSharedTable, kSystemTable };
+
 struct UnitTask {
     int p, s, n, lane;        // place, system, list entries
     int row;                  // the unit's list (list_row), or where more units are in range than it holds
                               // -1 - its group: every place of the system (the list at row 0) but the group's
     int k0;                   // the unit's first interacting atom
     int q0, q1;               // the lane's first two list entries (before clamping to n)
+    int2 types;               // kSystemTable: FFDev::sys_types of the system
     float4 c;                 // centroid and radius
     float4* ring;
 };
@@ -570,12 +575,14 @@ template <int N> __device__ __forceinline__ int join_lanes(float (&v)[N], int la
 // NI atoms of the unit, the first NL with Lennard-Jones (the others Coulomb only: their pairs skip it,
 // and the unit's charge is applied once, to the sum). JS: atom records per place. RELAX: coincident
 // atoms have no direction and add nothing. PI: the minimum image per pair.
-template <int JS, int NI, int NL, bool ENERGY, bool PT, bool RELAX, bool PI>
+template <int JS, int NI, int NL, bool ENERGY, PairForm PF, bool RELAX, bool PI>
 __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, const UnitTask& T, long long* __restrict__ force,
                                             int stride) {
     constexpr unsigned int kAll = 0xffffffffu;
-    extern __shared__ float4 stab[];  // PT: the type-pair table
-    const int lane = T.lane, nt = D.ntypes;
+    constexpr bool PT = PF != kAtomParams;
+    extern __shared__ float4 stab[];  // kSharedTable: the type-pair table
+    const float4* const table = PF == kSharedTable ? stab : D.types + T.types.x;
+    const int lane = T.lane, nt = PF == kSharedTable ? D.ntypes : T.types.y;
     const unsigned int* nb = D.nbr + (size_t)32 * max(T.row, 0);
     const int u0 = S.u0;
     const float4 c = T.c;
@@ -591,8 +598,8 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
         xi[a][2] = x.z;
         f[a][0] = f[a][1] = f[a][2] = 0.0f;
         if (PT) {
-            row[a] = stab + __float_as_int(x.w) * nt;
-            qi[a] = stab[__float_as_int(x.w)].w;
+            row[a] = table + __float_as_int(x.w) * nt;
+            qi[a] = table[__float_as_int(x.w)].w;
         } else {
             pi[a] = D.spar[a][T.p];
             qi[a] = pi[a].x;
@@ -736,36 +743,41 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
 // The unit's exact size (the same choice for every lane): 3 atoms of which one has LJ is a 3-site
 // water, with a pair table or without (20 steps of 40 boxes of 700 to 3100 waters around 64-type solutes
 // 5.95 -> 5.57 ms for the latter); other units take the full term for every atom.
-template <int JS, bool ENERGY, bool PT, bool RELAX, bool PI>
+template <int JS, bool ENERGY, PairForm PF, bool RELAX, bool PI>
 __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, const UnitTask& T, int ni, int nl,
                                               long long* force, int stride) {
-    if (JS >= 4 && ni == 4) return unit_forces<JS, JS >= 4 ? 4 : 1, JS >= 4 ? 4 : 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
+    if (JS >= 4 && ni == 4) return unit_forces<JS, JS >= 4 ? 4 : 1, JS >= 4 ? 4 : 1, ENERGY, PF, RELAX, PI>(D, S, T, force, stride);
     if (JS >= 3 && ni == 3) {
-        if (nl <= 1) return unit_forces<JS, JS >= 3 ? 3 : 1, 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
-        return unit_forces<JS, JS >= 3 ? 3 : 1, JS >= 3 ? 3 : 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
+        if (nl <= 1) return unit_forces<JS, JS >= 3 ? 3 : 1, 1, ENERGY, PF, RELAX, PI>(D, S, T, force, stride);
+        return unit_forces<JS, JS >= 3 ? 3 : 1, JS >= 3 ? 3 : 1, ENERGY, PF, RELAX, PI>(D, S, T, force, stride);
     }
-    if (JS >= 2 && ni == 2) return unit_forces<JS, JS >= 2 ? 2 : 1, JS >= 2 ? 2 : 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
-    unit_forces<JS, 1, 1, ENERGY, PT, RELAX, PI>(D, S, T, force, stride);
+    if (JS >= 2 && ni == 2) return unit_forces<JS, JS >= 2 ? 2 : 1, JS >= 2 ? 2 : 1, ENERGY, PF, RELAX, PI>(D, S, T, force, stride);
+    unit_forces<JS, 1, 1, ENERGY, PF, RELAX, PI>(D, S, T, force, stride);
 }
 
 // Blocks per SM: 64 registers a thread (32 warps per SM); 80 for units of four atoms. The larger variants
 // then spill a little and still gain: forces of 40 boxes with 64-type solutes take 1.09 ms at 128
 // registers, 0.98 at 80 and 0.97 at 64 (later, with the list build's code, 0.75 at 80 and 0.77 at 64: the
-// form without the type-pair table takes 80).
+// form without the type-pair table takes 80, and so does the one with tables per system: 20 steps of 20 boxes
+// of waters beside 20 with solutes 4.95 ms, at 64 registers 5.16, at 96 4.93, at 128 5.46; all without a table,
+// as such batches once were, 4.85).
 constexpr int force_blocks(int records) { return records <= 3 ? 8 : 6; }
 constexpr int kUntypedBlocks = 6;
 // Batches of at most kFewUnits units (two warps per scheduler) leave the SMs nearly empty: a warp's own
 // chain of instructions is then the time, and 128 registers let more of it overlap (512 waters, 20 steps
-// with energies and a frame: 475 against 537 us; at 2600 units, 683 against 662).
+// with energies and a frame: 475 against 537 us; at 2600 units, 683 against 662). With tables per system, whose
+// kernel is the larger, up to a wave of such blocks, twice that (1770 units in four boxes of the mix beside two
+// with solutes, 20 steps: 0.50 against 0.62 ms).
 constexpr int kFewUnits = 8 * kSMs, kFewBlocks = 4;
 
-template <int JS, bool ENERGY, bool PT, bool RELAX, int BLOCKS>
+// PF: kSharedTable, one table for the batch; kSystemTable, a table for some of its systems; kAtomParams, for none.
+template <int JS, bool ENERGY, PairForm PF, bool RELAX, int BLOCKS>
 __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long* __restrict__ force, int stride) {
-    extern __shared__ float4 stab[];  // PT: the type-pair table
+    extern __shared__ float4 stab[];  // kSharedTable: the type-pair table
     __shared__ float4 ring[kFW][kRing];
     chain_release();
     const int nt = D.ntypes;
-    if (PT) {
+    if (PF == kSharedTable) {
         for (int t = threadIdx.x; t < nt * nt; t += blockDim.x) stab[t] = D.types[t];
         __syncthreads();
     }
@@ -776,6 +788,7 @@ __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long*
     T.lane = (int)threadIdx.x & 31;
     T.s = on ? D.usys[T.p] : 0;
     const FFSys S = D.sys[T.s];
+    if (PF == kSystemTable) T.types = D.sys_types[T.s];
     chain_wait();
     if (!on) return;
     T.ring = ring[warp];
@@ -801,10 +814,12 @@ __global__ void __launch_bounds__(32 * kFW, BLOCKS) ff_force(FFDev D, long long*
     if (T.p == S.u0 && T.lane == 0) D.moved[T.s] = 0;  // for the next evaluation's ff_check
     T.k0 = kn.x;
     const int ni = kn.y & 0xff, nl = kn.y >> 8;
-    if (S.pair_image)
-        unit_dispatch<JS, ENERGY, PT, RELAX, true>(D, S, T, ni, nl, force, stride);
-    else
-        unit_dispatch<JS, ENERGY, PT, RELAX, false>(D, S, T, ni, nl, force, stride);
+    if (PF == kSystemTable && T.types.y == 0) {
+        if (S.pair_image) return unit_dispatch<JS, ENERGY, kAtomParams, RELAX, true>(D, S, T, ni, nl, force, stride);
+        return unit_dispatch<JS, ENERGY, kAtomParams, RELAX, false>(D, S, T, ni, nl, force, stride);
+    }
+    if (S.pair_image) return unit_dispatch<JS, ENERGY, PF, RELAX, true>(D, S, T, ni, nl, force, stride);
+    unit_dispatch<JS, ENERGY, PF, RELAX, false>(D, S, T, ni, nl, force, stride);
 }
 
 // Shared memory is set aside for the resident blocks only (each its ring, its table and 1 KB of the
@@ -818,9 +833,15 @@ cudaError_t launch_force_kernel(const FFDev& D, long long* f, int stride, cudaSt
         const size_t block_shared = sizeof(float4) * kFW * kRing + table + 1024;
         return launch_chained_l1<FFDev, long long*, int>(blocks * block_shared, kernel, grid, 32 * kFW, table, st, D, f, stride);
     };
-    if (!D.ntypes) return launch(kUntypedBlocks, ff_force<JS, ENERGY, false, RELAX, kUntypedBlocks>);
-    if (!RELAX && D.n_units <= kFewUnits) return launch(kFewBlocks, ff_force<JS, ENERGY, true, RELAX, kFewBlocks>);
-    return launch(force_blocks(JS), ff_force<JS, ENERGY, true, RELAX, force_blocks(JS)>);
+    if constexpr (!RELAX) {
+        if (D.sys_types && D.n_units <= 2 * kFewUnits)
+            return launch(kFewBlocks, ff_force<JS, ENERGY, kSystemTable, RELAX, kFewBlocks>);
+        if (D.ntypes && D.n_units <= kFewUnits)
+            return launch(kFewBlocks, ff_force<JS, ENERGY, kSharedTable, RELAX, kFewBlocks>);
+    }
+    if (D.sys_types) return launch(kUntypedBlocks, ff_force<JS, ENERGY, kSystemTable, RELAX, kUntypedBlocks>);
+    if (!D.ntypes) return launch(kUntypedBlocks, ff_force<JS, ENERGY, kAtomParams, RELAX, kUntypedBlocks>);
+    return launch(force_blocks(JS), ff_force<JS, ENERGY, kSharedTable, RELAX, force_blocks(JS)>);
 }
 
 // A capped relaxation forms no energies.

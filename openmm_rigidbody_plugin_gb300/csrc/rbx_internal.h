@@ -149,7 +149,7 @@ struct FFDev {
     // p: atom records x, y, z (at the image nearest the unit's centroid), type: record a of place p at
     // spos[a][p] (a < slots; those past the unit's atoms lie far outside every cutoff)
     float4* spos[kMaxUnit];
-    float4* spar[kMaxUnit];  // p: the atoms' parameters, likewise (more than kMaxTypes types only)
+    float4* spar[kMaxUnit];  // p: the atoms' parameters, likewise (batches without one table only)
     int slots;
     double* e_unit;       // [n_units] u: half pair-energy sums (energy evaluations)
     SystemChunks e_chunks;  // of the units of each system
@@ -166,10 +166,15 @@ struct FFDev {
     int* ncnt;               // [n_units] p: units in range at the last build; where that is more than cap the
                              // list is not used, and the force pass looks at every unit of the system
     float half_skin2;        // (skin/2)^2: a centroid moved this far since the build invalidates the lists
-    // Atom types (ntypes > 0): the distinct (sqrt(K) q, sigma/2, sqrt(epsilon)) of the interacting
-    // atoms; spos .w then holds the atom's type (int bits), and the force pass takes each pair's
-    // coefficients from a table of type pairs: entry (i, j) is K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j
-    const float4* types;     // [ntypes * ntypes] the type-pair table
+    // Atom types: the distinct (sqrt(K) q, sigma/2, sqrt(epsilon)) of the interacting atoms. In a system of at
+    // most kMaxTypes of them spos .w holds the atom's type (int bits), and the force pass takes each pair's
+    // coefficients from a table of type pairs: entry (i, j) is K q_i q_j, 12 C12, 6 C6, sqrt(K) q_j. One table of
+    // ntypes types for the whole batch where they fit one together; otherwise (ntypes 0) sys_types[s] is the
+    // (first entry, types) of system s's own, (0, 0) for a system of more types, which takes the atoms'
+    // parameters (sys_types null: every system). A system's form, and its results with it, so depend on
+    // its own atoms alone.
+    const float4* types;     // the type-pair table or tables
+    const int2* sys_types;   // [S] or null
     const int* atype;        // [n_int] type of each interacting atom
     int ntypes;
     double* energy;       // [S] potential energy per system (kJ/mol)

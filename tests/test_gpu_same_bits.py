@@ -1,5 +1,7 @@
-"""A body's step is the same bit for bit whatever else the handle holds: beside a body of more than 32 atoms
-(which selects another form of the step kernel) and, under NO-SQUISH, with refined energies on."""
+"""A body's step and a system's forces are the same bit for bit whatever else the handle holds: a body
+beside one of more than 32 atoms (which selects another form of the step kernel) or, under NO-SQUISH, with
+refined energies on; a system of few atom types beside others that together have too many for one
+pair table."""
 import numpy as np
 import pytest
 
@@ -49,3 +51,50 @@ def test_bodies_beside_a_large_one_and_with_refined_energies(mode, prec):
         bodies = s.body_indices > 0
         for a, b in zip(plain, refined):
             assert np.array_equal(a[bodies], b[bodies]), np.abs(a - b)[bodies].max()
+
+
+def _box(rng, edge, per_edge, types, sizes):
+    """Bodies near a lattice, atom n of type n % types, types with charges of their own."""
+    g = (np.arange(per_edge) + 0.5) * edge / per_edge
+    at = np.stack(np.meshgrid(g, g, g, indexing="ij"), axis=-1).reshape(-1, 3)
+    size = np.resize(sizes, len(at))
+    owner = np.repeat(np.arange(len(at)), size)
+    n = len(owner)
+    a = np.arange(n) - (np.cumsum(size) - size)[owner]
+    x = at[owner] + 0.1 * np.stack([a % 2, a // 2 % 2, a // 4], axis=1) + 0.01 * rng.standard_normal((n, 3))
+    t = np.arange(n) % types
+    return (x, (owner + 1).astype(np.int32), 0.4 * np.cos(0.3 + 0.9 * np.pi * t / types), 0.2 + 0.001 * (t % 17),
+            np.where(t % 3, 0.0, 0.2 + 0.003 * t))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "double"])
+@pytest.mark.parametrize("types,sizes,edge,per_edge", [
+    (3, [3], 3.0, 8),            # waters
+    (12, [3, 4, 1, 6], 3.4, 8),  # units of one to four atoms
+    (5, [3], 1.9, 5),            # one cell, the minimum image per pair
+    (32, [2], 3.0, 8)])
+def test_system_of_few_types_beside_one_of_many(types, sizes, edge, per_edge, precision):
+    from openmm_rigidbody_plugin_gb300 import batch, build
+    build.build_library()
+    rng = np.random.default_rng(types)
+    few, many = _box(rng, edge, per_edge, types, sizes), _box(rng, 3.2, 6, 77, [3, 5, 2])
+    other = _box(rng, 4.2, 9, 31, [3])  # few types of its own, together more than 32
+
+    def run(systems, edges):
+        x, _, q, s, e = (np.concatenate(c) for c in zip(*systems))
+        body = np.concatenate([w[1] + 10000 * i for i, w in enumerate(systems)]).astype(np.int32)
+        off = np.concatenate([[0], np.cumsum([len(w[0]) for w in systems])])
+        b = batch.BatchedSystems(np.full(len(x), 12.0), body, off, edges, [0.8] * len(systems), q, s, e, precision=precision)
+        b.set_state(x, np.zeros_like(x))
+        f, u = b.forces()
+        b.relax(4)
+        b.step(5, 0.001)
+        xs, vs = b.get_state()
+        n = off[1]
+        return f[:n], u[0], xs[:n], vs[:n], b.energies()[0]
+
+    alone = run([few], [edge])
+    for beside in ([few, many], [few, other], [few, many, other]):
+        edges = [edge] + [3.2 if w is many else 4.2 for w in beside[1:]]
+        for a, b in zip(alone, run(beside, edges)):
+            assert np.array_equal(a, b), np.abs(np.asarray(a) - np.asarray(b)).max()
