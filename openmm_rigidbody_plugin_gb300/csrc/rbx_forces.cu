@@ -636,6 +636,8 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                 const bool in = r2 < rc2 && !(PI && xq[b].x >= 0.5f * kFar) && !(RELAX && r2 < 1e-8f);
                 const float inv_r = rsqrtf(r2), inv_r2 = inv_r * inv_r;
                 const float rf = fmaf(inv_r, inv_r2, -two_krf);
+                // (energies with their roundings written out: the same in every form of the kernel)
+                const float coulomb_energy = __fadd_rn(__fmaf_rn(S.krf, r2, inv_r), -S.crf);
                 float gf;
                 if (a < NL) {
                     const float4 t = coefficients(a);
@@ -643,13 +645,12 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                     const float lj = inv_r6 * fmaf(t.y, inv_r6, -t.z);  // 12 C12 r^-12 - 6 C6 r^-6
                     gf = fmaf(t.x, rf, lj * inv_r2);
                     if (ENERGY) {
-                        const float ep = t.x * (inv_r + S.krf * r2 - S.crf) +
-                                         inv_r6 * (t.y * (1.0f / 12.0f) * inv_r6 - t.z * (1.0f / 6.0f));
-                        en.add(in ? ep : 0.0f);
+                        const float lj_energy = __fmaf_rn(__fmul_rn(t.y, 1.0f / 12.0f), inv_r6, -__fmul_rn(t.z, 1.0f / 6.0f));
+                        en.add(in ? __fmaf_rn(t.x, coulomb_energy, __fmul_rn(inv_r6, lj_energy)) : 0.0f);
                     }
                 } else {
                     gf = qj * rf;
-                    if (ENERGY) en.add(in ? qi[a] * qj * (inv_r + S.krf * r2 - S.crf) : 0.0f);
+                    if (ENERGY) en.add(in ? __fmul_rn(__fmul_rn(qi[a], qj), coulomb_energy) : 0.0f);
                 }
                 if (in) {
                     f[a][0] = fmaf(gf, d.x, f[a][0]);

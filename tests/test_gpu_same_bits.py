@@ -98,3 +98,35 @@ def test_system_of_few_types_beside_one_of_many(types, sizes, edge, per_edge, pr
         edges = [edge] + [3.2 if w is many else 4.2 for w in beside[1:]]
         for a, b in zip(alone, run(beside, edges)):
             assert np.array_equal(a, b), np.abs(np.asarray(a) - np.asarray(b)).max()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "double"])
+def test_waters_beside_units_of_other_sizes_and_in_batches_of_other_sizes(precision):
+    """What a batch chooses for all of its systems (records per place, registers of the force pass, the set-up
+    in one launch or in several) changes no system's bits."""
+    from openmm_rigidbody_plugin_gb300 import batch, build
+    build.build_library()
+    rng = np.random.default_rng(8)
+    waters = _box(rng, 3.0, 8, 3, [3])
+    fours, singles, crowd = _box(rng, 3.0, 6, 5, [4]), _box(rng, 3.0, 7, 2, [1]), _box(rng, 6.2, 14, 3, [3])
+    many = _box(rng, 3.2, 6, 77, [3, 5, 2])
+
+    def run(systems, edges):
+        x, _, q, s, e = (np.concatenate(c) for c in zip(*systems))
+        body = np.concatenate([w[1] + 10000 * i for i, w in enumerate(systems)]).astype(np.int32)
+        off = np.concatenate([[0], np.cumsum([len(w[0]) for w in systems])])
+        b = batch.BatchedSystems(np.full(len(x), 12.0), body, off, edges, [0.8] * len(systems), q, s, e, precision=precision)
+        b.set_state(x, np.zeros_like(x))
+        f, u = b.forces()
+        b.relax(4)
+        b.step(5, 0.001)
+        xs, vs = b.get_state()
+        n = off[1]
+        return f[:n], u[0], xs[:n], vs[:n], b.energies()[0]
+
+    alone = run([waters], [3.0])
+    for beside in ([(fours, 3.0)], [(singles, 3.0)], [(crowd, 6.2)], [(fours, 3.0), (crowd, 6.2)], [(many, 3.2), (crowd, 6.2)],
+                   [(many, 3.2), (fours, 3.0)]):
+        got = run([waters] + [w for w, _ in beside], [3.0] + [edge for _, edge in beside])
+        for a, b in zip(alone, got):
+            assert np.array_equal(a, b), np.abs(np.asarray(a) - np.asarray(b)).max()
