@@ -680,8 +680,8 @@ __device__ __forceinline__ void unit_forces(const FFDev& D, const FFSys& S, cons
                                          __int_as_float(q));
             const float ex = dx + e.x, ey = dy + e.y, ez = dz + e.z;
             const float lim = reach + cj.w;
-            const bool keep = e0 + lane < T.n && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < lim * lim &&
-                              !(T.row < 0 && D.sgrp[q] == -1 - T.row);
+            bool keep = e0 + lane < T.n && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < lim * lim;
+            if (T.row < 0) keep = keep && D.sgrp[q] != -1 - T.row;  // (a branch: as one condition 1.5 % slower)
             const unsigned int m = __ballot_sync(kAll, keep);
             if (keep) T.ring[(head + held + __popc(m & ((1u << lane) - 1u))) & (kRing - 1)] = e;
             held += __popc(m);
