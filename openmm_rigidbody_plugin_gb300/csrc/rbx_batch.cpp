@@ -186,7 +186,7 @@ int cells_per_edge(double L, double edge, int most) {
 // centroid (constant for a rigid body), and from the largest radius of each system its list cells
 // (at least cutoff + skin + two radii per edge, or half of that). The lists themselves are sized by
 // size_lists, once the state is on the device.
-int setup_lists(rbx_batch* b, const double* x) {
+int setup_lists(rbx_batch* b, void* stream, const double* x) {
     const int S = b->S;
     std::vector<FFSys> sys = b->sys_h;
     std::vector<double> rho(S, 0.0);  // largest atom distance from a unit centroid
@@ -235,8 +235,10 @@ int setup_lists(rbx_batch* b, const double* x) {
         const double reach = (double)f.rl + 2.0 * rho_max;
         b->list_expect[s] = 4.18879 * reach * reach * reach * (double)U / (L * L * L);
     }
-    BATCH_TRY(cudaMemcpy(b->d_sys.p, sys.data(), sizeof(FFSys) * (size_t)S, cudaMemcpyHostToDevice));
     b->sys_h = sys;
+    // (on the state's stream: the kernels that read it follow there)
+    BATCH_TRY(cudaMemcpyAsync(b->d_sys.p, b->sys_h.data(), sizeof(FFSys) * (size_t)S, cudaMemcpyHostToDevice,
+                              (cudaStream_t)stream));
     FFDev& D = b->ff;
     const bool small = prep_limit(most_units, most_cells);
     D.prep_units = small ? (int)most_units : 0;
@@ -698,7 +700,7 @@ int rbx_batch_set_state(rbx_batch* b, void* stream, const double* positions, con
     BATCH_TRY(cudaSetDevice(b->device));
     BATCH_TRY(cudaStreamSynchronize((cudaStream_t)stream));  // no force pass in flight on the old lists
     b->d_body0.release();  // no state, until all of the new one is in place
-    if ((rc = setup_lists(b, positions))) return rc;
+    if ((rc = setup_lists(b, stream, positions))) return rc;
     // positions and velocities into the device buffers, bodies built there (no host round trip)
     if ((rc = rbx_context_load(b->integ, stream, positions, velocities))) return rc;
     rbx_buffers rb;
