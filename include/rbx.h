@@ -425,6 +425,8 @@ int rbx_batch_set_graph_steps(rbx_batch* b, int k);
  * pass, so it no longer changes the schedule) and the graph run length; rbx_batch_get_tile_threads
  * the tile shape. rbx_batch_set_tuning and rbx_batch_set_tile_threads set them by hand. */
 int rbx_batch_autotune(rbx_batch* b, void* stream, double dt, int trial_steps, int* chosen);
+/* cell_threads (64, 128 or 256) is checked and handed back by rbx_batch_autotune, but unused: no kernel reads
+ * it. */
 int rbx_batch_set_tuning(rbx_batch* b, int cell_threads, int graph_steps);
 int rbx_batch_set_tile_threads(rbx_batch* b, int threads);
 int rbx_batch_get_tile_threads(rbx_batch* b, int* out);

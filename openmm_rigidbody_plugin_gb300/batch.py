@@ -208,6 +208,7 @@ class BatchedSystems:
         _lib.check(self._lib.rbx_batch_set_tile_threads(self._h, int(threads)))
 
     def set_tuning(self, cell_threads, graph_steps):
+        """Steps per captured graph; cell_threads (64, 128 or 256) is checked but unused."""
         _lib.check(self._lib.rbx_batch_set_tuning(self._h, int(cell_threads), int(graph_steps)))
 
     def set_timing(self, on):

@@ -16,13 +16,14 @@
 // One evaluation, all systems at once. Batches whose systems are all small (prep_limit) take
 //   ff_prep     one block per system: each unit's centroid, radius and displacement since the last
 //               build; lists that stay get their atoms' records at their places in cell order, the
-//               others a new cell order first (cells of at least cutoff + skin + twice the largest
-//               radius per edge, counted, scanned and sorted in shared memory)
+//               others a new cell order first (cells of at least the reach, cutoff + skin + twice the
+//               largest radius, or of half of it; counted, scanned and sorted in shared memory)
 // and the others the same in kernels over all units (ff_check, ff_bin, ff_scan, ff_scatter,
 // ff_place; those after ff_check return at once for systems whose lists stay). Then
 //   ff_force    one warp per unit (all systems). Where the lists are to be rebuilt the warp first
-//               builds its own: the units in range among the 27 cells around it (or, in a
-//               single-cell box, all units by minimum image), in place order. Then the forces: the
+//               builds its own: the units in range among the cells within one cell (of the reach) or
+//               two (of half of it) of its own, rows of cells trimmed to the chord of the reach (in a
+//               single-cell box: all units by minimum image), row by row. Then the forces: the
 //               unit's atoms in registers, each lane taking one listed unit at a time; per-lane
 //               partial sums joined by a fixed butterfly, no atomics; forces written as OpenMM fixed
 //               point (2^32) to the slots
@@ -164,7 +165,8 @@ __device__ __forceinline__ void settle(const FFDev& D, const DevBuf& B, int prec
 }
 
 // Exclusive scan of n counts by a block: each thread a run of them, the runs' sums by warp shuffles.
-// put(i, start) receives every start; count(i) is read once. Returns nothing; ends without a barrier.
+// put(i, start) receives every start. Each count is read twice, by the same thread and last before its put, which
+// may so overwrite it. Ends without a barrier.
 template <class Count, class Put>
 __device__ __forceinline__ void block_scan(int n, int* wsum, const Count& count, const Put& put) {
     const int tid = threadIdx.x, nthr = blockDim.x;
