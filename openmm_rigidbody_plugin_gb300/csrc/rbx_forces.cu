@@ -762,8 +762,8 @@ __device__ __forceinline__ void unit_dispatch(const FFDev& D, const FFSys& S, co
 // then spill a little and still gain: forces of 40 boxes with 64-type solutes take 1.09 ms at 128
 // registers, 0.98 at 80 and 0.97 at 64 (later, with the list build's code, 0.75 at 80 and 0.77 at 64: the
 // form without the type-pair table takes 80, and so does the one with tables per system: 20 steps of 20 boxes
-// of waters beside 20 with solutes 4.95 ms, at 64 registers 5.16, at 96 4.93, at 128 5.46; all without a table,
-// as such batches once were, 4.85).
+// of waters beside 20 with solutes 4.95 ms, at 64 registers 5.16, at 96 4.93, at 128 5.46; now 4.85, and 4.87
+// without any table, as such batches once were).
 constexpr int force_blocks(int records) { return records <= 3 ? 8 : 6; }
 constexpr int kUntypedBlocks = 6;
 // Batches of at most kFewUnits units (two warps per scheduler) leave the SMs nearly empty: a warp's own
